@@ -19,6 +19,7 @@ namespace adf {
 // tile (the halo column xb-1 and Vx at xb+64 included), rows j0-1 .. j0+ty.
 constexpr int kStageW = 72;
 constexpr int kStepRing = 2;  // the stage of plane k in use while k+1 lands
+constexpr int kMaxZc = 32;    // planes per step work item, at most
 
 enum : int {
   SF_MASK = 1,      // solve has a scatterer mask
@@ -69,7 +70,7 @@ struct SolveDev {
   const float* coef;      // a_l a_r a_hl a_hr b_l b_r b_hl b_hr (Float32)
   // injection / recording entries, grouped by (y tile, plane, channel)
   const int* tp_off;      // nty*nz*4 + 1 offsets into seg
-  const int4* seg;        // {cell (row*nxp + x), first entry, count, 0}
+  const int4* seg;        // {x | tile row << 9 | count << 16, ...}
   const float* ent_w;
   const int* ent_tx;      // src column of the entry's transceiver, -1: no source
   const int* ent_slot;    // contribution slot (c*ntx+tx)*8+corner or -1

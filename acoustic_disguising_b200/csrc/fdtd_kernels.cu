@@ -13,9 +13,13 @@
 // (plus the halo row), its lanes 4-cell quads, and the CTA walks the planes
 // in z keeping the z-neighbours in registers.  The new P of a plane goes
 // through shared memory for the x-1 / y-1 neighbours of the velocity update;
-// the halo row and column are recomputed, not exchanged.  Grids of many
-// such CTAs (eight per SM) keep HBM busy: the update is a short,
-// memory-bound stencil.
+// the halo row and column are recomputed, not exchanged.  Five such CTAs per
+// SM keep HBM busy while a plane's chain (stage loads, Float64 arithmetic,
+// exchange of the new P, Float64 arithmetic) runs in each; what bounds them is
+// that chain and the instructions around it, not HBM.  With the stage read
+// through shared-space addresses, on different banks, and the entries' code out
+// of the plane loop, a launch of 8 x 256^3 takes 0.82 ms without boundaries
+// (0.89 before) and 1.71 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
 //
 // Arithmetic: Arith<double> reproduces Julia's promotion (Float32 storage,
 // Float64 Domain scalars, src/kernels/updates.jl) with explicit round-to-
@@ -339,25 +343,28 @@ __device__ __forceinline__ void v_update_quad(const SolveDev& S, const RowCtx& r
 
 // ---------------------------------------------------------------------------
 // interp_trilinear! entries of one (y tile, plane, channel) bucket
-// (derivatives.jl:30-60).  Segments are cells {cell = r*nxp + x | n << 16};
+// (derivatives.jl:30-60).  Segments are cells {x | row << 9 | n << 16};
 // inside a cell the entries are in transceiver order: rec += w*f (stored per
 // entry, summed by the epilogue in corner order), then f += w*src[it].  The
 // CTA handles the cells of its x range [x_lo, x_hi) and records only those
 // it owns (row >= 1, x >= xb; the P bucket also carries the tile's halo row
-// with slot -1).  `cells` maps (r, x) -> shared memory.
+// with slot -1).  Cell (row, x) is base[row * pitch + x] in shared memory.
+// Out of line: few planes carry entries, and inlined its address arithmetic
+// is hoisted into every plane of the step loop.
 // ---------------------------------------------------------------------------
-template <typename CellAt>
-__device__ __forceinline__ void apply_entries(const SolveDev& S, int b, int e, int chan, int nxp,
-                                              int x_lo, int x_hi, int xb, bool records, int it,
-                                              int tid, int nthr, CellAt cell_at) {
+__device__ __noinline__ void apply_entries(const SolveDev& S, int T, int k, int chan, int x_lo,
+                                           int x_hi, int xb, bool records, int it, float* base,
+                                           int pitch) {
+  const int* tp = S.tp_off + ((long long)T * S.nz + k) * 4 + chan;
+  const int b = __ldg(tp), e = __ldg(tp + 1);
+  const int tid = threadIdx.y * 32 + threadIdx.x, nthr = blockDim.x * blockDim.y;
   const float* src = S.src[chan] + (long long)(it - 1) * S.src_ntx;
   for (int si = b + tid; si < e; si += nthr) {
     const int4 sg = __ldg(S.seg + si);
-    const int cell = sg.x & 0xFFFF, cnt = (int)((unsigned)sg.x >> 16);
-    const int r = cell / nxp, x = cell - r * nxp;
+    const int x = sg.x & 0x1FF, r = (sg.x >> 9) & 0x7F, cnt = (int)((unsigned)sg.x >> 16);
     if (x < x_lo || x >= x_hi) continue;
     const bool rec = records && r >= 1 && x >= xb;
-    float* c = cell_at(r, x);
+    float* c = base + r * pitch + x;
     float v = *c;
     if (cnt == 1) {
       const float w = __int_as_float(sg.y);
@@ -469,7 +476,7 @@ __device__ __forceinline__ void v_plain_quad(const Sc<R>& g, float4 Pc, float Px
 // ---------------------------------------------------------------------------
 constexpr int kMaxTy = 7;           // rows per tile (plus the halo row: 8 per warp)
 constexpr int kXT = 64;             // cells per x tile (4 warps)
-constexpr int kPnPitch = kXT + 4;   // shared new-P row: [3] = halo column, [4..] = cells
+constexpr int kPnPitch = kStageW;   // shared new-P row: [3] = halo column, [4..] = cells
 constexpr int kStepThreads = 32 * kXT / 16;  // warps of 4 quads x 8 rows
 
 // One stage: P, Vx, Vy of a plane ([3][ty+2][kStageW]) and, from the next
@@ -487,14 +494,17 @@ static_assert((stage_vz_offset(5 * kStageW) * 4) % 128 == 0, "Vz boxes start 128
 template <typename R>
 __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S, int4 item, int it,
                                           float* sPn, float* sV, const float* co, float* ring,
-                                          uint64_t* rbar) {
+                                          const unsigned char* s_fl, uint64_t* rbar) {
   const int lane = threadIdx.x, wid = threadIdx.y;
   const int tid = wid * 32 + lane, nthr = blockDim.x * blockDim.y;
   const int nx = S.nx, ny = S.ny, nz = S.nz, nxp = S.nxp, ty = S.ty, npml = S.npml;
   const int T = item.y & 0xFFFF, X = item.y >> 16;
   const int j0 = T * ty, xb = X * kXT;
   // this thread's tile row r (0 = halo row) and quad qx; its warp's quads
-  const int qx = 4 * wid + (lane & 3), r = lane >> 2;
+  // (rows in the order 0 2 1 3 4 6 5 7: the eight quads of a 128-bit access are
+  // two rows 144 floats apart, which lie on different banks)
+  const int rq = lane >> 2;
+  const int qx = 4 * wid + (lane & 3), r = (rq & 4) | ((rq & 1) << 1) | ((rq >> 1) & 1);
   const int wq0 = 4 * wid, wnq = 4, wr0 = 0, wnr = kMaxTy + 1;
   const int j = j0 - 1 + r, x0 = xb + 4 * qx;
   const bool row_ok = r <= ty && j >= 0 && j < ny;
@@ -578,14 +588,13 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
     if (act) Z0 = ldg4(vz0);
     if (hcol) Zh = __ldg(vz0 - 1);
   }
-  const int* tp = S.tp_off + (long long)T * nz * 4;
   for (int k = kfirst; k < z1; ++k) {
     const bool prologue = k < z0;
     rc.k = k;
     float* pn = sPn + (k & 1) * (kMaxTy + 1) * kPnPitch;
     const float* st = ring + slot_of(k) * kStageFloats;
     wait(k);
-    const int off0 = __ldg(tp + 4 * k), off1 = __ldg(tp + 4 * k + 1), off4 = __ldg(tp + 4 * k + 4);
+    const int fl = s_fl[k - kfirst];
     const bool pplane = k != nz - 1 && (!pcp || (k >= npml && k < nz - npml));
     const bool vplane = k >= 1 && (!vcp || (k > npml && k < nz - npml - 1));
     const bool wplain = wplain_rx && pplane && (prologue || vplane);
@@ -617,9 +626,8 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
     // every read of plane k's stage is done: refill its slot
     if (tid == 0 && k + kStepRing < z1) issue(k + kStepRing);
     // ---- q channel: inject/record on the new P (forward.jl:92) ----
-    if (off0 < off1) {
-      apply_entries(S, off0, off1, 0, nxp, xb - 1, xb + kXT, xb, !prologue, it, tid, nthr,
-                    [&](int rr, int x) { return pn + rr * kPnPitch + (x - xb + 4); });
+    if (fl & 1) {
+      apply_entries(S, T, k, 0, xb - 1, xb + kXT, xb, !prologue, it, pn + 4 - xb, kPnPitch);
       __syncthreads();
       if (act) Pn = ld4(pn + pq);
     }
@@ -638,7 +646,7 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
         }
       }
       // ---- f channel: inject/record on the new V (forward.jl:111-115) ----
-      if (off1 < off4) {
+      if (fl & 2) {
         float* sVx = sV;
         float* sVy = sV + kMaxTy * kXT;
         float* sVz = sV + 2 * kMaxTy * kXT;
@@ -649,14 +657,9 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
           st4(sVz + so, vz);
         }
         __syncthreads();
-        for (int c = 1; c <= 3; ++c) {
-          const int b = __ldg(tp + 4 * k + c), e = __ldg(tp + 4 * k + c + 1);
-          if (b < e)
-            apply_entries(S, b, e, c, nxp, xb, xb + kXT, xb, true, it, tid, nthr,
-                          [&](int rr, int x) {
-                            return sV + (c - 1) * kMaxTy * kXT + (rr - 1) * kXT + (x - xb);
-                          });
-        }
+        for (int c = 1; c <= 3; ++c)
+          apply_entries(S, T, k, c, xb, xb + kXT, xb, true, it,
+                        sV + (c - 1) * kMaxTy * kXT - kXT - xb, kXT);
         __syncthreads();
         if (vrow) {
           vx = ld4(sVx + so);
@@ -693,12 +696,13 @@ constexpr size_t kStepDynSmem = sizeof(float) * kStepRing * kStageFloats + 128;
 
 __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_kernel(const StepParams p) {
   extern __shared__ __align__(128) float dyn_smem[];
-  float* ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(dyn_smem) + 127) &
-                                         ~static_cast<uintptr_t>(127));
+  // (an index, not a rounded pointer, so that the compiler keeps shared-space accesses)
+  float* ring = dyn_smem + ((0u - smem_u32(dyn_smem)) & 127u) / 4u;
   __shared__ __align__(8) uint64_t rbar[kStepRing];
   __shared__ __align__(16) float sPn[2 * (kMaxTy + 1) * kPnPitch];
   __shared__ __align__(16) float sV[3 * kMaxTy * kXT];
   __shared__ float s_co[kMaxCoef];
+  __shared__ unsigned char s_fl[kMaxZc + 1];  // planes kfirst ..: 1 q entries, 2 f entries
   __shared__ __align__(16) SolveDev S;  // the solve descriptor, read in the hot loop
   const int4 item = p.items[blockIdx.x];
   const SolveDev& G = p.solves[item.x];
@@ -711,6 +715,11 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
     for (int w = tid; w < (int)(sizeof(SolveDev) / 4); w += nthr) dst[w] = src[w];
     const int ncoef = 8 * G.npml + 4;
     for (int w = tid; w < ncoef; w += nthr) s_co[w] = G.coef[w];
+    const int kfirst = item.z > 0 ? item.z - 1 : 0;
+    if (tid < item.w - kfirst) {
+      const int* tp = G.tp_off + ((long long)(item.y & 0xFFFF) * G.nz + kfirst + tid) * 4;
+      s_fl[tid] = (unsigned char)((tp[0] < tp[1] ? 1 : 0) | (tp[1] < tp[4] ? 2 : 0));
+    }
     if (tid == 0) {
       for (int q = 0; q < kStepRing; ++q) mbar_init(smem_u32(rbar + q), 1);
       fence_mbar_init();
@@ -718,9 +727,9 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
   }
   __syncthreads();
   if (S.flags & SF_FP32)
-    step_item<float>(p, S, item, it, sPn, sV, s_co, ring, rbar);
+    step_item<float>(p, S, item, it, sPn, sV, s_co, ring, s_fl, rbar);
   else
-    step_item<double>(p, S, item, it, sPn, sV, s_co, ring, rbar);
+    step_item<double>(p, S, item, it, sPn, sV, s_co, ring, s_fl, rbar);
 }
 
 // Per-step trace assembly (derivatives.jl:51-56 record sums in corner order,

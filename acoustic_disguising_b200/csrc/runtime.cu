@@ -91,6 +91,7 @@ void choose_tiles(int nx, int ny, int nz, int& nxp, int& ty, int& nzc, int& mw) 
   if (ty > step_max_ty()) ty = step_max_ty();
   if (ty > ny) ty = ny;
   if (nzc < 2) nzc = 2;
+  if (nzc > kMaxZc) nzc = kMaxZc;
   if (nzc > nz) nzc = nz;
 }
 
@@ -118,7 +119,7 @@ size_t solve_bytes_estimate(int64_t nx, int64_t ny, int64_t nz, int64_t npml, in
 static int build_entries(Solve& s, const float* const idx[4], const float* const w[4],
                          const int* src_col) {
   SolveDev& d = s.dev;
-  const int ntx = d.ntx, nx = d.nx, ny = d.ny, nz = d.nz, ty = d.ty, nxp = d.nxp;
+  const int ntx = d.ntx, nx = d.nx, ny = d.ny, nz = d.nz, ty = d.ty;
   struct E {
     long long key;  // bucket * 2^32 + cell
     int tx;
@@ -142,7 +143,7 @@ static int build_entries(Solve& s, const float* const idx[4], const float* const
         const int T = j / ty, r = j - T * ty + 1;
         const long long bucket = ((long long)T * nz + k) * 4 + c;
         const int col = src_col ? src_col[tx] : tx;
-        es.push_back({(bucket << 32) | (long long)(r * nxp + i), tx, (c * ntx + tx) * 8 + n, wv,
+        es.push_back({(bucket << 32) | (long long)(r << 9 | i), tx, (c * ntx + tx) * 8 + n, wv,
                       col});
         if (c == 0 && (j + 1) % ty == 0 && j + 1 < ny) {
           const long long b2 = ((long long)((j + 1) / ty) * nz + k) * 4;
@@ -168,7 +169,7 @@ static int build_entries(Solve& s, const float* const idx[4], const float* const
     while (cur_b <= b) off[(size_t)cur_b++] = (int)seg.size();
     size_t j = i;
     while (j < es.size() && es[j].key == es[i].key) ++j;
-    // {cell | count<<16, ...}: one entry inline {w, slot, src column},
+    // {x | tile row << 9 | count << 16, ...}: one entry inline {w, slot, src column},
     // more than one {first entry, 0, 0} into the entry arrays
     const int cell = (int)(es[i].key & 0xffffffffLL);
     const int cnt = (int)(j - i);
