@@ -82,6 +82,7 @@ struct SolveDev {
   float* vn_rec;
   const float* dir;       // [ntx][4]
   const uint32_t* mask_bits;  // [nz][ny][mw] or NULL
+  const unsigned char* closed;  // [x tiles][nty][nz] 1: closed cells in the tile's plane; NULL: no mask
   int* err;               // per-solve error word
   int pad_;
   // in-loop GF extrapolation, SF_GF only
@@ -125,6 +126,8 @@ struct EpiParams {
 // launch helpers implemented in fdtd_kernels.cu
 // one CTA per work item, blockDim (32, max_ty + 1); max_ty <= step_max_ty()
 cudaError_t launch_step(const StepParams& p, int grid, int max_ty, cudaStream_t s);
+// fills SolveDev.closed from the mask bits (set-up)
+cudaError_t launch_mask_tiles(const SolveDev& d, unsigned char* closed, cudaStream_t s);
 int step_max_ty();
 int step_x_tile();  // cells per x tile of a step work item
 cudaError_t step_ctas_per_sm(int* n);  // resident step-kernel CTAs per SM (occupancy)

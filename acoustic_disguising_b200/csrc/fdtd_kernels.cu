@@ -19,7 +19,7 @@
 // that chain and the instructions around it, not HBM.  With the stage read
 // through shared-space addresses, on different banks, and the entries' code out
 // of the plane loop, a launch of 8 x 256^3 takes 0.82 ms without boundaries
-// (0.89 before) and 1.71 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
+// (0.89 before) and 1.60 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
 //
 // Arithmetic: Arith<double> reproduces Julia's promotion (Float32 storage,
 // Float64 Domain scalars, src/kernels/updates.jl) with explicit round-to-
@@ -203,7 +203,7 @@ __device__ __forceinline__ float4 p_update_quad(const SolveDev& S, const RowCtx&
 template <typename R>
 __device__ __forceinline__ float p_update_cell(const SolveDev& S, const RowCtx& rc, const Sc<R>& g,
                                                const float* co, const float* st, float Z0,
-                                               float Z1, int c, int cst, int x) {
+                                               float Z1, int c, int cst, int x, bool masked) {
   using A = Arith<R>;
   const int nx = rc.nx, ny = rc.ny, nz = rc.nz, npml = rc.npml, j = rc.j, k = rc.k, nxp = rc.nxp;
   const bool rigid_y = j == ny - 1, rigid_z = k == nz - 1;
@@ -220,7 +220,7 @@ __device__ __forceinline__ float p_update_cell(const SolveDev& S, const RowCtx& 
   R dvz = A::mul(A::cv(dz), g.rdz);
   bool open = true;
   if (!plain_rigid) {
-    if (S.flags & SF_MASK) open = (S.mask_bits[((long long)k * ny + j) * S.mw + (x >> 3)] >> (4 * (x & 7))) & 1u;
+    if (masked) open = (S.mask_bits[((long long)k * ny + j) * S.mw + (x >> 3)] >> (4 * (x & 7))) & 1u;
     if (rc.pcpml) {
       const int xs = x < npml ? 0 : (x >= nx - npml ? 1 : -1);
       if (xs >= 0) {
@@ -496,7 +496,7 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
                                           float* sPn, float* sV, const float* co, float* ring,
                                           const unsigned char* s_fl, uint64_t* rbar) {
   const int lane = threadIdx.x, wid = threadIdx.y;
-  const int tid = wid * 32 + lane, nthr = blockDim.x * blockDim.y;
+  const int tid = wid * 32 + lane;
   const int nx = S.nx, ny = S.ny, nz = S.nz, nxp = S.nxp, ty = S.ty, npml = S.npml;
   const int T = item.y & 0xFFFF, X = item.y >> 16;
   const int j0 = T * ty, xb = X * kXT;
@@ -513,7 +513,6 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
   const int rb = (it - S.it_first) & 1, wb = rb ^ 1;
   const long long cs = S.chan_stride, plane = (long long)ny * nxp;
   float* fout = S.field + wb * S.buf_stride;
-  const bool has_mask = (S.flags & SF_MASK) != 0;
   const bool pcp = (S.flags & SF_PCPML) != 0, vcp = (S.flags & SF_VCPML) != 0;
   Sc<R> g;
   g.fq = Arith<R>::fq(S);
@@ -595,6 +594,7 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
     const float* st = ring + slot_of(k) * kStageFloats;
     wait(k);
     const int fl = s_fl[k - kfirst];
+    const bool has_mask = (fl & 4) != 0;  // elsewhere every cell of the tile's plane is open
     const bool pplane = k != nz - 1 && (!pcp || (k >= npml && k < nz - npml));
     const bool vplane = k >= 1 && (!vcp || (k > npml && k < nz - npml - 1));
     const bool wplain = wplain_rx && pplane && (prologue || vplane);
@@ -619,7 +619,8 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
     }
     if (hcol) {
       const float Zh1 = k + 1 < nz ? st[vzo + so - 1] : 0.f;
-      pn[pq - 1] = p_update_cell<R>(S, rc, g, co, st, Zh, Zh1, so - 1, cst, xb - 1);
+      pn[pq - 1] = p_update_cell<R>(S, rc, g, co, st, Zh, Zh1, so - 1, cst, xb - 1,
+                                       has_mask);
       Zh = Zh1;
     }
     __syncthreads();
@@ -702,7 +703,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
   __shared__ __align__(16) float sPn[2 * (kMaxTy + 1) * kPnPitch];
   __shared__ __align__(16) float sV[3 * kMaxTy * kXT];
   __shared__ float s_co[kMaxCoef];
-  __shared__ unsigned char s_fl[kMaxZc + 1];  // planes kfirst ..: 1 q entries, 2 f entries
+  __shared__ unsigned char s_fl[kMaxZc + 1];  // planes kfirst ..: 1 q, 2 f entries, 4 closed cells
   __shared__ __align__(16) SolveDev S;  // the solve descriptor, read in the hot loop
   const int4 item = p.items[blockIdx.x];
   const SolveDev& G = p.solves[item.x];
@@ -718,7 +719,11 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
     const int kfirst = item.z > 0 ? item.z - 1 : 0;
     if (tid < item.w - kfirst) {
       const int* tp = G.tp_off + ((long long)(item.y & 0xFFFF) * G.nz + kfirst + tid) * 4;
-      s_fl[tid] = (unsigned char)((tp[0] < tp[1] ? 1 : 0) | (tp[1] < tp[4] ? 2 : 0));
+      int f = (tp[0] < tp[1] ? 1 : 0) | (tp[1] < tp[4] ? 2 : 0);
+      if (G.closed && G.closed[((long long)(item.y >> 16) * G.nty + (item.y & 0xFFFF)) * G.nz +
+                               kfirst + tid])
+        f |= 4;
+      s_fl[tid] = (unsigned char)f;
     }
     if (tid == 0) {
       for (int q = 0; q < kStepRing; ++q) mbar_init(smem_u32(rbar + q), 1);
@@ -730,6 +735,42 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
     step_item<float>(p, S, item, it, sPn, sV, s_co, ring, s_fl, rbar);
   else
     step_item<double>(p, S, item, it, sPn, sV, s_co, ring, s_fl, rbar);
+}
+
+// closed[x tile][y tile][plane] = 1 where a cell of the tile's plane, its halo
+// row and column included, has a closed mask bit (set-up, once per mask): the
+// step kernel reads the mask on those planes of a tile only, so that the rest
+// of the grid has neither the load in the plane's chain nor the selects (512^3
+// with an ellipsoid 1.38 -> 1.20 ms a launch, 8 x 256^3 with a sphere
+// 1.71 -> 1.60).  One warp per (x, y, plane).
+__global__ void adf_mask_tiles_kernel(const uint32_t* bits, int nx, int ny, int nz, int mw, int ty,
+                                      int nty, int nxt, unsigned char* closed) {
+  const long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  if (t >= (long long)nxt * nty * nz) return;
+  const int k = (int)(t % nz), T = (int)(t / nz % nty), X = (int)(t / nz / nty);
+  const int lane = threadIdx.x & 31;
+  bool shut = false;
+  for (int r = lane >> 2; r <= ty; r += 8) {
+    const int j = T * ty - 1 + r;
+    if (j < 0 || j >= ny) continue;
+    // words of cells xb-8 .. xb+63; nibbles past nx are zero in the mask and not cells
+    for (int i = (X * kXT >> 3) - 1 + (lane & 3); i < (X + 1) * kXT >> 3; i += 4) {
+      const int n = nx - 8 * i;  // cells of the word inside the grid
+      if (i < 0 || n <= 0) continue;
+      const uint32_t full = n >= 8 ? 0xFFFFFFFFu : (1u << (4 * n)) - 1u;
+      shut = shut || (bits[((long long)k * ny + j) * mw + i] & full) != full;
+    }
+  }
+  shut = __any_sync(0xffffffffu, shut);
+  if (lane == 0) closed[t] = shut ? 1 : 0;
+}
+
+cudaError_t launch_mask_tiles(const SolveDev& d, unsigned char* closed, cudaStream_t s) {
+  const int nxt = (d.nxp + kXT - 1) / kXT;
+  const long long warps = (long long)nxt * d.nty * d.nz;
+  adf_mask_tiles_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(d.mask_bits, d.nx, d.ny, d.nz,
+                                                                    d.mw, d.ty, d.nty, nxt, closed);
+  return cudaGetLastError();
 }
 
 // Per-step trace assembly (derivatives.jl:51-56 record sums in corner order,

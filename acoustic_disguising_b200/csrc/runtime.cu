@@ -100,7 +100,10 @@ size_t solve_bytes_estimate(int64_t nx, int64_t ny, int64_t nz, int64_t npml, in
   int nxp, ty, nzc, mw;
   choose_tiles((int)nx, (int)ny, (int)nz, nxp, ty, nzc, mw);
   size_t b = 2ull * 4 * nz * ny * nxp * 4;
-  if (mask) b += (size_t)mw * ny * nz * 4;
+  if (mask) {  // the bits, and a byte per tile and plane
+    b += (size_t)mw * ny * nz * 4;
+    b += (size_t)((nxp + step_x_tile() - 1) / step_x_tile()) * ((ny + ty - 1) / ty) * nz;
+  }
   size_t n = npml;
   b += 2ull * 2 * 4 * (nz * ny * n + nz * n * nxp + n * ny * nxp);
   b += 2ull * 2 * 4 * (nz * ny * (n + 1) + nz * (n + 1) * nxp + (n + 1) * ny * nxp);
@@ -387,6 +390,16 @@ int solve_finalize(adf_ctx* ctx, Solve& s, const float* const idx[4], const floa
                    const int* src_col) {
   int rc = build_entries(s, idx, w, src_col);
   if (rc) return rc;
+  if (s.dev.flags & SF_MASK) {  // the mask was written earlier on the same stream
+    const int nxt = (s.dev.nxp + step_x_tile() - 1) / step_x_tile();
+    unsigned char* closed = dalloc<unsigned char>(s, (size_t)nxt * s.dev.nty * s.dev.nz, rc);
+    if (rc) return rc;
+    if (launch_mask_tiles(s.dev, closed, s.stream) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(ADF_E_DEVICE, "mask tile launch failed");
+    }
+    s.dev.closed = closed;
+  }
   // work items {solve, y tile | x tile << 16, z0, z1}: z chunks outer, then
   // y tiles, x tiles inner, so that tiles sharing halo rows run together and
   // the halo hits L2
