@@ -533,7 +533,7 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
   rc.vcpml = vcp;
   // warp-uniform: do all of the warp's rows and x cells take the plain P
   // (and, rows >= 1, V) updates?  The plane is checked per plane below.
-  bool wplain_rx;
+  bool wplain_rx, hplain_x;
   {
     const int wj0 = j0 - 1 + wr0, wj1 = wj0 + wnr - 1;  // rows: P on all, V from wj0 + 1
     const int wx0 = xb + 4 * wq0, wx1 = wx0 + 4 * wnq - 1;
@@ -545,6 +545,7 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
     ok = ok && wj0 + 1 >= 1 && (!vcp || (wj0 + 1 > npml && wj1 < ny - npml - 1));
     ok = ok && wx0 >= v_xmin && wx1 <= v_xmax;
     wplain_rx = ok;
+    hplain_x = xb - 1 >= p_xmin && xb - 1 <= p_xmax;  // the halo column's cells
   }
   const long long rowoff = (long long)(row_ok ? j : 0) * nxp + x0;
   const int pq = r * kPnPitch + 4 + 4 * qx;  // this quad in a shared new-P plane
@@ -619,7 +620,12 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
     }
     if (hcol) {
       const float Zh1 = k + 1 < nz ? st[vzo + so - 1] : 0.f;
-      pn[pq - 1] = p_update_cell<R>(S, rc, g, co, st, Zh, Zh1, so - 1, cst, xb - 1,
+      if (wplain && hplain_x && !has_mask)
+        pn[pq - 1] = p_plain<R>(st[so - 1], __fsub_rn(X4.x, st[cst + so - 1]),
+                                __fsub_rn(st[2 * cst + so - 1 + kStageW], st[2 * cst + so - 1]),
+                                __fsub_rn(Zh1, Zh), g);
+      else
+        pn[pq - 1] = p_update_cell<R>(S, rc, g, co, st, Zh, Zh1, so - 1, cst, xb - 1,
                                        has_mask);
       Zh = Zh1;
     }
