@@ -19,7 +19,9 @@
 // that chain and the instructions around it, not HBM.  With the stage read
 // through shared-space addresses, on different banks, and the entries' code out
 // of the plane loop, a launch of 8 x 256^3 takes 0.82 ms without boundaries
-// (0.89 before) and 1.60 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
+// (0.89 before) and 1.54 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
+// The plane loop's code has to stay small: a masked form of the plain update and
+// one with the x slab's memory each made it slower (1.57 and 1.66 ms).
 //
 // Arithmetic: Arith<double> reproduces Julia's promotion (Float32 storage,
 // Float64 Domain scalars, src/kernels/updates.jl) with explicit round-to-
@@ -398,27 +400,20 @@ __device__ __forceinline__ float v_plain(float V, float dp, R rd, const Sc<R>& g
   using A = Arith<R>;
   return A::rn(A::sub(A::cv(V), A::mul(g.fv, A::mul(A::cv(dp), rd))));
 }
-template <typename R, bool MASK>
+template <typename R>
 __device__ __forceinline__ float4 p_plain_quad(const Sc<R>& g, float4 P4, float4 X4, float X5,
-                                               float4 Y0, float4 Y1, float4 Z0, float4 Z1,
-                                               uint32_t nib) {
+                                               float4 Y0, float4 Y1, float4 Z0, float4 Z1) {
   float4 n;
   n.x = p_plain<R>(P4.x, __fsub_rn(X4.y, X4.x), __fsub_rn(Y1.x, Y0.x), __fsub_rn(Z1.x, Z0.x), g);
   n.y = p_plain<R>(P4.y, __fsub_rn(X4.z, X4.y), __fsub_rn(Y1.y, Y0.y), __fsub_rn(Z1.y, Z0.y), g);
   n.z = p_plain<R>(P4.z, __fsub_rn(X4.w, X4.z), __fsub_rn(Y1.z, Y0.z), __fsub_rn(Z1.z, Z0.z), g);
   n.w = p_plain<R>(P4.w, __fsub_rn(X5, X4.w), __fsub_rn(Y1.w, Y0.w), __fsub_rn(Z1.w, Z0.w), g);
-  if (MASK) {
-    n.x = (nib & 1u) ? n.x : P4.x;
-    n.y = (nib & 0x10u) ? n.y : P4.y;
-    n.z = (nib & 0x100u) ? n.z : P4.z;
-    n.w = (nib & 0x1000u) ? n.w : P4.w;
-  }
   return n;
 }
-template <typename R, bool MASK>
+template <typename R>
 __device__ __forceinline__ void v_plain_quad(const Sc<R>& g, float4 Pc, float Pxm, float4 Pym,
                                              float4 Pzm, float4 VX, float4 VY, float4 VZ,
-                                             uint32_t nib, float4& vx, float4& vy, float4& vz) {
+                                             float4& vx, float4& vy, float4& vz) {
   vx.x = v_plain<R>(VX.x, __fsub_rn(Pc.x, Pxm), g.rdx, g);
   vx.y = v_plain<R>(VX.y, __fsub_rn(Pc.y, Pc.x), g.rdx, g);
   vx.z = v_plain<R>(VX.z, __fsub_rn(Pc.z, Pc.y), g.rdx, g);
@@ -431,20 +426,6 @@ __device__ __forceinline__ void v_plain_quad(const Sc<R>& g, float4 Pc, float Px
   vz.y = v_plain<R>(VZ.y, __fsub_rn(Pc.y, Pzm.y), g.rdz, g);
   vz.z = v_plain<R>(VZ.z, __fsub_rn(Pc.z, Pzm.z), g.rdz, g);
   vz.w = v_plain<R>(VZ.w, __fsub_rn(Pc.w, Pzm.w), g.rdz, g);
-  if (MASK) {
-    vx.x = (nib & 0x2u) ? vx.x : VX.x;
-    vx.y = (nib & 0x20u) ? vx.y : VX.y;
-    vx.z = (nib & 0x200u) ? vx.z : VX.z;
-    vx.w = (nib & 0x2000u) ? vx.w : VX.w;
-    vy.x = (nib & 0x4u) ? vy.x : VY.x;
-    vy.y = (nib & 0x40u) ? vy.y : VY.y;
-    vy.z = (nib & 0x400u) ? vy.z : VY.z;
-    vy.w = (nib & 0x4000u) ? vy.w : VY.w;
-    vz.x = (nib & 0x8u) ? vz.x : VZ.x;
-    vz.y = (nib & 0x80u) ? vz.y : VZ.y;
-    vz.z = (nib & 0x800u) ? vz.z : VZ.z;
-    vz.w = (nib & 0x8000u) ? vz.w : VZ.w;
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -598,7 +579,7 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
     const bool has_mask = (fl & 4) != 0;  // elsewhere every cell of the tile's plane is open
     const bool pplane = k != nz - 1 && (!pcp || (k >= npml && k < nz - npml));
     const bool vplane = k >= 1 && (!vcp || (k > npml && k < nz - npml - 1));
-    const bool wplain = wplain_rx && pplane && (prologue || vplane);
+    const bool wplain = wplain_rx && pplane && (prologue || vplane) && !has_mask;
     float4 Pn = make_float4(0.f, 0.f, 0.f, 0.f), X4 = Pn, Y0 = Pn, Z1 = Pn;
     uint32_t nib = 0xFFFFu;
     if (act) {
@@ -612,15 +593,14 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
         nib = (__ldg(S.mask_bits + ((long long)k * ny + j) * S.mw + (x0 >> 3)) >> ((x0 & 4) * 4)) &
               0xFFFFu;
       if (wplain)
-        Pn = has_mask ? p_plain_quad<R, true>(g, P4, X4, X5, Y0, Y1, Z0, Z1, nib)
-                      : p_plain_quad<R, false>(g, P4, X4, X5, Y0, Y1, Z0, Z1, nib);
+        Pn = p_plain_quad<R>(g, P4, X4, X5, Y0, Y1, Z0, Z1);
       else
         Pn = p_update_quad<R>(S, rc, g, co, x0, vrow && !prologue, P4, X4, X5, Y0, Y1, Z0, Z1, nib);
       st4(pn + pq, Pn);
     }
     if (hcol) {
       const float Zh1 = k + 1 < nz ? st[vzo + so - 1] : 0.f;
-      if (wplain && hplain_x && !has_mask)
+      if (wplain && hplain_x)
         pn[pq - 1] = p_plain<R>(st[so - 1], __fsub_rn(X4.x, st[cst + so - 1]),
                                 __fsub_rn(st[2 * cst + so - 1 + kStageW], st[2 * cst + so - 1]),
                                 __fsub_rn(Zh1, Zh), g);
@@ -644,10 +624,7 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
         const float Pxm = pn[pq - 1];
         const float4 Pym = ld4(pn + pq - kPnPitch);
         if (wplain) {
-          if (has_mask)
-            v_plain_quad<R, true>(g, Pn, Pxm, Pym, Pzm, X4, Y0, Z0, nib, vx, vy, vz);
-          else
-            v_plain_quad<R, false>(g, Pn, Pxm, Pym, Pzm, X4, Y0, Z0, nib, vx, vy, vz);
+          v_plain_quad<R>(g, Pn, Pxm, Pym, Pzm, X4, Y0, Z0, vx, vy, vz);
         } else {
           v_update_quad<R>(S, rc, g, co, x0, Pn, Pxm, Pym, Pzm, X4, Y0, Z0, nib, vx, vy, vz);
         }
