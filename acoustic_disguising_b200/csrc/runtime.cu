@@ -90,6 +90,7 @@ void choose_tiles(int nx, int ny, int nz, int& nxp, int& ty, int& nzc, int& mw) 
   if (ty < 2) ty = 2;
   if (ty > step_max_ty()) ty = step_max_ty();
   if (ty > ny) ty = ny;
+  if (nzc == 0) return;  // chosen for the batch
   if (nzc < 2) nzc = 2;
   if (nzc > kMaxZc) nzc = kMaxZc;
   if (nzc > nz) nzc = nz;
@@ -400,16 +401,49 @@ int solve_finalize(adf_ctx* ctx, Solve& s, const float* const idx[4], const floa
     }
     s.dev.closed = closed;
   }
-  // work items {solve, y tile | x tile << 16, z0, z1}: z chunks outer, then
-  // y tiles, x tiles inner, so that tiles sharing halo rows run together and
-  // the halo hits L2
-  s.items.clear();
-  const int xt = step_x_tile(), nxt = (s.dev.nxp + xt - 1) / xt;
-  for (int z0 = 0; z0 < s.dev.nz; z0 += s.nzc)
-    for (int t = 0; t < s.dev.nty; ++t)
-      for (int x = 0; x < nxt; ++x)
-        s.items.push_back(make_int4(0, t | (x << 16), z0, std::min(z0 + s.nzc, s.dev.nz)));
   return ADF_OK;
+}
+
+// Work items {solve, y tile | x tile << 16, z0, z1}: z chunks outer, then y
+// tiles, x tiles inner, so that tiles sharing halo rows run together and the
+// halo hits L2.
+long long Solve::columns() const {
+  const int xt = step_x_tile();
+  return (long long)((dev.nxp + xt - 1) / xt) * dev.nty;
+}
+void Solve::add_items(int depth, std::vector<int4>& out) const {
+  const int xt = step_x_tile(), nxt = (dev.nxp + xt - 1) / xt;
+  if (nzc > 0) depth = nzc;
+  // as many chunks as that depth gives, of equal depth
+  const int chunks = (dev.nz + depth - 1) / depth;
+  depth = (dev.nz + chunks - 1) / chunks;
+  for (int z0 = 0; z0 < dev.nz; z0 += depth)
+    for (int t = 0; t < dev.nty; ++t)
+      for (int x = 0; x < nxt; ++x)
+        out.push_back(make_int4(0, t | (x << 16), z0, std::min(z0 + depth, dev.nz)));
+}
+
+// Planes per work item of the batch's solves that have no tuned depth.  A CTA
+// walks its planes one after the other and recomputes one plane before them:
+// deep items waste least, shallow ones spread a small batch over the GPU.  When
+// a batch fits the GPU's resident CTAs at a depth of at most 12, the shallowest
+// such depth is taken (96^3: 73 us a step at 16 planes, 31 at 4; 40^3: 81 and
+// 22 at 3); otherwise the deepest of 24, 12 and 8 that leaves two CTAs for each
+// resident one, so that the last ones even out (2 x 256^3: 467 us at 32 planes,
+// 432 at 24, 445 at 16; 224^3: 212, 184 and 197 us at 24, 12 and 8).
+int batch_depth(const std::vector<Solve*>& list, long long resident) {
+  auto items = [&](int depth) {
+    long long n = 0;
+    for (const Solve* s : list)
+      n += s->columns() * ((s->dev.nz + (s->nzc > 0 ? s->nzc : depth) - 1) /
+                           (s->nzc > 0 ? s->nzc : depth));
+    return n;
+  };
+  for (int depth = 2; depth <= 12; ++depth)
+    if (items(depth) <= resident) return depth;
+  for (int depth : {24, 12})
+    if (items(depth) >= 2 * resident) return depth;
+  return 8;
 }
 
 // ---------------------------------------------------------------------------
@@ -458,14 +492,17 @@ int Batch::setup(adf_ctx* ctx, const std::vector<Solve*>& list) {
   }
   // interleave items of different solves so the batch stays balanced
   {
+    const int depth = batch_depth(list, ctx->step_ctas);
+    std::vector<std::vector<int4>> own(ns);
+    for (int i = 0; i < ns; ++i) list[i]->add_items(depth, own[i]);
     std::vector<size_t> pos(ns, 0);
     bool any = true;
     while (any) {
       any = false;
       for (int i = 0; i < ns; ++i) {
         // a few consecutive items per solve keep neighbouring tiles together
-        for (int k = 0; k < 8 && pos[i] < list[i]->items.size(); ++k) {
-          int4 it = list[i]->items[pos[i]++];
+        for (int k = 0; k < 8 && pos[i] < own[i].size(); ++k) {
+          int4 it = own[i][pos[i]++];
           it.x = i;
           items.push_back(it);
           any = true;
@@ -813,6 +850,9 @@ int adf_ctx_create(int device, size_t hbm_budget, adf_ctx** out) {
   c->nsm = prop.multiProcessorCount;
   c->smem_per_sm = (int)prop.sharedMemPerMultiprocessor;
   c->smem_optin = (int)prop.sharedMemPerBlockOptin;
+  int per_sm = 0;
+  if (step_ctas_per_sm(&per_sm) != cudaSuccess) cudaGetLastError();
+  c->step_ctas = std::max(1, per_sm) * c->nsm;
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete c;
     return fail(ADF_E_DEVICE, "stream creation failed");

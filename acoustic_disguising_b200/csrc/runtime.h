@@ -17,6 +17,7 @@ struct adf_ctx {
   int nsm = 148;
   int smem_per_sm = 233472;
   int smem_optin = 232448;
+  int step_ctas = 0;  // step-kernel CTAs the GPU holds at once
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // stream-ordered pool of the GF engine's solve memory; it keeps freed
@@ -57,8 +58,9 @@ inline hm::Dom to_dom(const adf_domain& d) {
   return o;
 }
 
-// Tile shape per grid size: rows per tile and z-chunk depth.  Chosen by the
-// autotuner (tune.cpp) and cached in a JSON table beside the library.
+// Tile shape per grid size: rows per tile and z-chunk depth (0: chosen for the
+// whole batch, Batch::setup).  Chosen by the autotuner (tune.cpp) and cached in
+// a JSON table beside the library.
 struct Tune {
   int ty;
   int nzc;
@@ -72,7 +74,7 @@ struct Solve {
   unsigned char fmap_host[4 * 128];  // the tensor maps of dev.fmap (copied to the device)
   std::vector<void*> allocs;
   size_t bytes = 0;
-  int nzc = 32;
+  int nzc = 0;             // planes per work item, 0: chosen for the batch
   uint32_t* mask_bits = nullptr;
   float* coef_dev = nullptr;
   float* dir_dev = nullptr;
@@ -82,7 +84,8 @@ struct Solve {
   cudaStream_t stream = nullptr;
   cudaStream_t alloc_stream = nullptr;  // stream-ordered allocation from alloc_pool when set
   cudaMemPool_t alloc_pool = nullptr;
-  std::vector<int4> items;  // {0, y tile | x tile << 16, z0, z1}
+  long long columns() const;                                // x tiles x y tiles
+  void add_items(int depth, std::vector<int4>& out) const;  // {0, y tile | x tile << 16, z0, z1}
   ~Solve();
   void release();
 };
@@ -119,6 +122,7 @@ struct Batch {
 };
 
 void choose_tiles(int nx, int ny, int nz, int& nxp, int& ty, int& nzc, int& mw);
+int batch_depth(const std::vector<Solve*>& list, long long resident);
 size_t solve_bytes_estimate(int64_t nx, int64_t ny, int64_t nz, int64_t npml, int64_t ntx,
                             int64_t nt, bool mask);
 int solve_alloc(adf_ctx* ctx, Solve& s, const hm::Dom& dom, int npml, bool has_mask, int arith,

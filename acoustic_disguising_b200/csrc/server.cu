@@ -63,15 +63,16 @@ struct GfJob {
   bool cancel = false;
   std::unique_ptr<Solve> solve;
   size_t est = 0;
-  long long items = 0;  // step-kernel work items (CTAs per step launch)
+  long long items = 0;  // step work in work items (gf_items)
 };
 
-// Work items one step launch runs for this request's grid (as solve_finalize
-// builds them: x tiles x y tiles x z chunks).
+// Step work of this request's grid, in work items (x tiles x y tiles x z chunks)
+// of the tuned depth, or of 16 planes where the depth is the batch's choice.
 static long long gf_items(const adf_gf_request& r) {
   int nxp, ty, nzc, mw;
   choose_tiles((int)r.dom.nx, (int)r.dom.ny, (int)r.dom.nz, nxp, ty, nzc, mw);
   const long long xt = step_x_tile();
+  if (nzc == 0) nzc = 16;
   return (nxp + xt - 1) / xt * ((r.dom.ny + ty - 1) / ty) * ((r.dom.nz + nzc - 1) / nzc);
 }
 

@@ -56,7 +56,7 @@ static Tune default_tune(int nx, int ny, int nz) {
   // plus the recomputed halo row) and recompute the fewest halo rows.
   t.ty = 7;
   (void)nx;
-  t.nzc = 16;
+  t.nzc = 0;  // the batch's choice (batch_depth)
   (void)ny;
   return t;
 }

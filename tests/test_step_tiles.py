@@ -27,3 +27,37 @@ def test_closed_cells_on_tile_edges(adf, oracle, ctx, nx, ny, nz, npml):
     assert not mask.all()
     gpu, cpu = run_both(adf, oracle, (d, o, g, cp, mask, field))
     assert_parity(gpu, cpu, 1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nz", [4, 5, 13, 34])
+def test_shallow_items(adf, oracle, ctx, nz):
+    """A small run takes the shallowest work items: two planes, the last item
+    one (the rigid plane alone) when nz is odd."""
+    case = make_case(adf, oracle, 40, 30, nz, steps=25, npml=min(4, (nz - 2) // 2), shape="none",
+                     seed=nz, n_rec=6)
+    gpu, cpu = run_both(adf, oracle, case)
+    assert_parity(gpu, cpu, 1e-6)
+
+
+@pytest.mark.gpu
+def test_depth_of_a_batch_changes_nothing(adf, ctx):
+    """Ten solves share deeper items than one alone: the traces stay bit for
+    bit those of the plain path."""
+    from test_fdtd_parity import C0, DT, DX, RHO
+
+    def request(n, k):
+        d = adf.Domain(tmax=29.5 * DT, xmax=(n - 1) * DX / 2, nx=n, c0=C0, r0=RHO, cf=0.5)
+        tf, _ = adf.impulsive_wavelet(d, 9000.0)
+        rp, rn = adf.fibonacci_sphere(30, 0.5 * d.xmax)
+        return adf.GfRequest(d, [0.3 * d.xmax, 0.02 * k * d.xmax, 0.0], [1.0, 0, 0, 0], tf, rp, rn,
+                             npml=6, pml_fc=2000.0, scatterer="sphere",
+                             scatterer_kw=dict(radius=0.2 * d.xmax))
+    sizes = [96, 90, 85, 96, 64, 71, 96, 96, 80, 96]
+    batch = [request(n, k) for k, n in enumerate(sizes)]
+    alone = [request(n, k) for k, n in enumerate(sizes)]
+    adf.gf_solve_batch(batch, batched=True)
+    adf.gf_solve_batch(alone, batched=False)
+    for a, b in zip(batch, alone):
+        assert np.abs(a.p).max() > 0
+        assert np.array_equal(a.p, b.p) and np.array_equal(a.vn, b.vn)
