@@ -126,6 +126,11 @@ struct EpiParams {
 // launch helpers implemented in fdtd_kernels.cu
 // one CTA per work item, blockDim (32, max_ty + 1); max_ty <= step_max_ty()
 cudaError_t launch_step(const StepParams& p, int grid, int max_ty, cudaStream_t s);
+// layout conversions of a call's arrays (runtime.cu): src[c][r] -> dst[r][c] over
+// cols x rows, and rows of `width` floats from one pitch to another
+cudaError_t launch_transpose(const float* src, float* dst, int rows, int cols, cudaStream_t s);
+cudaError_t launch_repitch(const float* src, long long src_pitch, float* dst, long long dst_pitch,
+                           int width, long long rows, cudaStream_t s);
 // fills SolveDev.closed from the mask bits (set-up)
 cudaError_t launch_mask_tiles(const SolveDev& d, unsigned char* closed, cudaStream_t s);
 int step_max_ty();

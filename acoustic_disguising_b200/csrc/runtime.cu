@@ -125,78 +125,81 @@ static int build_entries(Solve& s, const float* const idx[4], const float* const
   SolveDev& d = s.dev;
   const int ntx = d.ntx, nx = d.nx, ny = d.ny, nz = d.nz, ty = d.ty;
   struct E {
-    long long key;  // bucket * 2^32 + cell
-    int tx;
+    int cell;   // x | tile row << 9
     int slot;
     float w;
-    int col;        // src column, -1 when the transceiver never injects
+    int col;    // src column, -1 when the transceiver never injects
   };
-  std::vector<E> es;
-  es.reserve((size_t)ntx * 36);
+  const size_t nb = (size_t)d.nty * nz * 4;  // buckets (y tile, plane, channel)
   std::vector<unsigned char> inb((size_t)4 * ntx, 0);
+  // visits every corner as (bucket, entry), channels outer, transceivers inner
+  auto each = [&](auto&& put) {
+    for (int c = 0; c < 4; ++c)
+      for (int tx = 0; tx < ntx; ++tx) {
+        if (!inb[(size_t)c * ntx + tx]) continue;
+        const int I = (int)idx[c][3 * tx], J = (int)idx[c][3 * tx + 1], K = (int)idx[c][3 * tx + 2];
+        const int col = src_col ? src_col[tx] : tx;
+        for (int n = 0; n < 8; ++n) {
+          const int i = I - 1 + (n & 1), j = J - 1 + ((n >> 1) & 1), k = K - 1 + (n >> 2);
+          const float wv = w[c][8 * tx + n];
+          const int T = j / ty, r = j - T * ty + 1;
+          put(((size_t)T * nz + k) * 4 + c, E{r << 9 | i, (c * ntx + tx) * 8 + n, wv, col});
+          if (c == 0 && (j + 1) % ty == 0 && j + 1 < ny)
+            put(((size_t)((j + 1) / ty) * nz + k) * 4, E{i, -1, wv, col});
+        }
+      }
+  };
   for (int c = 0; c < 4; ++c)
     for (int tx = 0; tx < ntx; ++tx) {
       const int I = (int)idx[c][3 * tx], J = (int)idx[c][3 * tx + 1], K = (int)idx[c][3 * tx + 2];
-      const bool ok = I >= 1 && I < nx && J >= 1 && J < ny && K >= 1 && K < nz;
-      inb[(size_t)c * ntx + tx] = ok;
-      if (!ok) continue;
-      for (int n = 0; n < 8; ++n) {
-        const int ii = n & 1, jj = (n >> 1) & 1, kk = n >> 2;
-        const int i = I - 1 + ii, j = J - 1 + jj, k = K - 1 + kk;
-        const float wv = w[c][8 * tx + n];
-        const int T = j / ty, r = j - T * ty + 1;
-        const long long bucket = ((long long)T * nz + k) * 4 + c;
-        const int col = src_col ? src_col[tx] : tx;
-        es.push_back({(bucket << 32) | (long long)(r << 9 | i), tx, (c * ntx + tx) * 8 + n, wv,
-                      col});
-        if (c == 0 && (j + 1) % ty == 0 && j + 1 < ny) {
-          const long long b2 = ((long long)((j + 1) / ty) * nz + k) * 4;
-          es.push_back({(b2 << 32) | (long long)i, tx, -1, wv, col});
-        }
-      }
+      inb[(size_t)c * ntx + tx] = I >= 1 && I < nx && J >= 1 && J < ny && K >= 1 && K < nz;
     }
-  std::stable_sort(es.begin(), es.end(), [](const E& a, const E& b) {
-    return a.key < b.key || (a.key == b.key && a.tx < b.tx);
-  });
-  const long long nb = (long long)d.nty * nz * 4;
-  std::vector<int> off((size_t)nb + 1, 0);
+  // counting sort by bucket (keeps the transceiver order), then by cell inside
+  // each: a bucket holds a few cells
+  std::vector<unsigned> at(nb + 1, 0);
+  each([&](size_t b, const E&) { ++at[b + 1]; });
+  for (size_t b = 0; b < nb; ++b) at[b + 1] += at[b];
+  std::vector<E> es(at[nb]);
+  {
+    std::vector<unsigned> next(at.begin(), at.end() - 1);
+    each([&](size_t b, const E& e) { es[next[b]++] = e; });
+  }
+  std::vector<int> off(nb + 1, 0);
   std::vector<int4> seg;
   std::vector<float> ew;
   std::vector<int> etx, eslot;
-  ew.reserve(es.size());
-  etx.reserve(es.size());
-  eslot.reserve(es.size());
-  size_t i = 0;
-  long long cur_b = 0;
-  for (; i < es.size();) {
-    const long long b = es[i].key >> 32;
-    while (cur_b <= b) off[(size_t)cur_b++] = (int)seg.size();
-    size_t j = i;
-    while (j < es.size() && es[j].key == es[i].key) ++j;
-    // {x | tile row << 9 | count << 16, ...}: one entry inline {w, slot, src column},
-    // more than one {first entry, 0, 0} into the entry arrays
-    const int cell = (int)(es[i].key & 0xffffffffLL);
-    const int cnt = (int)(j - i);
-    int4 sg;
-    sg.x = cell | (cnt << 16);
-    if (cnt == 1) {
-      std::memcpy(&sg.y, &es[i].w, 4);
-      sg.z = es[i].slot;
-      sg.w = es[i].col;
-    } else {
-      sg.y = (int)ew.size();
-      sg.z = 0;
-      sg.w = 0;
-      for (size_t k = i; k < j; ++k) {
-        ew.push_back(es[k].w);
-        etx.push_back(es[k].col);
-        eslot.push_back(es[k].slot);
+  seg.reserve(es.size());
+  for (size_t b = 0; b < nb; ++b) {
+    off[b] = (int)seg.size();
+    std::stable_sort(es.begin() + at[b], es.begin() + at[b + 1],
+                     [](const E& p, const E& q) { return p.cell < q.cell; });
+    for (size_t i = at[b]; i < at[b + 1];) {
+      size_t j = i;
+      while (j < at[b + 1] && es[j].cell == es[i].cell) ++j;
+      // {x | tile row << 9 | count << 16, ...}: one entry inline {w, slot, src column},
+      // more than one {first entry, 0, 0} into the entry arrays
+      const int cnt = (int)(j - i);
+      int4 sg;
+      sg.x = es[i].cell | (cnt << 16);
+      if (cnt == 1) {
+        std::memcpy(&sg.y, &es[i].w, 4);
+        sg.z = es[i].slot;
+        sg.w = es[i].col;
+      } else {
+        sg.y = (int)ew.size();
+        sg.z = 0;
+        sg.w = 0;
+        for (size_t k = i; k < j; ++k) {
+          ew.push_back(es[k].w);
+          etx.push_back(es[k].col);
+          eslot.push_back(es[k].slot);
+        }
       }
+      seg.push_back(sg);
+      i = j;
     }
-    seg.push_back(sg);
-    i = j;
   }
-  while (cur_b <= nb) off[(size_t)cur_b++] = (int)seg.size();
+  off[nb] = (int)seg.size();
   int rc = ADF_OK;
   int* d_off = dalloc<int>(s, off.size(), rc);
   int4* d_seg = dalloc<int4>(s, seg.size(), rc);
@@ -360,31 +363,22 @@ int solve_alloc(adf_ctx* ctx, Solve& s, const hm::Dom& dom, int npml, bool has_m
   return ADF_OK;
 }
 
-int solve_alloc_traces(Solve& s, bool need_vsrc) {
+// (the caller's traces fill all of them)
+int solve_alloc_traces(Solve& s) {
   SolveDev& d = s.dev;
   const size_t n = (size_t)d.nt * d.ntx;
   d.src_ntx = d.ntx;
   int rc = ADF_OK;
   for (int c = 0; c < 4; ++c) {
     d.rec[c] = dalloc<float>(s, n, rc);
-    if (rc) return rc;
-    cudaMemsetAsync(d.rec[c], 0, n * 4, s.stream);
-  }
-  for (int c = 0; c < 4; ++c) {
     d.src[c] = dalloc<float>(s, n, rc);
-    if (rc) return rc;
-    cudaMemsetAsync(d.src[c], 0, n * 4, s.stream);
   }
   d.vn_src = dalloc<float>(s, n, rc);
   d.vn_rec = dalloc<float>(s, n, rc);
   float* dir = dalloc<float>(s, (size_t)4 * d.ntx, rc);
-  if (rc) return rc;
-  cudaMemsetAsync(d.vn_src, 0, n * 4, s.stream);
-  cudaMemsetAsync(d.vn_rec, 0, n * 4, s.stream);
   d.dir = dir;
   s.dir_dev = dir;
-  (void)need_vsrc;
-  return ADF_OK;
+  return rc;
 }
 
 int solve_finalize(adf_ctx* ctx, Solve& s, const float* const idx[4], const float* const w[4],
@@ -454,8 +448,8 @@ void Batch::release() {
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
   graph_exec = nullptr;
   graph_steps = 0;
-  if (d_solves) cudaFree(d_solves);
-  if (d_items) cudaFree(d_items);
+  if (d_solves) cudaFreeAsync(d_solves, alloc_stream);
+  if (d_items) cudaFreeAsync(d_items, alloc_stream);
   d_solves = nullptr;
   d_items = nullptr;
   cap_solves = cap_items = 0;
@@ -515,8 +509,11 @@ int Batch::setup(adf_ctx* ctx, const std::vector<Solve*>& list) {
     release();
     cap_solves = std::max(ns, 1);
     cap_items = std::max(n_items, 1);
-    if (cudaMalloc(&d_solves, sizeof(SolveDev) * cap_solves) != cudaSuccess ||
-        cudaMalloc(&d_items, sizeof(int4) * cap_items) != cudaSuccess) {
+    alloc_stream = ctx->stream;
+    if (cudaMallocFromPoolAsync((void**)&d_solves, sizeof(SolveDev) * cap_solves, ctx->pool,
+                                ctx->stream) != cudaSuccess ||
+        cudaMallocFromPoolAsync((void**)&d_items, sizeof(int4) * cap_items, ctx->pool,
+                                ctx->stream) != cudaSuccess) {
       cudaGetLastError();
       return fail(ADF_E_NOMEM, "batch descriptor allocation failed");
     }
@@ -714,34 +711,19 @@ using namespace adf;
 // ---------------------------------------------------------------------------
 // layout helpers
 // ---------------------------------------------------------------------------
-// Julia (nt, ntx) time-fastest  <->  device [nt][ntx] transceiver-fastest
-static void transpose_to_dev_layout(const float* jl, float* out, int64_t nt, int64_t ntx) {
-  const int64_t B = 64;
-  for (int64_t t0 = 0; t0 < nt; t0 += B)
-    for (int64_t x0 = 0; x0 < ntx; x0 += B)
-      for (int64_t x = x0; x < std::min(ntx, x0 + B); ++x)
-        for (int64_t t = t0; t < std::min(nt, t0 + B); ++t) out[t * ntx + x] = jl[t + nt * x];
-}
-static void transpose_to_julia(const float* dv, float* jl, int64_t nt, int64_t ntx) {
-  const int64_t B = 64;
-  for (int64_t x0 = 0; x0 < ntx; x0 += B)
-    for (int64_t t0 = 0; t0 < nt; t0 += B)
-      for (int64_t t = t0; t < std::min(nt, t0 + B); ++t)
-        for (int64_t x = x0; x < std::min(ntx, x0 + B); ++x) jl[t + nt * x] = dv[t * ntx + x];
-}
+// Each array crosses as the caller holds it, through a device buffer `stage`
+// that the next one reuses in stream order; kernels convert the layout.  A
+// pageable source is staged before cudaMemcpyAsync returns, and a copy to
+// pageable memory has arrived when it returns.
 
-// Uploads on stream `st`, so the kernels that follow on it are ordered after
-// them; the staging vector is reused only once its copy has completed.
-static cudaError_t upload_traces(Solve& s, const adf_txgrid* txs, cudaStream_t st) {
+// Julia (nt, ntx) time-fastest -> device [nt][ntx] transceiver-fastest
+static cudaError_t upload_traces(Solve& s, const adf_txgrid* txs, float* stage, cudaStream_t st) {
   SolveDev& d = s.dev;
-  const int64_t nt = d.nt, ntx = d.ntx;
-  std::vector<float> tmp((size_t)(nt * ntx));
+  const size_t bytes = (size_t)d.nt * d.ntx * 4;
   cudaError_t e = cudaSuccess;
   auto up = [&](const float* jl, float* dst) {
-    if (e != cudaSuccess) return;
-    transpose_to_dev_layout(jl, tmp.data(), nt, ntx);
-    e = cudaMemcpyAsync(dst, tmp.data(), tmp.size() * 4, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(stage, jl, bytes, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = launch_transpose(stage, dst, d.nt, d.ntx, st);
   };
   for (int c = 0; c < 4; ++c) {
     up(txs->src[c], d.src[c]);
@@ -750,74 +732,77 @@ static cudaError_t upload_traces(Solve& s, const adf_txgrid* txs, cudaStream_t s
   up(txs->vn_src, d.vn_src);
   up(txs->vn_rec, d.vn_rec);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(s.dir_dev, txs->dir, (size_t)4 * ntx * 4, cudaMemcpyHostToDevice, st);
+    e = cudaMemcpyAsync(s.dir_dev, txs->dir, (size_t)4 * d.ntx * 4, cudaMemcpyHostToDevice, st);
   return e;
 }
 
-// Device (step-major) traces -> the caller's Julia (nt, ntx) arrays.  Stops at
-// the first failed copy and returns its error; nothing is transposed from it.
-static cudaError_t download_trace(Solve& s, std::vector<float>& tmp, const float* src, float* jl) {
-  const cudaError_t e = cudaMemcpy(tmp.data(), src, tmp.size() * 4, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) transpose_to_julia(tmp.data(), jl, s.dev.nt, s.dev.ntx);
-  return e;
-}
-
-static cudaError_t download_traces(Solve& s, adf_txgrid* txs) {
+// Device (step-major) traces -> the caller's Julia (nt, ntx) arrays; with
+// `sources` also p_src and vn_src, which the GF extrapolation writes.  Stops at
+// the first failed copy and returns its error.
+static cudaError_t download_traces(Solve& s, adf_txgrid* txs, bool sources, float* stage,
+                                   cudaStream_t st) {
   SolveDev& d = s.dev;
-  std::vector<float> tmp((size_t)(d.nt * d.ntx));
+  const size_t bytes = (size_t)d.nt * d.ntx * 4;
   cudaError_t e = cudaSuccess;
-  for (int c = 0; c < 4 && e == cudaSuccess; ++c) {
-    e = download_trace(s, tmp, d.rec[c], txs->rec[c]);
-    if (c > 0 && e == cudaSuccess) e = download_trace(s, tmp, d.src[c], txs->src[c]);
+  auto down = [&](const float* src, float* jl) {
+    if (e == cudaSuccess) e = launch_transpose(src, stage, d.ntx, d.nt, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(jl, stage, bytes, cudaMemcpyDeviceToHost, st);
+  };
+  for (int c = 0; c < 4; ++c) {
+    down(d.rec[c], txs->rec[c]);
+    if (c > 0) down(d.src[c], txs->src[c]);
   }
-  if (e == cudaSuccess) e = download_trace(s, tmp, d.vn_rec, txs->vn_rec);
+  down(d.vn_rec, txs->vn_rec);
+  if (sources) {
+    down(d.src[0], txs->src[0]);
+    down(d.vn_src, txs->vn_src);
+  }
   return e;
 }
 
-// the GF extrapolation writes p_src and vn_src rows: both come back too
-static cudaError_t download_gf_sources(Solve& s, adf_txgrid* txs) {
-  SolveDev& d = s.dev;
-  std::vector<float> tmp((size_t)(d.nt * d.ntx));
-  cudaError_t e = download_trace(s, tmp, d.src[0], txs->src[0]);
-  if (e == cudaSuccess) e = download_trace(s, tmp, d.vn_src, txs->vn_src);
-  return e;
+// psi: Julia (npml,ny,nz,2) / (nx,npml,nz,2) / (nx,ny,npml,2) <-> device.  An
+// upload fills both buffers, a download takes the one given.
+static size_t psi_floats(const SolveDev& d, int axis, bool vside) {
+  const size_t n = vside ? d.npml + 1 : d.npml;
+  const size_t nx = d.nx, ny = d.ny, nz = d.nz;
+  return 2 * n * (axis == 0 ? ny * nz : axis == 1 ? nx * nz : nx * ny);
 }
-
-// psi: Julia (npml,ny,nz,2) / (nx,npml,nz,2) / (nx,ny,npml,2) <-> device.
-// Uploads are stream-ordered on `st`; downloads are synchronous copies taken
-// after the caller has synchronised the stream that wrote the memory.
 static cudaError_t psi_copy(Solve& s, int axis, bool vside, float* host, bool upload, int buffer,
-                            cudaStream_t st) {
+                            float* stage, cudaStream_t st) {
   SolveDev& d = s.dev;
   const long long n = vside ? d.npml + 1 : d.npml;
   float* base = vside ? d.psi_v[axis] : d.psi_p[axis];
   const long long side = vside ? d.psi_v_side[axis] : d.psi_p_side[axis];
-  float* dev = base + (long long)buffer * 2 * side;
-  if (axis == 0) {  // rows of n values per side; device pitch npp / nvp, side 1 offset
-    const size_t pitch = (size_t)(vside ? d.nvp : d.npp) * 4;
-    const size_t rows = (size_t)d.ny * d.nz;
-    const long long first1 = vside ? d.nx - d.npml - 1 : d.nx - d.npml;  // side 1's first cell
-    // (a grid narrower than npml+1 cells never uses side 1: any in-row offset does)
-    const long long off1 = first1 < 0 ? 0 : first1 - (vside ? d.xs1v : d.xs1p);
-    for (int sd = 0; sd < 2; ++sd) {
-      float* dv = dev + sd * side + (sd ? off1 : 0);
-      float* hs = host + (size_t)sd * rows * n;
-      const cudaError_t e =
-          upload ? cudaMemcpy2DAsync(dv, pitch, hs, (size_t)n * 4, (size_t)n * 4, rows,
-                                     cudaMemcpyHostToDevice, st)
-                 : cudaMemcpy2D(hs, (size_t)n * 4, dv, pitch, (size_t)n * 4, rows,
-                                cudaMemcpyDeviceToHost);
-      if (e != cudaSuccess) return e;
+  const size_t bytes = psi_floats(d, axis, vside) * 4;
+  // a block of rows of `width` floats: its place in a device buffer, in the host array
+  auto move = [&](float* dev, long long pitch, float* st_rows, int width, long long rows) {
+    return upload ? launch_repitch(st_rows, width, dev, pitch, width, rows, st)
+                  : launch_repitch(dev, pitch, st_rows, width, width, rows, st);
+  };
+  cudaError_t e = cudaSuccess;
+  if (upload) e = cudaMemcpyAsync(stage, host, bytes, cudaMemcpyHostToDevice, st);
+  for (int b = upload ? 0 : buffer; b <= (upload ? 1 : buffer); ++b) {
+    float* dev = base + (long long)b * 2 * side;
+    if (axis == 0) {  // rows of n values per side; device pitch npp / nvp, side 1 offset
+      const long long rows = (long long)d.ny * d.nz;
+      const long long first1 = vside ? d.nx - d.npml - 1 : d.nx - d.npml;  // side 1's first cell
+      // (a grid narrower than npml+1 cells never uses side 1: any in-row offset does)
+      const long long off1 = first1 < 0 ? 0 : first1 - (vside ? d.xs1v : d.xs1p);
+      for (int sd = 0; sd < 2 && e == cudaSuccess; ++sd)
+        e = move(dev + sd * side + (sd ? off1 : 0), vside ? d.nvp : d.npp, stage + sd * rows * n,
+                 (int)n, rows);
+    } else if (e == cudaSuccess) {
+      e = move(dev, d.nxp, stage, d.nx, axis == 1 ? n * d.nz * 2 : d.ny * n * 2);
     }
-    return cudaSuccess;
   }
-  const size_t rows = axis == 1 ? (size_t)n * d.nz * 2 : (size_t)d.ny * n * 2;
-  if (upload)
-    return cudaMemcpy2DAsync(dev, (size_t)d.nxp * 4, host, (size_t)d.nx * 4, (size_t)d.nx * 4,
-                             rows, cudaMemcpyHostToDevice, st);
-  return cudaMemcpy2D(host, (size_t)d.nx * 4, dev, (size_t)d.nxp * 4, (size_t)d.nx * 4, rows,
-                      cudaMemcpyDeviceToHost);
+  if (!upload && e == cudaSuccess)
+    e = cudaMemcpyAsync(host, stage, bytes, cudaMemcpyDeviceToHost, st);
+  return e;
 }
+
+// The context's pool after a run that took its memory from it: back to what it
+// held before, or to this much where that is less.
+constexpr size_t kPoolKeep = (size_t)1 << 30;
 
 // ---------------------------------------------------------------------------
 // C-ABI
@@ -1113,11 +1098,33 @@ static int run_fdtd_impl(adf_ctx* ctx, const adf_domain* d, float* field, adf_tx
               (size_t)8 * kGfRing * gf->n_rec;
     if (use_tc) need += sizeof(float) * gf_tc_packed_floats(gf->nt_gf, gf->n_src, gf->n_rec);
   }
+  // the layout conversions' buffer: the largest of a trace and a CPML array
+  const size_t n1 = (size_t)npml + 1, face = (size_t)std::max(
+      {d->ny * d->nz, d->nx * d->nz, d->nx * d->ny});
+  const size_t stage_floats = std::max((size_t)d->nt * txs->ntx, npml > 0 ? 2 * n1 * face : 0);
+  need += 4 * stage_floats;
   if (need > ctx->budget) return fail(ADF_E_BUDGET, "solve exceeds the context's HBM budget");
+  // Memory comes from the context's pool and goes back to the driver when the
+  // call returns, beyond what stays for the next one.  (Declared before the
+  // solve and the batch, whose memory returns to the pool first.)
+  struct PoolTrim {
+    adf_ctx* c;
+    uint64_t held = 0;
+    explicit PoolTrim(adf_ctx* ctx) : c(ctx) {
+      cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrReservedMemCurrent, &held);
+    }
+    ~PoolTrim() {
+      cudaStreamSynchronize(c->stream);
+      cudaMemPoolTrimTo(c->pool, std::max((size_t)held, kPoolKeep));
+    }
+  } trim(ctx);
   auto s = std::make_unique<Solve>();
+  s->alloc_stream = ctx->stream;
+  s->alloc_pool = ctx->pool;
   const hm::Dom dom = to_dom(*d);
   int rc = solve_alloc(ctx, *s, dom, (int)npml, mask != nullptr, flags, (int)txs->ntx);
-  if (!rc) rc = solve_alloc_traces(*s, true);
+  if (!rc) rc = solve_alloc_traces(*s);
+  float* stage = rc ? nullptr : solve_dalloc<float>(*s, stage_floats, rc);
   if (rc) return rc;
   // Every upload below is a stream-ordered copy on the context stream: the
   // zeroing above, the copies, the set-up kernels and the steps run in that
@@ -1129,30 +1136,32 @@ static int run_fdtd_impl(adf_ctx* ctx, const adf_domain* d, float* field, adf_tx
     if (ue == cudaSuccess && e != cudaSuccess) ue = e;
   };
   // field -> buffer 0 (input of step start_step)
-  up(cudaMemcpy2DAsync(sd.field, (size_t)sd.nxp * 4, field, (size_t)d->nx * 4, (size_t)d->nx * 4,
-                       (size_t)d->ny * d->nz * 4, cudaMemcpyHostToDevice, st));
+  const size_t field_rows = (size_t)d->ny * d->nz * 4;
+  if (sd.nxp == sd.nx)
+    up(cudaMemcpyAsync(sd.field, field, field_rows * sd.nx * 4, cudaMemcpyHostToDevice, st));
+  else
+    up(cudaMemcpy2DAsync(sd.field, (size_t)sd.nxp * 4, field, (size_t)d->nx * 4, (size_t)d->nx * 4,
+                         field_rows, cudaMemcpyHostToDevice, st));
   if (mask) {
     uint8_t* jl = nullptr;
     const size_t mb = (size_t)4 * d->nx * d->ny * d->nz;
-    if (cudaMalloc(&jl, mb) != cudaSuccess) {
+    if (cudaMallocFromPoolAsync((void**)&jl, mb, ctx->pool, st) != cudaSuccess) {
       cudaGetLastError();
       return fail(ADF_E_NOMEM, "mask staging alloc failed");
     }
     up(cudaMemcpyAsync(jl, mask, mb, cudaMemcpyHostToDevice, st));
     up(launch_pack_mask(jl, sd.nx, sd.ny, sd.nz, sd.mw, s->mask_bits, st));
-    up(cudaStreamSynchronize(st));
-    cudaFree(jl);
+    cudaFreeAsync(jl, st);
   }
   if (npml > 0) {
     up(cudaMemcpyAsync(s->coef_dev, cpml->coef, (size_t)(8 * npml + 4) * 4,
                        cudaMemcpyHostToDevice, st));
-    for (int a = 0; a < 3; ++a)
-      for (int b = 0; b < 2; ++b) {
-        if (cpml->mv[a]) up(psi_copy(*s, a, false, cpml->mv[a], true, b, st));
-        if (cpml->mp[a]) up(psi_copy(*s, a, true, cpml->mp[a], true, b, st));
-      }
+    for (int a = 0; a < 3; ++a) {
+      if (cpml->mv[a]) up(psi_copy(*s, a, false, cpml->mv[a], true, 0, stage, st));
+      if (cpml->mp[a]) up(psi_copy(*s, a, true, cpml->mp[a], true, 0, stage, st));
+    }
   }
-  up(upload_traces(*s, txs, st));
+  up(upload_traces(*s, txs, stage, st));
   if (use_gf) {  // GF tensors, 0-based columns, Float64 pin history
     const size_t ng = (size_t)gf->nt_gf * gf->n1 * gf->n2;
     for (int k = 0; k < ntens && !rc; ++k) {
@@ -1324,17 +1333,23 @@ static int run_fdtd_impl(adf_ctx* ctx, const adf_domain* d, float* field, adf_tx
   }
   // output buffer of the last executed step
   const int fb = (int)((stop_step - start_step + 1) & 1);
-  cudaError_t e = cudaMemcpy2D(field, (size_t)d->nx * 4, sd.field + (size_t)fb * sd.buf_stride,
-                               (size_t)sd.nxp * 4, (size_t)d->nx * 4,
-                               (size_t)d->ny * d->nz * 4, cudaMemcpyDeviceToHost);
+  const float* last = sd.field + (size_t)fb * sd.buf_stride;
+  cudaError_t e =
+      sd.nxp == sd.nx
+          ? cudaMemcpyAsync(field, last, field_rows * sd.nx * 4, cudaMemcpyDeviceToHost, st)
+          : cudaMemcpy2DAsync(field, (size_t)d->nx * 4, last, (size_t)sd.nxp * 4, (size_t)d->nx * 4,
+                              field_rows, cudaMemcpyDeviceToHost, st);
   if (npml > 0)
     for (int a = 0; a < 3 && e == cudaSuccess; ++a) {
-      if (cpml->mv[a]) e = psi_copy(*s, a, false, cpml->mv[a], false, fb, st);
-      if (cpml->mp[a] && e == cudaSuccess) e = psi_copy(*s, a, true, cpml->mp[a], false, fb, st);
+      if (cpml->mv[a]) e = psi_copy(*s, a, false, cpml->mv[a], false, fb, stage, st);
+      if (cpml->mp[a] && e == cudaSuccess)
+        e = psi_copy(*s, a, true, cpml->mp[a], false, fb, stage, st);
     }
-  if (e == cudaSuccess) e = download_traces(*s, txs);
-  if (use_gf && e == cudaSuccess) e = download_gf_sources(*s, txs);
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e == cudaSuccess) e = download_traces(*s, txs, use_gf, stage, st);
+  {
+    const cudaError_t es = cudaStreamSynchronize(st);  // also after a failed enqueue
+    if (e == cudaSuccess) e = es;
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(ADF_E_DEVICE, std::string("download: ") + cudaGetErrorString(e));

@@ -95,6 +95,7 @@ struct Batch {
   SolveDev* d_solves = nullptr;
   int4* d_items = nullptr;
   int cap_solves = 0, cap_items = 0;
+  cudaStream_t alloc_stream = nullptr;  // d_solves and d_items come from the context's pool
   int n_items = 0, grid = 1, max_ntx = 0;
   int max_ty = 1;            // tallest tile in the batch: the block is (32, max_ty + 1)
   int max_gf_nsrc = 0;       // > 0: some solve runs the in-loop GF extrapolation
@@ -127,7 +128,7 @@ size_t solve_bytes_estimate(int64_t nx, int64_t ny, int64_t nz, int64_t npml, in
                             int64_t nt, bool mask);
 int solve_alloc(adf_ctx* ctx, Solve& s, const hm::Dom& dom, int npml, bool has_mask, int arith,
                 int ntx);
-int solve_alloc_traces(Solve& s, bool need_vsrc);
+int solve_alloc_traces(Solve& s);
 int solve_finalize(adf_ctx* ctx, Solve& s, const float* const idx[4], const float* const w[4],
                    const int* src_col);
 template <typename T>
