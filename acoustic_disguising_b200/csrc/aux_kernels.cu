@@ -258,15 +258,10 @@ __global__ void adf_gf_prefilter_kernel(int ncol, int n, const float* __restrict
   cf[n + 1] = 2.0 * cf[n] - cf[n - 1];
 }
 
-// Evaluation: one thread per output sample and column; Flat() outside the
-// input axis, times dt_out/dt_in, rounded to Float32, divided by unit32.
-__global__ void adf_gf_resample_kernel(int ncol, int n, int nt_out, double t_in0, double dt_in,
-                                       double t_out0, double dt_out, const double* coef,
-                                       float* out, float unit32) {
-  const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (k >= (long long)nt_out * ncol) return;
-  const int c = (int)(k / nt_out), j = (int)(k - (long long)c * nt_out);
-  const double* cf = coef + (long long)(n + 2) * c;
+// Output sample j of a column with coefficients cf: Flat() outside the input
+// axis, times dt_out/dt_in, rounded to Float32, divided by unit32.
+__device__ __forceinline__ float gf_sample(const double* cf, int n, int j, double t_in0, double dt_in,
+                                           double t_out0, double dt_out, float unit32) {
   const double tt = t_out0 + (double)j * dt_out;
   double x = (tt - t_in0) / dt_in + 1.0;
   x = fmin(fmax(x, 1.0), (double)n);
@@ -277,13 +272,126 @@ __global__ void adf_gf_resample_kernel(int ncol, int n, int nt_out, double t_in0
   const double w1 = (3.0 * d * d * d - 6.0 * d * d + 4.0) / 6.0;
   const double w2 = (-3.0 * d * d * d + 3.0 * d * d + 3.0 * d + 1.0) / 6.0;
   const double v = cf[i - 1] * w0 + cf[i] * w1 + cf[i + 1] * w2 + cf[i + 2] * w3;
-  out[k] = __fdiv_rn((float)(v * (dt_out / dt_in)), unit32);
+  return __fdiv_rn((float)(v * (dt_out / dt_in)), unit32);
 }
 
+// Evaluation: one thread per output sample and column.
+__global__ void adf_gf_resample_kernel(int ncol, int n, int nt_out, double t_in0, double dt_in,
+                                       double t_out0, double dt_out, const double* coef,
+                                       float* out, float unit32) {
+  const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (k >= (long long)nt_out * ncol) return;
+  const int c = (int)(k / nt_out), j = (int)(k - (long long)c * nt_out);
+  out[k] = gf_sample(coef + (long long)(n + 2) * c, n, j, t_in0, dt_in, t_out0, dt_out, unit32);
+}
+
+// The same for columns that fit a block's shared memory, prefilter and evaluation
+// in one kernel, one block per column: the samples are read once and the
+// coefficients never leave the SM.  The tridiagonal recurrences forget by
+// 2 - sqrt(3) per sample, so every thread solves its own stretch of the column
+// and starts each sweep kGfWarm samples outside it: 0.268^64 = 2e-37 of the
+// neighbouring values is left of the start, far below Float64's last place.  (A
+// column with a sample that is not finite is swept by one thread, which spreads
+// it as the sequential recurrence does.)  The Thomas division by 4 - cpv[i-1] is
+// a product with cpv[i], its reciprocal.  2000 -> 700 samples x 4096 columns:
+// 1.25 ms as two kernels with a thread per column, whose 66 MB of coefficients
+// were written and read at a stride of a column; 0.19 ms here, bound by the
+// instructions of the sweeps (half the issue slots).
+constexpr int kGfWarm = 64;
+constexpr int kGfThreads = 128;
+constexpr int kGfPivots = 48;  // the pivots are constant to the last place from here on
+size_t gf_fused_smem(long long n) { return (size_t)(8 * (n + 2) + 8 * (n + 1) + 4 * n); }
+
+__global__ void __launch_bounds__(kGfThreads) adf_gf_postprocess_kernel(
+    int n, int nt_out, double t_in0, double dt_in, double t_out0, double dt_out,
+    const float* __restrict__ in, const double* __restrict__ cpv, float* __restrict__ out,
+    float unit32, int denoise) {
+  extern __shared__ __align__(16) double smem_d[];
+  double* const cf = smem_d;               // coefficients 0 .. n+1
+  double* const fw = smem_d + n + 2;       // forward sweep, 1-based
+  float* const y = reinterpret_cast<float*>(fw + n + 1);
+  __shared__ float s_max[kGfThreads / 32];
+  const int tid = threadIdx.x;
+  const float* a = in + (long long)blockIdx.x * n;
+  float mx = __int_as_float(0xff800000);
+  bool fine = true;
+  for (int t = tid; t < n; t += kGfThreads) {
+    const float v = a[t];
+    y[t] = v;
+    mx = fmaxf(mx, v);
+    fine = fine && isfinite(v);
+  }
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((tid & 31) == 0) s_max[tid >> 5] = mx;
+  fine = __syncthreads_and(fine);
+  for (int w = 0; w < kGfThreads / 32; ++w) mx = fmaxf(mx, s_max[w]);
+  const double thr = 1e-4 * (double)mx;
+  auto at = [&](int i) {  // 1-based sample, denoised
+    const float v = y[i - 1];
+    return (denoise && (double)fabsf(v) < thr) ? 0.0 : (double)v;
+  };
+  const double c_inf = cpv[min(kGfPivots, n - 1)];
+  auto piv = [&](int i) { return i < kGfPivots ? __ldg(cpv + i) : c_inf; };
+  // this thread's stretch [lo, hi) of the unknowns 2 .. n-1 (of odd length, so that
+  // the lanes' samples lie on different banks)
+  const int per = fine ? (n - 2 + kGfThreads - 1) / kGfThreads | 1 : n - 2;
+  const int lo = min(2 + tid * per, n), hi = min(lo + per, n);
+  const double first = at(1), last = at(n);
+  if (lo < hi) {
+    const int from = fine ? max(2, lo - kGfWarm) : 2;
+    double d = 0.0;
+    for (int i = from; i < hi; ++i) {
+      double rhs = 6.0 * at(i);
+      if (i == 2) rhs -= first;
+      if (i == n - 1) rhs -= last;
+      d = (rhs - d) * piv(i);
+      if (i >= lo) fw[i] = d;
+    }
+  }
+  __syncthreads();
+  if (lo < hi) {
+    const int from = fine ? min(n - 1, hi - 1 + kGfWarm) : n - 1;
+    double c = 0.0;
+    for (int i = from; i >= lo; --i) {
+      c = i == n - 1 ? fw[i] : fw[i] - piv(i) * c;
+      if (i < hi) cf[i] = c;
+    }
+  }
+  if (tid == 0) {
+    cf[1] = first;
+    cf[n] = last;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    cf[0] = 2.0 * cf[1] - cf[2];
+    cf[n + 1] = 2.0 * cf[n] - cf[n - 1];
+  }
+  __syncthreads();
+  for (int j = tid; j < nt_out; j += kGfThreads)
+    out[(long long)blockIdx.x * nt_out + j] =
+        gf_sample(cf, n, j, t_in0, dt_in, t_out0, dt_out, unit32);
+}
+
+// Scratch doubles per column that launch_gf_postprocess needs: none where the
+// fused kernel takes the call.
+size_t gf_postprocess_scratch(int n, size_t smem_cap) {
+  return gf_fused_smem(n) + 256 <= smem_cap ? 0 : (size_t)n + 2;
+}
+
+// (coef NULL: the fused kernel)
 cudaError_t launch_gf_postprocess(int ncol, int n, int nt_out, double t_in0, double dt_in,
                                   double t_out0, double dt_out, const float* in,
                                   const double* cpv, double* coef, float* out, float unit32,
                                   int denoise, cudaStream_t s) {
+  if (!coef) {
+    const size_t smem = gf_fused_smem(n);
+    const cudaError_t fe = cudaFuncSetAttribute(
+        (const void*)adf_gf_postprocess_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (fe != cudaSuccess) return fe;
+    adf_gf_postprocess_kernel<<<ncol, kGfThreads, smem, s>>>(n, nt_out, t_in0, dt_in, t_out0, dt_out,
+                                                            in, cpv, out, unit32, denoise);
+    return cudaGetLastError();
+  }
   adf_gf_prefilter_kernel<<<(ncol + 127) / 128, 128, 0, s>>>(ncol, n, in, cpv, coef, denoise);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;

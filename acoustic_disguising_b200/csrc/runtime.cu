@@ -38,6 +38,7 @@ cudaError_t launch_gf_postprocess(int ncol, int n, int nt_out, double t_in0, dou
                                   double t_out0, double dt_out, const float* in,
                                   const double* cpv, double* coef, float* out, float unit32,
                                   int denoise, cudaStream_t s);
+size_t gf_postprocess_scratch(int n, size_t smem_cap);
 int static_cpml_max_npml();
 cudaError_t static_cpml_scratch(double** d64, float** d32);
 
@@ -803,6 +804,17 @@ static cudaError_t psi_copy(Solve& s, int axis, bool vside, float* host, bool up
 // The context's pool after a run that took its memory from it: back to what it
 // held before, or to this much where that is less.
 constexpr size_t kPoolKeep = (size_t)1 << 30;
+struct PoolTrim {
+  adf_ctx* c;
+  uint64_t held = 0;
+  explicit PoolTrim(adf_ctx* ctx) : c(ctx) {
+    cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrReservedMemCurrent, &held);
+  }
+  ~PoolTrim() {
+    cudaStreamSynchronize(c->stream);
+    cudaMemPoolTrimTo(c->pool, std::max((size_t)held, kPoolKeep));
+  }
+};
 
 // ---------------------------------------------------------------------------
 // C-ABI
@@ -1104,20 +1116,7 @@ static int run_fdtd_impl(adf_ctx* ctx, const adf_domain* d, float* field, adf_tx
   const size_t stage_floats = std::max((size_t)d->nt * txs->ntx, npml > 0 ? 2 * n1 * face : 0);
   need += 4 * stage_floats;
   if (need > ctx->budget) return fail(ADF_E_BUDGET, "solve exceeds the context's HBM budget");
-  // Memory comes from the context's pool and goes back to the driver when the
-  // call returns, beyond what stays for the next one.  (Declared before the
-  // solve and the batch, whose memory returns to the pool first.)
-  struct PoolTrim {
-    adf_ctx* c;
-    uint64_t held = 0;
-    explicit PoolTrim(adf_ctx* ctx) : c(ctx) {
-      cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrReservedMemCurrent, &held);
-    }
-    ~PoolTrim() {
-      cudaStreamSynchronize(c->stream);
-      cudaMemPoolTrimTo(c->pool, std::max((size_t)held, kPoolKeep));
-    }
-  } trim(ctx);
+  PoolTrim trim(ctx);  // (before the solve and the batch, which return their memory first)
   auto s = std::make_unique<Solve>();
   s->alloc_stream = ctx->stream;
   s->alloc_pool = ctx->pool;
@@ -1470,25 +1469,18 @@ int adf_gf_postprocess(adf_ctx* ctx, int64_t ncol, int64_t nt_in, double t_in0, 
   const int n = (int)nt_in;
   std::vector<double> cpv((size_t)n + 1, 0.0);  // Thomas pivots of (1, 4, 1)
   for (int i = 2; i <= n - 1; ++i) cpv[(size_t)i] = 1.0 / (4.0 - (i > 2 ? cpv[(size_t)i - 1] : 0.0));
-  float* din = nullptr;
-  float* dout = nullptr;
-  double* dcoef = nullptr;
-  double* dcp = nullptr;
-  auto release = [&]() {
-    cudaFree(din);
-    cudaFree(dout);
-    cudaFree(dcoef);
-    cudaFree(dcp);
-  };
-  if (cudaMalloc(&din, (size_t)4 * n * ncol) != cudaSuccess ||
-      cudaMalloc(&dout, (size_t)4 * nt_out * ncol) != cudaSuccess ||
-      cudaMalloc(&dcoef, (size_t)8 * (n + 2) * ncol) != cudaSuccess ||
-      cudaMalloc(&dcp, (size_t)8 * (n + 1)) != cudaSuccess) {
-    release();
-    cudaGetLastError();
-    return fail(ADF_E_NOMEM, "adf_gf_postprocess: device allocation failed");
-  }
   cudaStream_t st = ctx->stream;
+  PoolTrim trim(ctx);
+  Solve mem;  // holds the call's device memory
+  mem.alloc_stream = st;
+  mem.alloc_pool = ctx->pool;
+  int rc = ADF_OK;
+  const size_t scratch = gf_postprocess_scratch(n, (size_t)ctx->smem_optin) * (size_t)ncol;
+  float* din = solve_dalloc<float>(mem, (size_t)n * ncol, rc);
+  float* dout = rc ? nullptr : solve_dalloc<float>(mem, (size_t)nt_out * ncol, rc);
+  double* dcoef = rc || !scratch ? nullptr : solve_dalloc<double>(mem, scratch, rc);
+  double* dcp = rc ? nullptr : solve_dalloc<double>(mem, (size_t)n + 1, rc);
+  if (rc) return fail(ADF_E_NOMEM, "adf_gf_postprocess: device allocation failed");
   cudaMemcpyAsync(din, in, (size_t)4 * n * ncol, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(dcp, cpv.data(), (size_t)8 * (n + 1), cudaMemcpyHostToDevice, st);
   cudaEventRecord(ctx->ev0, st);
@@ -1500,10 +1492,9 @@ int adf_gf_postprocess(adf_ctx* ctx, int64_t ncol, int64_t nt_in, double t_in0, 
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   float ms = 0.f;
   if (e == cudaSuccess) cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  release();
   if (e != cudaSuccess) return fail(ADF_E_DEVICE, cudaGetErrorString(e));
   ctx->last_ms = ms;
-  ctx->launches = 2;
+  ctx->launches = scratch ? 2 : 1;
   ctx->h2d_bytes = (int64_t)4 * n * ncol;
   ctx->d2h_bytes = (int64_t)4 * nt_out * ncol;
   return ADF_OK;

@@ -88,3 +88,33 @@ def test_impulsive_gfs_pipeline(adf, oracle, ctx):
                 want = R[:, cols].astype(np.float64)
                 assert np.abs(want).max() > 0
                 assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want), (i, typ, ch)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [4, 5, 47, 48, 49, 50, 130, 131, 259, 2000, 11600, 11700])
+def test_gf_postprocess_stretches(adf, oracle, ctx, n):
+    """The prefilter solved in stretches of a column: fewer samples than
+    threads, the first pivots' end, one sample more or less than whole
+    stretches, and both sides of the longest column the fused kernel holds
+    (232448 B of shared memory: 20 n + 24 + 256 <= 232448, n <= 11608).  Noise at full amplitude,
+    so that every coefficient depends on its neighbours; the Float32 result
+    is within an ulp or two of the oracle's (1e-6 in the 2-norm)."""
+    rng = np.random.default_rng(n)
+    a = np.asfortranarray(rng.standard_normal((n, 3)), np.float32)
+    nt_out = max(3, n // 3)
+    out = adf.gf_postprocess(a, 0.0, 1.0, nt_out, -1.5, 3.1, unit=2.5, denoise=False)
+    ref = oracle.gf_postprocess(a, 0.0, 1.0, nt_out, -1.5, 3.1, unit=2.5, denoise=False)
+    assert np.linalg.norm(out.astype(np.float64) - ref) <= 1e-6 * np.linalg.norm(ref)
+
+
+@pytest.mark.gpu
+def test_gf_postprocess_not_finite(adf, oracle, ctx):
+    """A NaN or an infinity spreads over its column as in the sequential sweep
+    and leaves the others alone."""
+    a = traces(nt=600, ncol=4)
+    a[300, 1] = np.nan
+    a[5, 2] = np.inf
+    out = adf.gf_postprocess(a, 0.0, 1.0, 250, 0.0, 2.3, denoise=False)
+    ref = oracle.gf_postprocess(a, 0.0, 1.0, 250, 0.0, 2.3, denoise=False)
+    assert np.array_equal(np.isfinite(out), np.isfinite(ref))
+    assert np.isfinite(out[:, [0, 3]]).all()
