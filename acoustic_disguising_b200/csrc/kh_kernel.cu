@@ -57,25 +57,24 @@ namespace {
 constexpr int KH_WARPS = KH_NWARPS;
 constexpr int KH_THREADS = 32 * KH_WARPS;
 constexpr int KH_RW = KH_NRW;            // targets per warp
-constexpr int KH_G = KH_NG;              // surface points summed before each compensated add
+constexpr int KH_G = KH_NG;              // surface points summed before each compensated add (one part)
 constexpr int KH_RT = KH_WARPS * KH_RW;  // targets per CTA
 constexpr int KH_SC_MAX = 32;            // surface points per staged chunk
-// Output samples per lane, T, is a template parameter: 17 (128 registers)
-// costs about 8 % less per sample than 13 (112 registers) on long traces, but
-// its CTAs cover 544 samples against 416, so short traces pad more.  The
-// launcher takes the one with the smaller padded cost.
-constexpr int KH_T_LONG = 17, KH_T_SHORT = 13;
-constexpr double KH_T_LONG_COST = 0.917;  // per-sample cost of 17 relative to 13
-
-int kh_samples_per_lane(int nt) {
-  const double c17 = KH_T_LONG_COST * (double)((nt + 32 * KH_T_LONG - 1) / (32 * KH_T_LONG)) *
-                     (32 * KH_T_LONG);
-  const double c13 = (double)((nt + 32 * KH_T_SHORT - 1) / (32 * KH_T_SHORT)) * (32 * KH_T_SHORT);
-  return c17 < c13 ? KH_T_LONG : KH_T_SHORT;
-}
+// Output samples per lane, T, is a template parameter: a CTA covers 32 T samples,
+// and a longer T costs less per sample (kKhT).  The launcher covers the trace
+// with blocks of the longest and, where that pads less, a last block of a
+// shorter one.
+struct KhT {
+  int T;
+  double cost;  // of a block, relative to T = 17
+};
+constexpr KhT kKhT[3] = {{17, 1.0}, {13, 0.811}, {7, 0.492}};  // measured, 592 CTAs x 1024 points
 
 struct KhParams {
   int ns, nr, nt;
+  int t_base;       // first output sample of this launch
+  int splits;       // parts of the surface, one per blockIdx.z
+  int group;        // points summed before each compensated add, a power of two
   int sc;           // surface points per chunk
   int rowpad;       // staged floats per channel and surface point (multiple of 4)
   int pad;          // zero samples in front of each padded input column
@@ -97,6 +96,7 @@ struct KhParams {
                         // the pair of sample t at 2 (pad + t)
   const float* cs_f;    // running sum of in_f, same layout (velocity output)
   float* out;           // (nt, nr)
+  float2* part;         // splits > 1: [splits][nr][nt] {sum, compensation} instead
   int* err;
   unsigned wait_limit;  // polls of a chunk's bounded wait (kWaitLimit)
   int skip_chunk;       // test hook: chunk whose copies are not issued (-1: none)
@@ -117,7 +117,10 @@ __global__ void __launch_bounds__(KH_THREADS, 1) adf_kh_pressure_kernel(KhParams
   __shared__ int s_abort;  // a chunk's bounded wait gave up
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tile = blockIdx.x;
-  const int tb = blockIdx.y * (32 * T);
+  const int tb = p.t_base + blockIdx.y * (32 * T);
+  // this CTA's part of the surface
+  const int s_lo = (int)((long long)p.ns * blockIdx.z / p.splits);
+  const int s_hi = (int)((long long)p.ns * (blockIdx.z + 1) / p.splits);
   const int r_base = tile * KH_RT;
   const int2 lob = p.tile_lo[tile];
   const int lo_min = lob.x, lo_max = lob.y;
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(KH_THREADS, 1) adf_kh_pressure_kernel(KhParams
   float* taps = par0 + 2 * NPAR * npair;
   float* my_taps = taps + warp * (KH_RW * 2 * LM);
 
-  const int nchunks = (p.ns + p.sc - 1) / p.sc;
+  const int nchunks = (s_hi - s_lo + p.sc - 1) / p.sc;
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&full[0]), 1);
     mbar_init(smem_u32(&full[1]), 1);
@@ -150,8 +153,8 @@ __global__ void __launch_bounds__(KH_THREADS, 1) adf_kh_pressure_kernel(KhParams
 
   // bulk copies of chunk c (one thread)
   auto stage = [&](int c) {
-    const int s0 = c * p.sc;
-    const int nsc = min(p.sc, p.ns - s0);
+    const int s0 = s_lo + c * p.sc;
+    const int nsc = min(p.sc, s_hi - s0);
     const uint32_t mb = smem_u32(&full[c & 1]);
     const uint32_t row_bytes = (uint32_t)p.rowpad * 4u;
     // the buffer's previous contents were read through the generic proxy
@@ -170,8 +173,8 @@ __global__ void __launch_bounds__(KH_THREADS, 1) adf_kh_pressure_kernel(KhParams
   };
   // pair geometry of chunk c in FP64 (all threads)
   auto params = [&](int c) {
-    const int s0 = c * p.sc;
-    const int nsc = min(p.sc, p.ns - s0);
+    const int s0 = s_lo + c * p.sc;
+    const int nsc = min(p.sc, s_hi - s0);
     float* pb = par0 + (c & 1) * NPAR * npair;
     int* pr_lo = reinterpret_cast<int*>(pb);
     int* pr_n = pr_lo + npair;
@@ -263,7 +266,7 @@ __global__ void __launch_bounds__(KH_THREADS, 1) adf_kh_pressure_kernel(KhParams
       s_abort = 1;  // read by every thread after the barrier below
       ok = false;
     }
-    const int nsc = min(p.sc, p.ns - c * p.sc);
+    const int nsc = min(p.sc, s_hi - s_lo - c * p.sc);
     const float* win = smem + (c & 1) * wbuf;
     const float* pb = par0 + (c & 1) * NPAR * npair;
     const int* pr_lo = reinterpret_cast<const int*>(pb);
@@ -334,7 +337,7 @@ __global__ void __launch_bounds__(KH_THREADS, 1) adf_kh_pressure_kernel(KhParams
         }
       }
       // compensated accumulation over groups of surface points
-      if (sl % KH_G == KH_G - 1 || sl == nsc - 1) {
+      if (((sl + 1) & (p.group - 1)) == 0 || sl == nsc - 1) {
 #pragma unroll
         for (int rho = 0; rho < KH_RW; ++rho)
 #pragma unroll
@@ -370,10 +373,32 @@ __global__ void __launch_bounds__(KH_THREADS, 1) adf_kh_pressure_kernel(KhParams
     if (r >= p.nr) continue;
     const int t0 = tb + T * lane;
     float* o = p.out + (size_t)r * p.nt + t0;
+    float2* q = p.part + ((size_t)blockIdx.z * p.nr + r) * p.nt + t0;
 #pragma unroll
-    for (int j = 0; j < T; ++j)
-      if (t0 + j < p.nt) o[j] = sum[rho][j];
+    for (int j = 0; j < T; ++j) {
+      if (t0 + j >= p.nt) continue;
+      if (p.splits == 1)
+        o[j] = sum[rho][j];
+      else
+        q[j] = make_float2(sum[rho][j], comp[rho][j]);
+    }
   }
+}
+
+// Adds the surface parts of output samples t0 .. t1-1, in part order, in Float64.
+__global__ void adf_kh_combine_kernel(const float2* __restrict__ part, float* __restrict__ out,
+                                      int nr, int nt, int t0, int t1, int splits) {
+  const long long n = (long long)nr * nt;
+  for (int r = blockIdx.x; r < nr; r += gridDim.x)
+    for (int t = t0 + (int)threadIdx.x; t < t1; t += blockDim.x) {
+      const long long i = (long long)r * nt + t;
+      double a = 0.0;
+      for (int z = 0; z < splits; ++z) {
+        const float2 v = part[z * n + i];
+        a += (double)v.x - (double)v.y;
+      }
+      out[i] = (float)a;
+    }
 }
 
 // FP32 FMA throughput probe: 8 independent chains per thread, enough warps
@@ -479,6 +504,29 @@ __global__ void adf_kh_gather_kernel(const float* q, const float* f, int ntx, in
   }
 }
 
+// Parts of the surface for a launch of `ctas` CTAs over `samples` of the trace.
+// One CTA per SM runs at a time, so a call with few targets leaves SMs idle and a
+// middling one a last wave that is nearly empty; each part repeats a CTA's start
+// (about two surface points' time) and costs one pass over its share of the
+// partial sums.  Estimated in us from the measured time of a surface point.
+// 200 points -> 48 targets x 700 samples: 283 us in one part, 49 in 16 or more;
+// 2048 -> 4096 x 500: 6.95 and 6.16 ms.
+static int kh_splits(int nsm, long long ctas, int ns, int nr, int samples, double point_us) {
+  int best = 1;
+  double best_us = 1e300;
+  for (int s = 1; s <= 32 && ns / s >= (s > 1 ? KH_G : 1); ++s) {
+    const double bytes = 16.0 * s * samples * nr;  // written and read once
+    if (s > 1 && bytes > 512e6) break;
+    const double us = std::ceil((double)ctas * s / nsm) * ((double)ns / s + 2.0) * point_us +
+                      (s > 1 ? 4.0 + bytes / 5e6 : 0.0);
+    if (us < 0.98 * best_us) {
+      best = s;
+      best_us = us;
+    }
+  }
+  return best;
+}
+
 // in_q / in_f either host arrays (nt, ns) or, with `dev`, columns of
 // device-resident traces (pressure only).
 static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const float* in_f,
@@ -523,10 +571,26 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
   }
   rs = rs * (1 + 1e-12) + 1e-12;
   const double inv_c0dt = 1.0 / (d->c0 * d->dt);
-  const int T = kh_samples_per_lane(nt), TB = 32 * T;  // output samples per lane, per CTA
+  // Time blocks: whole blocks of the longest T, and a last one of the shortest
+  // that holds the rest (2048 samples: 3 x 544 + 416, none padded)
+  struct Launch {
+    int t, nb, t_base;  // kKhT index, blocks, first sample
+    int rowpad, sc, splits;
+    size_t smem;
+  };
+  std::vector<Launch> runs;
+  {
+    const int tb0 = 32 * kKhT[0].T;
+    int whole = nt / tb0, rest = nt - whole * tb0, last = 0;
+    for (int t = 1; t < 3; ++t)
+      if (rest <= 32 * kKhT[t].T) last = t;
+    if (rest > 0 && last == 0) ++whole;
+    if (whole > 0) runs.push_back({0, whole, 0, 0, 0, 1, 0});
+    if (rest > 0 && last > 0) runs.push_back({last, 1, nt - rest, 0, 0, 1, 0});
+  }
   const int ntiles = (nr + KH_RT - 1) / KH_RT;
   std::vector<int2> tlo((size_t)ntiles);
-  int wmax = 0, lo_all = 0;
+  int spread = 0, lo_all = 0;  // largest lo_max - lo_min of a tile, largest lo_max
   for (int t = 0; t < ntiles; ++t) {
     double dmin = 1e300, dmax = 0;
     for (int r = t * KH_RT; r < std::min(nr, (t + 1) * KH_RT); ++r) {
@@ -541,41 +605,54 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
     int lo_max = (int)std::max(0.0, std::min(lmax, (double)nt + 1));
     lo_min = std::min(lo_min, lo_max);
     tlo[(size_t)t] = make_int2(lo_min, lo_max);
-    wmax = std::max(wmax, TB + (lo_max - lo_min) + lm - 1);
+    spread = std::max(spread, lo_max - lo_min);
     lo_all = std::max(lo_all, lo_max);
   }
   // multiple of 4 floats so the tap buffer behind the rows stays 16-B aligned
   // A staged row starts up to 3 samples early (16-B aligned source) and is a
   // multiple of 4 floats, so every bulk copy and the tap buffer stay aligned.
-  const int rowpad = (wmax + 3 + 3) / 4 * 4;
   const size_t tap_bytes = (size_t)KH_WARPS * KH_RW * 2 * lm * 4;
   const int nrow = kind ? 3 : 2;  // staged rows per surface point
-  // double-buffered windows and pair parameters (lo, n, wb, 5 coefficients)
-  const size_t per_s = 2 * ((size_t)nrow * rowpad * 4 + (size_t)8 * KH_RT * 4);
   const size_t smem_cap = (size_t)ctx->smem_optin - 256;  // static mbarriers
-  int sc = KH_SC_MAX;
-  while (sc > 1 && per_s * sc + tap_bytes > smem_cap) --sc;
-  const size_t smem = per_s * sc + tap_bytes;
+  long long t_end = 0;  // samples that the blocks cover
+  for (Launch& l : runs) {
+    const int tb = 32 * kKhT[l.t].T, wmax = tb + spread + lm - 1;
+    l.rowpad = (wmax + 3 + 3) / 4 * 4;
+    // double-buffered windows and pair parameters (lo, n, wb, 5 coefficients)
+    const size_t per_s = 2 * ((size_t)nrow * l.rowpad * 4 + (size_t)8 * KH_RT * 4);
+    l.sc = KH_SC_MAX;
+    while (l.sc > 1 && per_s * l.sc + tap_bytes > smem_cap) --l.sc;
+    l.smem = per_s * l.sc + tap_bytes;
+    if (l.smem > smem_cap)
+      return fail(ADF_E_ARG, "adf_kh_pressure: the targets' delay spread needs a " +
+                                 std::to_string(wmax) + "-sample window, more than shared memory holds");
+    t_end = std::max(t_end, (long long)l.t_base + (long long)l.nb * tb);
+  }
   // Input columns are zero-padded so that every staged window lies inside
   // its column: pad zeros before sample 0 cover the earliest window start,
   // the tail covers the last time block's window end.
-  const int nblk = (nt + TB - 1) / TB;
   const int pad = (lo_all + lm + 4 + 3) / 4 * 4;
-  const long long pitch = ((long long)pad + (long long)nblk * TB + lo_all + 16 + 3) / 4 * 4;
-  if (smem > smem_cap)
-    return fail(ADF_E_ARG, "adf_kh_pressure: the targets' delay spread needs a " +
-                               std::to_string(wmax) + "-sample window, more than shared memory holds");
+  const long long pitch = ((long long)pad + t_end + lo_all + 16 + 3) / 4 * 4;
+  int splits = 1;  // the most of any launch
+  for (Launch& l : runs) {
+    if (ctx->kh_skip_chunk < 0)
+      l.splits = kh_splits(ctx->nsm, (long long)ntiles * l.nb, ns, nr, std::min(nt - l.t_base, l.nb * 32 * kKhT[l.t].T),
+                           1.7 * kKhT[l.t].cost * lm / 16.0);
+    splits = std::max(splits, l.splits);
+  }
 
   // scratch from the context's pool: after the first call of a size the
   // memory stays mapped and later calls take it without driver allocations
   DevBuf<double> dsp(ctx), dsn(ctx), drp(ctx), drn(ctx);
   DevBuf<float> dq(ctx), df(ctx), dqf(ctx), dc(ctx), dout(ctx);
+  DevBuf<float2> dpart(ctx);
   DevBuf<int2> dtlo(ctx);
   DevBuf<int> derr(ctx);
   if (!dsp.alloc((size_t)3 * ns) || !dsn.alloc((size_t)3 * ns) || !drp.alloc((size_t)3 * nr) ||
       !dq.alloc((size_t)pitch * ns) || !df.alloc((size_t)pitch * ns) ||
       !dqf.alloc((size_t)2 * pitch * ns) ||
       !dout.alloc((size_t)nt * nr) ||
+      (splits > 1 && !dpart.alloc((size_t)splits * nt * nr)) ||
       !dtlo.alloc((size_t)ntiles) || !derr.alloc(1) ||
       (kind && (!drn.alloc((size_t)3 * nr) || !dc.alloc((size_t)pitch * ns))))
     return fail(ADF_E_NOMEM, "adf_kh_pressure: device allocation failed");
@@ -620,7 +697,6 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
 
   KhParams p;
   p.ns = ns; p.nr = nr; p.nt = nt;
-  p.sc = sc; p.rowpad = rowpad;
   p.pad = pad; p.pitch = pitch;
   p.inv_c0dt = inv_c0dt;
   p.hw = hw;
@@ -636,7 +712,7 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
   p.dt_sigma = (float)(d->dt / d->sigma);
   p.sp = dsp.p; p.sn = dsn.p; p.rp = drp.p; p.rn = drn.p;
   p.tile_lo = dtlo.p;
-  p.in_qf = dqf.p; p.cs_f = dc.p; p.out = dout.p;
+  p.in_qf = dqf.p; p.cs_f = dc.p; p.out = dout.p; p.part = dpart.p;
   p.err = derr.p;
   // the one-shot test hook of adf_kh_test_fault
   p.wait_limit = ctx->kh_wait_limit ? ctx->kh_wait_limit : kWaitLimit;
@@ -648,21 +724,36 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
   using KhFn = void (*)(KhParams);
   // (taps past the window are zero, so a wider instantiation gives the same
   // sums with more FMAs: the narrowest that holds the window is taken)
-  static const KhFn kfn[3][2][2] = {
-      {{adf_kh_pressure_kernel<16, 0, KH_T_SHORT>, adf_kh_pressure_kernel<16, 0, KH_T_LONG>},
-       {adf_kh_pressure_kernel<16, 1, KH_T_SHORT>, adf_kh_pressure_kernel<16, 1, KH_T_LONG>}},
-      {{adf_kh_pressure_kernel<24, 0, KH_T_SHORT>, adf_kh_pressure_kernel<24, 0, KH_T_LONG>},
-       {adf_kh_pressure_kernel<24, 1, KH_T_SHORT>, adf_kh_pressure_kernel<24, 1, KH_T_LONG>}},
-      {{adf_kh_pressure_kernel<32, 0, KH_T_SHORT>, adf_kh_pressure_kernel<32, 0, KH_T_LONG>},
-       {adf_kh_pressure_kernel<32, 1, KH_T_SHORT>, adf_kh_pressure_kernel<32, 1, KH_T_LONG>}}};
-  const KhFn fn = kfn[lm == 16 ? 0 : (lm == 24 ? 1 : 2)][kind ? 1 : 0][T == KH_T_LONG ? 1 : 0];
-  e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return fail(ADF_E_DEVICE, std::string("kh smem: ") + cudaGetErrorString(e));
-  const dim3 grid((unsigned)ntiles, (unsigned)((nt + TB - 1) / TB));
+#define ADF_KH(lm, kind)                                                             \
+  {adf_kh_pressure_kernel<lm, kind, kKhT[0].T>, adf_kh_pressure_kernel<lm, kind, kKhT[1].T>, \
+   adf_kh_pressure_kernel<lm, kind, kKhT[2].T>}
+  const KhFn kfn[3][2][3] = {{ADF_KH(16, 0), ADF_KH(16, 1)},
+                                    {ADF_KH(24, 0), ADF_KH(24, 1)},
+                                    {ADF_KH(32, 0), ADF_KH(32, 1)}};
+#undef ADF_KH
+  int64_t launches = 0;
   cudaEventRecord(ctx->ev0, st);
-  fn<<<grid, KH_THREADS, smem, st>>>(p);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return fail(ADF_E_DEVICE, std::string("kh launch: ") + cudaGetErrorString(e));
+  for (const Launch& l : runs) {
+    const KhFn fn = kfn[lm == 16 ? 0 : (lm == 24 ? 1 : 2)][kind ? 1 : 0][l.t];
+    e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
+    if (e != cudaSuccess) return fail(ADF_E_DEVICE, std::string("kh smem: ") + cudaGetErrorString(e));
+    p.t_base = l.t_base;
+    p.splits = l.splits;
+    // (parts sum their points in another order than one pass does: groups half as
+    // long keep their error below its, at 1 % of the time)
+    p.group = l.splits > 1 ? KH_G / 2 : KH_G;
+    p.sc = l.sc;
+    p.rowpad = l.rowpad;
+    fn<<<dim3((unsigned)ntiles, (unsigned)l.nb, (unsigned)l.splits), KH_THREADS, l.smem, st>>>(p);
+    e = cudaGetLastError();
+    if (e == cudaSuccess && l.splits > 1) {
+      adf_kh_combine_kernel<<<std::min(nr, ctx->nsm * 8), 256, 0, st>>>(
+          dpart.p, dout.p, nr, nt, l.t_base, std::min(nt, l.t_base + l.nb * 32 * kKhT[l.t].T), l.splits);
+      e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) return fail(ADF_E_DEVICE, std::string("kh launch: ") + cudaGetErrorString(e));
+    launches += l.splits > 1 ? 2 : 1;
+  }
   cudaEventRecord(ctx->ev1, st);
   int herr = 0;
   cudaMemcpyAsync(out, dout.p, (size_t)4 * nt * nr, cudaMemcpyDeviceToHost, st);
@@ -674,7 +765,7 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
   ctx->last_ms = ms;
   ctx->kh_ms = ms;
-  ctx->launches = 1;
+  ctx->launches = launches;
   ctx->h2d_bytes = (int64_t)48 * ns + (kind ? 48 : 24) * (int64_t)nr +
                    (dev ? 0 : (int64_t)(kind ? 12 : 8) * nt * ns);
   ctx->d2h_bytes = (int64_t)4 * nt * nr;

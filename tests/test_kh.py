@@ -171,3 +171,25 @@ def test_kh_bounded_wait_ends_in_an_error_code(adf, oracle, ctx, skip):
     assert ei.value.code == -6, ei.value
     out, ref = run_pair(adf, oracle, c)  # the hook is one-shot
     assert rel_l2(out, ref) <= RTOL_L2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ns,nr,nt", [
+    (9, 17, 545),     # too few points to part; a second block of one sample
+    (16, 5, 544),     # two parts of eight points, one whole block
+    (37, 33, 768),    # 544 + 224: the shortest block, full
+    (37, 33, 769),    # 544 + 225: one sample more, the middle block
+    (100, 16, 960),   # 544 + 416
+    (100, 16, 961),   # two long blocks
+    (300, 20, 200),   # the shortest block alone, the surface in many parts
+])
+def test_kh_parts_and_time_blocks(adf, oracle, ctx, ns, nr, nt):
+    """The surface summed in parts and the trace covered by blocks of different
+    length: every sample written once, each part's points counted once, at the
+    accuracy of the one-part sum."""
+    c = case(ns, nr, nt, 5e-6, 0.25, 0.35)
+    out, ref = run_pair(adf, oracle, c)
+    assert np.abs(ref).max() > 0
+    assert rel_l2(out, ref) <= 1e-6
+    if nt > 544:
+        assert np.abs(ref[544:]).max() > 0 and rel_l2(out[544:], ref[544:]) <= 1e-6
