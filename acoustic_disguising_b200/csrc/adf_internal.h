@@ -125,7 +125,9 @@ struct EpiParams {
 
 // launch helpers implemented in fdtd_kernels.cu
 // one CTA per work item, blockDim (32, max_ty + 1); max_ty <= step_max_ty()
-cudaError_t launch_step(const StepParams& p, int grid, int max_ty, cudaStream_t s);
+// `overlap`: the kernel may start while the one before it in the stream runs
+// (programmatic dependent launch); not after anything that writes the descriptors
+cudaError_t launch_step(const StepParams& p, int grid, int max_ty, bool overlap, cudaStream_t s);
 // layout conversions of a call's arrays (runtime.cu): src[c][r] -> dst[r][c] over
 // cols x rows, and rows of `width` floats from one pitch to another
 cudaError_t launch_transpose(const float* src, float* dst, int rows, int cols, cudaStream_t s);
@@ -136,9 +138,9 @@ cudaError_t launch_mask_tiles(const SolveDev& d, unsigned char* closed, cudaStre
 int step_max_ty();
 int step_x_tile();  // cells per x tile of a step work item
 cudaError_t step_ctas_per_sm(int* n);  // resident step-kernel CTAs per SM (occupancy)
-cudaError_t launch_epilogue(const EpiParams& p, int max_ntx, cudaStream_t s);
+cudaError_t launch_epilogue(const EpiParams& p, int max_ntx, bool overlap, cudaStream_t s);
 cudaError_t launch_gf_extrapolate(const EpiParams& p, int max_blocks, int max_nsrc, bool reduce,
-                                  cudaStream_t s);
+                                  bool overlap, cudaStream_t s);
 // far-lag part of the in-loop GF extrapolation for the block of kGfBlock steps
 // that starts at launch-step p.step
 cudaError_t launch_gf_near_pack(const SolveDev& d, float* near, cudaStream_t s);

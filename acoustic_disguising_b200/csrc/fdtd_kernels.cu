@@ -691,7 +691,10 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
   const int4 item = p.items[blockIdx.x];
   const SolveDev& G = p.solves[item.x];
   const int it = G.it_base + p.step;
-  if (it > G.it_stop) return;
+  if (it > G.it_stop) {
+    pdl_wait();  // this kernel is not over before those it depends on
+    return;
+  }
   const int tid = threadIdx.y * 32 + threadIdx.x, nthr = blockDim.x * blockDim.y;
   {
     const int* src = reinterpret_cast<const int*>(&G);
@@ -713,6 +716,10 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
       fence_mbar_init();
     }
   }
+  // Up to here only the descriptors and tables of the set-up were read.  The field,
+  // the sources and the records belong to the kernels before.
+  pdl_wait();
+  pdl_trigger();  // after the wait: one step's kernels start ahead, not a chain of them
   __syncthreads();
   if (S.flags & SF_FP32)
     step_item<float>(p, S, item, it, sPn, sV, s_co, ring, s_fl, rbar);
@@ -759,6 +766,8 @@ cudaError_t launch_mask_tiles(const SolveDev& d, unsigned char* closed, cudaStre
 // Per-step trace assembly (derivatives.jl:51-56 record sums in corner order,
 // v2vn! :85-90, vn2v! :92-97 into row it+1).
 __global__ void adf_fdtd_epilogue_kernel(const EpiParams p) {
+  pdl_trigger();
+  pdl_wait();
   const SolveDev& S = p.solves[blockIdx.y];
   const int it = S.it_base + p.step;
   if (it > S.it_stop) return;
@@ -842,6 +851,8 @@ __device__ __forceinline__ void gf_finish(const SolveDev& S, int o, int it, int 
 // per source (ks = 1) that block completes the source itself.  Rows before
 // `it` of pin come from gf_pin; row `it` is formed here and block 0 files it.
 __global__ void __launch_bounds__(256, 4) adf_gf_extrapolate_kernel(const EpiParams p) {
+  pdl_trigger();
+  pdl_wait();
   const SolveDev& S = p.solves[blockIdx.y];
   const int it = S.it_base + p.step;
   if (it > S.it_stop || it >= S.nt || !(S.flags & SF_GF)) return;
@@ -1129,10 +1140,29 @@ cudaError_t launch_advance(SolveDev* solves, int n, int by, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_step(const StepParams& p, int grid, int max_ty, cudaStream_t s) {
+// A launch that may overlap the end of the kernel before it: the launch latency
+// and, in the step kernel, the reading of descriptors and tables go on while that
+// one finishes.
+template <typename P>
+static cudaError_t launch_overlapped(void (*kernel)(P), dim3 grid, dim3 block, size_t smem,
+                                     bool overlap, cudaStream_t s, P p) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &a;
+  c.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, p);
+}
+
+cudaError_t launch_step(const StepParams& p, int grid, int max_ty, bool overlap, cudaStream_t s) {
   (void)max_ty;  // the block always holds kMaxTy rows; shorter tiles idle the rest
-  adf_fdtd_step_kernel<<<grid, dim3(32, kXT / 16), kStepDynSmem, s>>>(p);
-  return cudaGetLastError();
+  return launch_overlapped(adf_fdtd_step_kernel, dim3(grid), dim3(32, kXT / 16), kStepDynSmem,
+                           overlap, s, p);
 }
 
 int step_max_ty() { return kMaxTy; }
@@ -1143,11 +1173,12 @@ cudaError_t step_ctas_per_sm(int* n) {
 int step_x_tile() { return kXT; }
 
 cudaError_t launch_gf_extrapolate(const EpiParams& p, int max_blocks, int max_nsrc, bool reduce,
-                                  cudaStream_t s) {
+                                  bool overlap, cudaStream_t s) {
   // (source, receiver split) blocks of the largest map in the batch, then,
   // when some solve splits its receivers, the fixed-order reduction
-  adf_gf_extrapolate_kernel<<<dim3(max_blocks > 0 ? max_blocks : 1, p.n_solves), 256, 0, s>>>(p);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_overlapped(adf_gf_extrapolate_kernel,
+                                    dim3(max_blocks > 0 ? max_blocks : 1, p.n_solves), dim3(256), 0,
+                                    overlap, s, p);
   if (e != cudaSuccess || !reduce) return e;
   adf_gf_reduce_kernel<<<dim3((max_nsrc + 127) / 128, p.n_solves), 128, 0, s>>>(p);
   return cudaGetLastError();
@@ -1189,13 +1220,12 @@ cudaError_t launch_gf_far(const EpiParams& p, int max_blocks, int max_nsrc, cuda
   return cudaGetLastError();
 }
 
-cudaError_t launch_epilogue(const EpiParams& p, int max_ntx, cudaStream_t s) {
+cudaError_t launch_epilogue(const EpiParams& p, int max_ntx, bool overlap, cudaStream_t s) {
   int threads = 128;
   int gx = (max_ntx + threads - 1) / threads;
   if (gx < 1) gx = 1;
-  dim3 grid(gx, p.n_solves);
-  adf_fdtd_epilogue_kernel<<<grid, threads, 0, s>>>(p);
-  return cudaGetLastError();
+  return launch_overlapped(adf_fdtd_epilogue_kernel, dim3(gx, p.n_solves), dim3(threads), 0, overlap,
+                           s, p);
 }
 
 }  // namespace adf

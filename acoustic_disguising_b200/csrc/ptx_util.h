@@ -71,6 +71,12 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* map, int x
       "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(mbar)
       : "memory");
 }
+// Programmatic dependent launch: lets the next kernel of the stream start once
+// every block got here; waits until the kernels before have completed and their
+// writes are visible (nothing to wait for in a kernel launched without it).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }

@@ -556,7 +556,10 @@ int Batch::launch_step(adf_ctx* ctx, int step) {
       cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
   if (timed && cudaEventRecordWithFlags(ctx->kev[2 * step], ctx->stream, evf) != cudaSuccess)
     return fail(ADF_E_DEVICE, std::string("event record: ") + cudaGetErrorString(cudaGetLastError()));
-  cudaError_t e = adf::launch_step(p, grid, max_ty, ctx->stream);
+  // Kernels of a step overlap their predecessor's end, except under the per-launch
+  // timing; the first of a chunk may follow the kernel that advances it_base.
+  const bool overlap = !ctx->kernel_timing;
+  cudaError_t e = adf::launch_step(p, grid, max_ty, overlap && step > 0, ctx->stream);
   if (e != cudaSuccess)
     return fail(ADF_E_DEVICE, std::string("step launch failed: ") + cudaGetErrorString(e) +
                                   " (grid " + std::to_string(grid) + ")");
@@ -567,7 +570,7 @@ int Batch::launch_step(adf_ctx* ctx, int step) {
   ep.n_solves = (int)solves.size();
   ep.step = step;
   cudaError_t e2;
-  if ((e2 = launch_epilogue(ep, max_ntx, ctx->stream)) != cudaSuccess)
+  if ((e2 = launch_epilogue(ep, max_ntx, overlap, ctx->stream)) != cudaSuccess)
     return fail(ADF_E_DEVICE, std::string("epilogue launch failed: ") + cudaGetErrorString(e2));
   if (max_gf_nsrc > 0) {  // in-loop GF extrapolation, then vn2v! of those solves
     // the far lags of a block of steps, at the block's first launch-step
@@ -577,7 +580,8 @@ int Batch::launch_step(adf_ctx* ctx, int step) {
     if ((max_gf_far_blocks > 0 || max_gf_tc_blocks > 0) && step % kGfBlock == 0 &&
         (e2 = launch_gf_far(ep, max_gf_far_blocks, max_gf_nsrc, ctx->stream)) != cudaSuccess)
       return fail(ADF_E_DEVICE, std::string("GF launch failed: ") + cudaGetErrorString(e2));
-    if ((e2 = launch_gf_extrapolate(ep, max_gf_blocks, max_gf_nsrc, gf_reduce, ctx->stream)) !=
+    if ((e2 = launch_gf_extrapolate(ep, max_gf_blocks, max_gf_nsrc, gf_reduce, overlap,
+                                    ctx->stream)) !=
         cudaSuccess)
       return fail(ADF_E_DEVICE, std::string("GF launch failed: ") + cudaGetErrorString(e2));
   }
