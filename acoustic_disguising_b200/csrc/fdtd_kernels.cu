@@ -19,7 +19,7 @@
 // that chain and the instructions around it, not HBM.  With the stage read
 // through shared-space addresses, on different banks, and the entries' code out
 // of the plane loop, a launch of 8 x 256^3 takes 0.82 ms without boundaries
-// (0.89 before) and 1.54 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
+// (0.89 before) and 1.42 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
 // The plane loop's code has to stay small: a masked form of the plain update and
 // one with the x slab's memory each made it slower (1.57 and 1.66 ms).
 //
@@ -29,12 +29,13 @@
 // difference is x*(1/dx) in place of x/dx.  Arith<float> is the all-Float32
 // variant.  Injection/recording (derivatives.jl:30-60) is pure Float32 with
 // separate multiply and add, as the reference computes it.
+#include <cstddef>
+
 #include "adf_internal.h"
 #include "ptx_util.h"
 
 namespace adf {
 
-constexpr int kMaxCoef = 8 * 63 + 4;  // CPML coefficients for npml <= 63
 
 // ---------------------------------------------------------------------------
 // Arithmetic policies
@@ -94,107 +95,131 @@ struct Sc {  // per-solve update scalars in registers
   R fq, fv, rdx, rdy, rdz;
 };
 
-// Per-(row, plane) geometry shared by the cells of a quad, uniform across a warp.
-struct RowCtx {
-  int nx, ny, nz, npml, nxp, j, k, rb, wb;
-  bool pcpml, vcpml;
+// What the CPML updates of a work item need, in shared memory: per array (p x,
+// y, z, v x, y, z) the buffer read, the one written and, for the x and y slabs,
+// the plane stride; the coefficients of the tile's columns ([3] is the halo
+// column's), rows and planes; and where the z slabs' layers lie (-1: none).
+// (Element offsets are 32-bit: a buffer holds at most 4 x 512 x 512 x 68.)  A
+// boundary warp's length sets its CTA's pace, so what does not change from plane
+// to plane is worked out once per item: 8 x 256^3 with CPML 1.36 -> 1.28 ms.
+struct PmlTab {
+  const float* rd[6];
+  float* wr[6];
+  int stride[6];
+  alignas(16) float xpa[68];  // (read four at a time)
+  alignas(16) float xpb[68];
+  alignas(16) float xva[68];
+  alignas(16) float xvb[68];
+  float ypa[8], ypb[8], yva[8], yvb[8];
+  float zpa[kMaxZc + 1], zpb[kMaxZc + 1], zva[kMaxZc + 1], zvb[kMaxZc + 1];
+  int zp[kMaxZc + 1], zv[kMaxZc + 1];
 };
 
-// ---------------------------------------------------------------------------
-// Pressure update of the quad x0..x0+3 of row j, plane k (update_p_cpml!,
-// update_p_mask!, update_p! on the rigid planes; updates.jl:21-136).
-// Inputs are the plane's P, Vx (x0..x0+4), Vy (rows j, j+1) and Vz (planes
-// k, k+1) from the input buffer.  Row- and plane-wide conditions (rigid
-// planes, y/z slabs) are warp-uniform branches; the x slab is a per-cell
-// block taken only by quads that touch it.  `owned` stores the new CPML
-// memory; recomputed halo cells and the prologue plane leave it alone.
-// ---------------------------------------------------------------------------
+static_assert(offsetof(PmlTab, xpa) % 16 == 0 && offsetof(PmlTab, xpb) % 16 == 0 &&
+                  offsetof(PmlTab, xva) % 16 == 0 && offsetof(PmlTab, xvb) % 16 == 0,
+              "a quad's coefficients are one aligned float4");
+
+// A thread's quad, for the planes of an item.
+struct Quad {
+  // cell e: bit e P updated (x <= nx-2), 4+e Vx updated (1 <= x < nx), 8+e in the
+  // grid (x < nx), 12+e P has x-slab memory, 16+e Vx has; bit 20: cells in both x
+  // slabs (narrow grids)
+  uint32_t bits;
+  int j, x0, r;
+  int px, vx;  // x-slab memory of plane 0
+  int py, vy;  // y-slab memory of plane 0, -1: none
+};
+
+// x-slab memory of a quad with cells in both slabs: cell by cell.
 template <typename R>
-__device__ __forceinline__ float4 p_update_quad(const SolveDev& S, const RowCtx& rc, const Sc<R>& g,
-                                                const float* co, int x0, bool owned, float4 P4,
-                                                float4 X4, float X5, float4 Y0, float4 Y1,
-                                                float4 Z0, float4 Z1, uint32_t nib) {
-  using A = Arith<R>;
-  const int nx = rc.nx, ny = rc.ny, nz = rc.nz, npml = rc.npml, j = rc.j, k = rc.k;
-  const bool rigid_y = j == ny - 1, rigid_z = k == nz - 1;
-  // rigid planes use update_p! (-2V/d at the wall, no CPML, no mask); the
-  // (ny, nz) corner is not updated at all
-  const bool plain_rigid = rigid_y || rigid_z;
-  const bool corner = rigid_y && rigid_z;
-  if (plain_rigid) nib = 0xFFFFu;
-  const float Pv[4] = {P4.x, P4.y, P4.z, P4.w};
-  const float dxv[4] = {__fsub_rn(X4.y, X4.x), __fsub_rn(X4.z, X4.y), __fsub_rn(X4.w, X4.z),
-                        __fsub_rn(X5, X4.w)};
-  const float dyv[4] = {rigid_y ? __fmul_rn(-2.0f, Y0.x) : __fsub_rn(Y1.x, Y0.x),
-                        rigid_y ? __fmul_rn(-2.0f, Y0.y) : __fsub_rn(Y1.y, Y0.y),
-                        rigid_y ? __fmul_rn(-2.0f, Y0.z) : __fsub_rn(Y1.z, Y0.z),
-                        rigid_y ? __fmul_rn(-2.0f, Y0.w) : __fsub_rn(Y1.w, Y0.w)};
-  const float dzv[4] = {rigid_z ? __fmul_rn(-2.0f, Z0.x) : __fsub_rn(Z1.x, Z0.x),
-                        rigid_z ? __fmul_rn(-2.0f, Z0.y) : __fsub_rn(Z1.y, Z0.y),
-                        rigid_z ? __fmul_rn(-2.0f, Z0.z) : __fsub_rn(Z1.z, Z0.z),
-                        rigid_z ? __fmul_rn(-2.0f, Z0.w) : __fsub_rn(Z1.w, Z0.w)};
-  R dvx[4], dvy[4], dvz[4];
-  bool upd[4];
+__device__ __forceinline__ void x_slabs_narrow(R (&d)[4], const PmlTab& Q, int arr, int pitch,
+                                               int side1, int first1, int row, int x0, uint32_t in,
+                                               bool store, const float* a, const float* b) {
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    dvx[e] = A::mul(A::cv(dxv[e]), g.rdx);
-    dvy[e] = A::mul(A::cv(dyv[e]), g.rdy);
-    dvz[e] = A::mul(A::cv(dzv[e]), g.rdz);
-    upd[e] = x0 + e <= nx - 2 && !corner;
+    if (!((in >> e) & 1u)) continue;
+    const int x = x0 + e;
+    const int o = row * pitch + (x < first1 ? x : x + side1);
+    float m = Q.rd[arr][o];
+    cpml_apply<R>(d[e], m, a[e], b[e]);
+    if (store) Q.wr[arr][o] = m;
   }
-  if (rc.pcpml && !plain_rigid) {
-    const bool s0 = x0 < npml, s1 = x0 + 3 >= nx - npml;
-    // x slab: the quad's memory of a side is one aligned float4 (both sides
-    // only on grids narrower than two slabs and a quad: one after the other)
-    const long long row = ((long long)k * ny + j) * S.npp;
-    for (int sd = 0; sd < 2; ++sd) {
-      if (!(sd == 0 ? s0 : s1)) continue;
-      const long long o = sd == 0 ? row + x0 : S.psi_p_side[0] + row + (x0 - S.xs1p);
-      const float4 t = ld4(S.psi_p[0] + rc.rb * S.psi_p_buf[0] + o);
-      float m[4] = {t.x, t.y, t.z, t.w};
+}
+
+// ---------------------------------------------------------------------------
+// Pressure update of a quad of plane k (update_p_cpml!, update_p_mask!,
+// update_p! on the rigid planes; updates.jl:21-136), u = k - kfirst.  Inputs are
+// the plane's P, Vx (x0..x0+4), Vy (rows j, j+1) and Vz (planes k, k+1) from the
+// input buffer.  Row- and plane-wide conditions (rigid planes, y/z slabs) are
+// warp-uniform or nearly so; the x slab is a block taken only by quads that
+// touch it.  `owned` stores the new CPML memory; recomputed halo cells and the
+// prologue plane leave it alone.
+// ---------------------------------------------------------------------------
+template <typename R>
+__device__ __forceinline__ float4 p_update_quad(const SolveDev& S, const PmlTab& Q, const Quad& q,
+                                                const Sc<R>& g, bool pcpml, int k, int u, bool owned,
+                                                float4 P4, float4 X4, float X5, float4 Y0, float4 Y1,
+                                                float4 Z0, float4 Z1, uint32_t nib) {
+  using A = Arith<R>;
+  const bool rigid_y = q.j == S.ny - 1, rigid_z = k == S.nz - 1;
+  // rigid planes use update_p! (-2V/d at the wall, no CPML, no mask); the
+  // (ny, nz) corner is not updated at all
+  if (rigid_y) Y1 = neg4(Y0);
+  if (rigid_z) Z1 = neg4(Z0);
+  if (rigid_y || rigid_z) nib = 0xFFFFu;
+  uint32_t up = q.bits & 15u;
+  if (rigid_y && rigid_z) up = 0;
+  R dx[4] = {A::mul(A::cv(__fsub_rn(X4.y, X4.x)), g.rdx), A::mul(A::cv(__fsub_rn(X4.z, X4.y)), g.rdx),
+             A::mul(A::cv(__fsub_rn(X4.w, X4.z)), g.rdx), A::mul(A::cv(__fsub_rn(X5, X4.w)), g.rdx)};
+  R dy[4] = {A::mul(A::cv(__fsub_rn(Y1.x, Y0.x)), g.rdy), A::mul(A::cv(__fsub_rn(Y1.y, Y0.y)), g.rdy),
+             A::mul(A::cv(__fsub_rn(Y1.z, Y0.z)), g.rdy), A::mul(A::cv(__fsub_rn(Y1.w, Y0.w)), g.rdy)};
+  R dz[4] = {A::mul(A::cv(__fsub_rn(Z1.x, Z0.x)), g.rdz), A::mul(A::cv(__fsub_rn(Z1.y, Z0.y)), g.rdz),
+             A::mul(A::cv(__fsub_rn(Z1.z, Z0.z)), g.rdz), A::mul(A::cv(__fsub_rn(Z1.w, Z0.w)), g.rdz)};
+  if (pcpml && !rigid_y && !rigid_z) {
+    if (q.bits & 0xF000u) {
+      const float4 a4 = ld4(Q.xpa + 4 + 4 * (q.x0 / 4 % 16)), b4 = ld4(Q.xpb + 4 + 4 * (q.x0 / 4 % 16));
+      const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+      if (q.bits & (1u << 20)) {
+        x_slabs_narrow<R>(dx, Q, 0, S.npp, (int)S.psi_p_side[0] - S.xs1p, S.npml, k * S.ny + q.j, q.x0,
+                          q.bits >> 12, owned, a, b);
+      } else {
+        const int o = q.px + k * Q.stride[0];
+        const float4 t = ld4(Q.rd[0] + o);
+        float m[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int x = x0 + e;
-        const int side = x < npml ? 0 : (x >= nx - npml ? 1 : -1);
-        if (side == sd && upd[e]) {
-          const int l = side == 0 ? x : x - (nx - npml);
-          cpml_apply<R>(dvx[e], m[e], co[side * npml + l], co[4 * npml + 2 + side * npml + l]);
-        }
+        for (int e = 0; e < 4; ++e)
+          if ((q.bits >> (12 + e)) & 1u) cpml_apply<R>(dx[e], m[e], a[e], b[e]);
+        // cells outside the slab or not updated write back what they read
+        if (owned) st4(Q.wr[0] + o, make_float4(m[0], m[1], m[2], m[3]));
       }
-      // cells outside the slab or not updated write back what they read
-      if (owned) st4(S.psi_p[0] + rc.wb * S.psi_p_buf[0] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
-    const int ysd = j < npml ? 0 : (j >= ny - npml ? 1 : -1);
-    if (ysd >= 0) {  // y slab: the whole quad, cells that are not updated keep their memory
-      const int yl = ysd == 0 ? j : j - (ny - npml);
-      const long long o = ysd * S.psi_p_side[1] + ((long long)k * npml + yl) * rc.nxp + x0;
-      const float4 m4 = ld4(S.psi_p[1] + rc.rb * S.psi_p_buf[1] + o);
-      float m[4] = {m4.x, m4.y, m4.z, m4.w};
-      const float a = co[ysd * npml + yl], b = co[4 * npml + 2 + ysd * npml + yl];
+    if (q.py >= 0) {  // y slab: the whole quad, cells that are not updated keep their memory
+      const int o = q.py + k * Q.stride[1];
+      const float4 t = ld4(Q.rd[1] + o);
+      float m[4] = {t.x, t.y, t.z, t.w};
+      const float a = Q.ypa[q.r], b = Q.ypb[q.r];
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        if (upd[e]) cpml_apply<R>(dvy[e], m[e], a, b);
-      if (owned) st4(S.psi_p[1] + rc.wb * S.psi_p_buf[1] + o, make_float4(m[0], m[1], m[2], m[3]));
+        if ((up >> e) & 1u) cpml_apply<R>(dy[e], m[e], a, b);
+      if (owned) st4(Q.wr[1] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
-    const int zsd = k < npml ? 0 : (k >= nz - npml ? 1 : -1);
-    if (zsd >= 0) {
-      const int zl = zsd == 0 ? k : k - (nz - npml);
-      const long long o = zsd * S.psi_p_side[2] + ((long long)zl * ny + j) * rc.nxp + x0;
-      const float4 m4 = ld4(S.psi_p[2] + rc.rb * S.psi_p_buf[2] + o);
-      float m[4] = {m4.x, m4.y, m4.z, m4.w};
-      const float a = co[zsd * npml + zl], b = co[4 * npml + 2 + zsd * npml + zl];
+    if (Q.zp[u] >= 0) {
+      const int o = Q.zp[u] + q.j * S.nxp + q.x0;
+      const float4 t = ld4(Q.rd[2] + o);
+      float m[4] = {t.x, t.y, t.z, t.w};
+      const float a = Q.zpa[u], b = Q.zpb[u];
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        if (upd[e]) cpml_apply<R>(dvz[e], m[e], a, b);
-      if (owned) st4(S.psi_p[2] + rc.wb * S.psi_p_buf[2] + o, make_float4(m[0], m[1], m[2], m[3]));
+        if ((up >> e) & 1u) cpml_apply<R>(dz[e], m[e], a, b);
+      if (owned) st4(Q.wr[2] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
   }
+  const float Pv[4] = {P4.x, P4.y, P4.z, P4.w};
   float o[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    const float n =
-        A::rn(A::sub(A::cv(Pv[e]), A::mul(g.fq, A::add(A::add(dvx[e], dvy[e]), dvz[e]))));
-    o[e] = (upd[e] && ((nib >> (4 * e)) & 1u)) ? n : Pv[e];
+    const float n = A::rn(A::sub(A::cv(Pv[e]), A::mul(g.fq, A::add(A::add(dx[e], dy[e]), dz[e]))));
+    o[e] = ((up >> e) & (nib >> (4 * e)) & 1u) ? n : Pv[e];
   }
   return make_float4(o[0], o[1], o[2], o[3]);
 }
@@ -203,11 +228,11 @@ __device__ __forceinline__ float4 p_update_quad(const SolveDev& S, const RowCtx&
 // the staged plane `st` (P, Vx, Vy of plane k; `c` the cell's offset in a
 // channel, `cst` the channel stride) and Vz of planes k and k+1 (Z0, Z1).
 template <typename R>
-__device__ __forceinline__ float p_update_cell(const SolveDev& S, const RowCtx& rc, const Sc<R>& g,
-                                               const float* co, const float* st, float Z0,
-                                               float Z1, int c, int cst, int x, bool masked) {
+__device__ __forceinline__ float p_update_cell(const SolveDev& S, const PmlTab& Q, const Sc<R>& g,
+                                               bool pcpml, const float* st, float Z0, float Z1, int c,
+                                               int cst, int x, int j, int r, int k, int u, bool masked) {
   using A = Arith<R>;
-  const int nx = rc.nx, ny = rc.ny, nz = rc.nz, npml = rc.npml, j = rc.j, k = rc.k, nxp = rc.nxp;
+  const int nx = S.nx, ny = S.ny, nz = S.nz, npml = S.npml, nxp = S.nxp;
   const bool rigid_y = j == ny - 1, rigid_z = k == nz - 1;
   const bool plain_rigid = rigid_y || rigid_z;
   const bool upd = x <= nx - 2 && !(rigid_y && rigid_z);
@@ -223,27 +248,19 @@ __device__ __forceinline__ float p_update_cell(const SolveDev& S, const RowCtx& 
   bool open = true;
   if (!plain_rigid) {
     if (masked) open = (S.mask_bits[((long long)k * ny + j) * S.mw + (x >> 3)] >> (4 * (x & 7))) & 1u;
-    if (rc.pcpml) {
-      const int xs = x < npml ? 0 : (x >= nx - npml ? 1 : -1);
-      if (xs >= 0) {
-        const int l = xs == 0 ? x : x - (nx - npml);
-        float m = S.psi_p[0][rc.rb * S.psi_p_buf[0] + xs * S.psi_p_side[0] +
-                             ((long long)k * ny + j) * S.npp + (xs == 0 ? x : x - S.xs1p)];
-        cpml_apply<R>(dvx, m, co[xs * npml + l], co[4 * npml + 2 + xs * npml + l]);
+    if (pcpml) {
+      if (x < npml || x >= nx - npml) {
+        float m = Q.rd[0][(k * ny + j) * S.npp + (x < npml ? x : (int)S.psi_p_side[0] + x - S.xs1p)];
+        cpml_apply<R>(dvx, m, Q.xpa[3], Q.xpb[3]);
       }
-      const int ysd = j < npml ? 0 : (j >= ny - npml ? 1 : -1);
-      if (ysd >= 0) {
-        const int yl = ysd == 0 ? j : j - (ny - npml);
-        float m = S.psi_p[1][rc.rb * S.psi_p_buf[1] + ysd * S.psi_p_side[1] +
-                             ((long long)k * npml + yl) * nxp + x];
-        cpml_apply<R>(dvy, m, co[ysd * npml + yl], co[4 * npml + 2 + ysd * npml + yl]);
+      if (j < npml || j >= ny - npml) {
+        float m = Q.rd[1][(j < npml ? 0 : (int)S.psi_p_side[1]) +
+                          (k * npml + (j < npml ? j : j - (ny - npml))) * nxp + x];
+        cpml_apply<R>(dvy, m, Q.ypa[r], Q.ypb[r]);
       }
-      const int zsd = k < npml ? 0 : (k >= nz - npml ? 1 : -1);
-      if (zsd >= 0) {
-        const int zl = zsd == 0 ? k : k - (nz - npml);
-        float m = S.psi_p[2][rc.rb * S.psi_p_buf[2] + zsd * S.psi_p_side[2] +
-                             ((long long)zl * ny + j) * nxp + x];
-        cpml_apply<R>(dvz, m, co[zsd * npml + zl], co[4 * npml + 2 + zsd * npml + zl]);
+      if (Q.zp[u] >= 0) {
+        float m = Q.rd[2][Q.zp[u] + j * nxp + x];
+        cpml_apply<R>(dvz, m, Q.zpa[u], Q.zpb[u]);
       }
     }
   }
@@ -257,86 +274,69 @@ __device__ __forceinline__ float p_update_cell(const SolveDev& S, const RowCtx& 
 // x < nx; CPML with the half-grid coefficients (npml+1 layers).
 // ---------------------------------------------------------------------------
 template <typename R>
-__device__ __forceinline__ void v_update_quad(const SolveDev& S, const RowCtx& rc, const Sc<R>& g,
-                                              const float* co, int x0, float4 Pc, float Pxm,
-                                              float4 Pym, float4 Pzm, float4 VX, float4 VY,
+__device__ __forceinline__ void v_update_quad(const SolveDev& S, const PmlTab& Q, const Quad& q,
+                                              const Sc<R>& g, bool vcpml, int k, int u, float4 Pc,
+                                              float Pxm, float4 Pym, float4 Pzm, float4 VX, float4 VY,
                                               float4 VZ, uint32_t nib, float4& vxo, float4& vyo,
                                               float4& vzo) {
   using A = Arith<R>;
-  const int nx = rc.nx, ny = rc.ny, nz = rc.nz, npml = rc.npml, nm = npml + 1, j = rc.j, k = rc.k;
-  const float Pv[4] = {Pc.x, Pc.y, Pc.z, Pc.w};
-  const float Pl[4] = {Pxm, Pc.x, Pc.y, Pc.z};
-  const float Py[4] = {Pym.x, Pym.y, Pym.z, Pym.w};
-  const float Pz[4] = {Pzm.x, Pzm.y, Pzm.z, Pzm.w};
-  const float Vx[4] = {VX.x, VX.y, VX.z, VX.w};
-  const float Vy[4] = {VY.x, VY.y, VY.z, VY.w};
-  const float Vz[4] = {VZ.x, VZ.y, VZ.z, VZ.w};
-  R dx[4], dy[4], dz[4];
-  bool in[4];
+  const uint32_t in = (q.bits >> 8) & 15u;
+  R dx[4] = {A::mul(A::cv(__fsub_rn(Pc.x, Pxm)), g.rdx), A::mul(A::cv(__fsub_rn(Pc.y, Pc.x)), g.rdx),
+             A::mul(A::cv(__fsub_rn(Pc.z, Pc.y)), g.rdx), A::mul(A::cv(__fsub_rn(Pc.w, Pc.z)), g.rdx)};
+  R dy[4] = {A::mul(A::cv(__fsub_rn(Pc.x, Pym.x)), g.rdy), A::mul(A::cv(__fsub_rn(Pc.y, Pym.y)), g.rdy),
+             A::mul(A::cv(__fsub_rn(Pc.z, Pym.z)), g.rdy), A::mul(A::cv(__fsub_rn(Pc.w, Pym.w)), g.rdy)};
+  R dz[4] = {A::mul(A::cv(__fsub_rn(Pc.x, Pzm.x)), g.rdz), A::mul(A::cv(__fsub_rn(Pc.y, Pzm.y)), g.rdz),
+             A::mul(A::cv(__fsub_rn(Pc.z, Pzm.z)), g.rdz), A::mul(A::cv(__fsub_rn(Pc.w, Pzm.w)), g.rdz)};
+  if (vcpml) {
+    if (q.bits & 0xF0000u) {
+      const float4 a4 = ld4(Q.xva + 4 + 4 * (q.x0 / 4 % 16)), b4 = ld4(Q.xvb + 4 + 4 * (q.x0 / 4 % 16));
+      const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+      if (q.bits & (1u << 20)) {
+        x_slabs_narrow<R>(dx, Q, 3, S.nvp, (int)S.psi_v_side[0] - S.xs1v, S.npml + 1, k * S.ny + q.j,
+                          q.x0, q.bits >> 16, true, a, b);
+      } else {
+        const int o = q.vx + k * Q.stride[3];
+        const float4 t = ld4(Q.rd[3] + o);
+        float m[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    dx[e] = A::mul(A::cv(__fsub_rn(Pv[e], Pl[e])), g.rdx);
-    dy[e] = A::mul(A::cv(__fsub_rn(Pv[e], Py[e])), g.rdy);
-    dz[e] = A::mul(A::cv(__fsub_rn(Pv[e], Pz[e])), g.rdz);
-    in[e] = x0 + e < nx;
-  }
-  if (rc.vcpml) {
-    const bool s0 = x0 <= npml, s1 = x0 + 3 >= nx - npml - 1;
-    // x slab: one aligned float4 per side, the sides one after the other
-    const long long row = ((long long)k * ny + j) * S.nvp;
-    for (int sd = 0; sd < 2; ++sd) {
-      if (!(sd == 0 ? s0 : s1)) continue;
-      const long long o = sd == 0 ? row + x0 : S.psi_v_side[0] + row + (x0 - S.xs1v);
-      const float4 t = ld4(S.psi_v[0] + rc.rb * S.psi_v_buf[0] + o);
-      float m[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int x = x0 + e;
-        const int side = x <= npml ? 0 : (x >= nx - npml - 1 ? 1 : -1);
-        if (side == sd && in[e] && x >= 1) {
-          const int l = side == 0 ? x : x - (nx - npml - 1);
-          cpml_apply<R>(dx[e], m[e], co[2 * npml + side * nm + l], co[6 * npml + 2 + side * nm + l]);
-        }
+        for (int e = 0; e < 4; ++e)
+          if ((q.bits >> (16 + e)) & 1u) cpml_apply<R>(dx[e], m[e], a[e], b[e]);
+        st4(Q.wr[3] + o, make_float4(m[0], m[1], m[2], m[3]));
       }
-      st4(S.psi_v[0] + rc.wb * S.psi_v_buf[0] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
-    const int ysd = j < 1 ? -1 : (j <= npml ? 0 : (j >= ny - npml - 1 ? 1 : -1));
-    if (ysd >= 0) {
-      const int yl = ysd == 0 ? j : j - (ny - npml - 1);
-      const long long o = ysd * S.psi_v_side[1] + ((long long)k * nm + yl) * rc.nxp + x0;
-      const float4 m4 = ld4(S.psi_v[1] + rc.rb * S.psi_v_buf[1] + o);
-      float m[4] = {m4.x, m4.y, m4.z, m4.w};
-      const float a = co[2 * npml + ysd * nm + yl], b = co[6 * npml + 2 + ysd * nm + yl];
+    if (q.vy >= 0) {
+      const int o = q.vy + k * Q.stride[4];
+      const float4 t = ld4(Q.rd[4] + o);
+      float m[4] = {t.x, t.y, t.z, t.w};
+      const float a = Q.yva[q.r], b = Q.yvb[q.r];
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        if (in[e]) cpml_apply<R>(dy[e], m[e], a, b);
-      st4(S.psi_v[1] + rc.wb * S.psi_v_buf[1] + o, make_float4(m[0], m[1], m[2], m[3]));
+        if ((in >> e) & 1u) cpml_apply<R>(dy[e], m[e], a, b);
+      st4(Q.wr[4] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
-    const int zsd = k < 1 ? -1 : (k <= npml ? 0 : (k >= nz - npml - 1 ? 1 : -1));
-    if (zsd >= 0) {
-      const int zl = zsd == 0 ? k : k - (nz - npml - 1);
-      const long long o = zsd * S.psi_v_side[2] + ((long long)zl * ny + j) * rc.nxp + x0;
-      const float4 m4 = ld4(S.psi_v[2] + rc.rb * S.psi_v_buf[2] + o);
-      float m[4] = {m4.x, m4.y, m4.z, m4.w};
-      const float a = co[2 * npml + zsd * nm + zl], b = co[6 * npml + 2 + zsd * nm + zl];
+    if (Q.zv[u] >= 0) {
+      const int o = Q.zv[u] + q.j * S.nxp + q.x0;
+      const float4 t = ld4(Q.rd[5] + o);
+      float m[4] = {t.x, t.y, t.z, t.w};
+      const float a = Q.zva[u], b = Q.zvb[u];
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        if (in[e]) cpml_apply<R>(dz[e], m[e], a, b);
-      st4(S.psi_v[2] + rc.wb * S.psi_v_buf[2] + o, make_float4(m[0], m[1], m[2], m[3]));
+        if ((in >> e) & 1u) cpml_apply<R>(dz[e], m[e], a, b);
+      st4(Q.wr[5] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
   }
+  const uint32_t ux = (q.bits >> 4) & 15u, uy = q.j >= 1 ? in : 0u, uz = k >= 1 ? in : 0u;
+  const float Vx[4] = {VX.x, VX.y, VX.z, VX.w}, Vy[4] = {VY.x, VY.y, VY.z, VY.w},
+              Vz[4] = {VZ.x, VZ.y, VZ.z, VZ.w};
   float ox[4], oy[4], oz[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    const bool ux = in[e] && x0 + e >= 1 && ((nib >> (4 * e + 1)) & 1u);
-    const bool uy = in[e] && j >= 1 && ((nib >> (4 * e + 2)) & 1u);
-    const bool uz = in[e] && k >= 1 && ((nib >> (4 * e + 3)) & 1u);
     const float nxv = A::rn(A::sub(A::cv(Vx[e]), A::mul(g.fv, dx[e])));
     const float nyv = A::rn(A::sub(A::cv(Vy[e]), A::mul(g.fv, dy[e])));
     const float nzv = A::rn(A::sub(A::cv(Vz[e]), A::mul(g.fv, dz[e])));
-    ox[e] = ux ? nxv : Vx[e];
-    oy[e] = uy ? nyv : Vy[e];
-    oz[e] = uz ? nzv : Vz[e];
+    ox[e] = ((ux >> e) & (nib >> (4 * e + 1)) & 1u) ? nxv : Vx[e];
+    oy[e] = ((uy >> e) & (nib >> (4 * e + 2)) & 1u) ? nyv : Vy[e];
+    oz[e] = ((uz >> e) & (nib >> (4 * e + 3)) & 1u) ? nzv : Vz[e];
   }
   vxo = make_float4(ox[0], ox[1], ox[2], ox[3]);
   vyo = make_float4(oy[0], oy[1], oy[2], oy[3]);
@@ -473,8 +473,8 @@ static_assert((kStageFloats * 4) % 128 == 0, "stages stay 128-B aligned");
 static_assert((stage_vz_offset(5 * kStageW) * 4) % 128 == 0, "Vz boxes start 128-B aligned");
 
 template <typename R>
-__device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S, int4 item, int it,
-                                          float* sPn, float* sV, const float* co, float* ring,
+__device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, int4 item, int it,
+                                          float* sPn, float* sV, float* ring,
                                           const unsigned char* s_fl, uint64_t* rbar) {
   const int lane = threadIdx.x, wid = threadIdx.y;
   const int tid = wid * 32 + lane;
@@ -501,17 +501,42 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
   g.rdx = Arith<R>::rdx(S);
   g.rdy = Arith<R>::rdy(S);
   g.rdz = Arith<R>::rdz(S);
-  RowCtx rc;
-  rc.nx = nx;
-  rc.ny = ny;
-  rc.nz = nz;
-  rc.npml = npml;
-  rc.nxp = nxp;
-  rc.j = j;
-  rc.rb = rb;
-  rc.wb = wb;
-  rc.pcpml = pcp;
-  rc.vcpml = vcp;
+  Quad q;
+  q.j = j;
+  q.x0 = x0;
+  q.r = r;
+  q.bits = 0;
+  q.px = q.vx = 0;
+  q.py = q.vy = -1;
+  {
+    int seen = 0;  // x slabs that the quad's cells lie in: 1 left, 2 right
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int x = x0 + e;
+      if (x <= nx - 2) q.bits |= 1u << e;
+      if (x >= 1 && x < nx) q.bits |= 16u << e;
+      if (x < nx) q.bits |= 256u << e;
+      if (pcp && x <= nx - 2 && (x < npml || x >= nx - npml)) {
+        q.bits |= 4096u << e;
+        seen |= x < npml ? 1 : 2;
+      }
+      if (vcp && x >= 1 && x < nx && (x <= npml || x >= nx - npml - 1)) {
+        q.bits |= 65536u << e;
+        seen |= x <= npml ? 4 : 8;
+      }
+    }
+    if ((seen & 3) == 3 || (seen & 12) == 12) q.bits |= 1u << 20;
+    if (act && pcp) {
+      q.px = j * S.npp + ((seen & 1) ? x0 : (int)S.psi_p_side[0] + x0 - S.xs1p);
+      const int ys = j < npml ? 0 : (j >= ny - npml ? 1 : -1);
+      if (ys >= 0) q.py = ys * (int)S.psi_p_side[1] + (ys == 0 ? j : j - (ny - npml)) * nxp + x0;
+    }
+    if (vrow && vcp) {
+      q.vx = j * S.nvp + ((seen & 4) ? x0 : (int)S.psi_v_side[0] + x0 - S.xs1v);
+      const int ys = j < 1 ? -1 : (j <= npml ? 0 : (j >= ny - npml - 1 ? 1 : -1));
+      if (ys >= 0) q.vy = ys * (int)S.psi_v_side[1] + (ys == 0 ? j : j - (ny - npml - 1)) * nxp + x0;
+    }
+  }
   // warp-uniform: do all of the warp's rows and x cells take the plain P
   // (and, rows >= 1, V) updates?  The plane is checked per plane below.
   bool wplain_rx, hplain_x;
@@ -571,11 +596,11 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
   }
   for (int k = kfirst; k < z1; ++k) {
     const bool prologue = k < z0;
-    rc.k = k;
+    const int u = k - kfirst;
     float* pn = sPn + (k & 1) * (kMaxTy + 1) * kPnPitch;
     const float* st = ring + slot_of(k) * kStageFloats;
     wait(k);
-    const int fl = s_fl[k - kfirst];
+    const int fl = s_fl[u];
     const bool has_mask = (fl & 4) != 0;  // elsewhere every cell of the tile's plane is open
     const bool pplane = k != nz - 1 && (!pcp || (k >= npml && k < nz - npml));
     const bool vplane = k >= 1 && (!vcp || (k > npml && k < nz - npml - 1));
@@ -595,7 +620,8 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
       if (wplain)
         Pn = p_plain_quad<R>(g, P4, X4, X5, Y0, Y1, Z0, Z1);
       else
-        Pn = p_update_quad<R>(S, rc, g, co, x0, vrow && !prologue, P4, X4, X5, Y0, Y1, Z0, Z1, nib);
+        Pn = p_update_quad<R>(S, Q, q, g, pcp, k, u, vrow && !prologue, P4, X4, X5, Y0, Y1, Z0, Z1,
+                              nib);
       st4(pn + pq, Pn);
     }
     if (hcol) {
@@ -605,8 +631,8 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
                                 __fsub_rn(st[2 * cst + so - 1 + kStageW], st[2 * cst + so - 1]),
                                 __fsub_rn(Zh1, Zh), g);
       else
-        pn[pq - 1] = p_update_cell<R>(S, rc, g, co, st, Zh, Zh1, so - 1, cst, xb - 1,
-                                       has_mask);
+        pn[pq - 1] = p_update_cell<R>(S, Q, g, pcp, st, Zh, Zh1, so - 1, cst, xb - 1, j, r, k, u,
+                                      has_mask);
       Zh = Zh1;
     }
     __syncthreads();
@@ -626,7 +652,7 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
         if (wplain) {
           v_plain_quad<R>(g, Pn, Pxm, Pym, Pzm, X4, Y0, Z0, vx, vy, vz);
         } else {
-          v_update_quad<R>(S, rc, g, co, x0, Pn, Pxm, Pym, Pzm, X4, Y0, Z0, nib, vx, vy, vz);
+          v_update_quad<R>(S, Q, q, g, vcp, k, u, Pn, Pxm, Pym, Pzm, X4, Y0, Z0, nib, vx, vy, vz);
         }
       }
       // ---- f channel: inject/record on the new V (forward.jl:111-115) ----
@@ -667,6 +693,48 @@ __device__ __forceinline__ void step_item(const StepParams& p, const SolveDev& S
   }
 }
 
+// Fills the item's table: coefficients of cells in no slab are never read.
+__device__ __forceinline__ void pml_table(const SolveDev& G, PmlTab& Q, int4 item, int it, int kfirst,
+                                          int tid, int nthr) {
+  const int n = G.npml, nb = 4 * n + 2;
+  if (n == 0) {
+    for (int u = tid; u < item.w - kfirst; u += nthr) Q.zp[u] = Q.zv[u] = -1;
+    return;
+  }
+  const float* co = G.coef;
+  if (tid < 6) {
+    const int a = tid % 3, rb = (it - G.it_first) & 1;
+    const bool v = tid >= 3;
+    float* base = v ? G.psi_v[a] : G.psi_p[a];
+    const long long buf = v ? G.psi_v_buf[a] : G.psi_p_buf[a];
+    Q.rd[tid] = base + rb * buf;
+    Q.wr[tid] = base + (rb ^ 1) * buf;
+    Q.stride[tid] = a == 0 ? G.ny * (v ? G.nvp : G.npp) : (n + (v ? 1 : 0)) * G.nxp;
+  }
+  // index of the coefficient of cell x of an axis of m cells, -1: no slab
+  auto cp = [&](int x, int m) { return x < 0 || x >= m ? -1 : x < n ? x : (x >= m - n ? n + x - (m - n) : -1); };
+  auto cv = [&](int x, int m) {
+    return x < 0 || x >= m ? -1 : x <= n ? 2 * n + x : (x >= m - n - 1 ? 3 * n + 1 + x - (m - n - 1) : -1);
+  };
+  auto fill = [&](float* pa, float* pb, float* va, float* vb, int i, int x, int m) {
+    const int p = cp(x, m), v = cv(x, m);
+    if (p >= 0) pa[i] = co[p], pb[i] = co[nb + p];
+    if (v >= 0) va[i] = co[v], vb[i] = co[nb + v];
+  };
+  const int xb = (item.y >> 16) * kXT, j0 = (item.y & 0xFFFF) * G.ty;
+  for (int i = 3 + tid; i < 68; i += nthr) fill(Q.xpa, Q.xpb, Q.xva, Q.xvb, i, xb + i - 4, G.nx);
+  for (int i = tid; i < 8; i += nthr) fill(Q.ypa, Q.ypb, Q.yva, Q.yvb, i, j0 - 1 + i, G.ny);
+  for (int u = tid; u < item.w - kfirst; u += nthr) {
+    const int k = kfirst + u, p = cp(k, G.nz), v = k >= 1 ? cv(k, G.nz) : -1;
+    fill(Q.zpa, Q.zpb, Q.zva, Q.zvb, u, k, G.nz);
+    const int pl = G.ny * G.nxp;
+    Q.zp[u] = p < 0 ? -1 : (p >= n ? (int)G.psi_p_side[2] : 0) + (p >= n ? p - n : p) * pl;
+    Q.zv[u] = v < 0 ? -1
+                    : (v >= 3 * n + 1 ? (int)G.psi_v_side[2] : 0) +
+                          (v >= 3 * n + 1 ? v - 3 * n - 1 : v - 2 * n) * pl;
+  }
+}
+
 // Shared memory: the staged-plane ring (dynamic, kStepRing * kStageFloats
 // floats) plus the new-P planes, the f-channel staging and the descriptor:
 // 33.4 KB per CTA; five CTAs per SM (the register budget: 102 per thread,
@@ -685,7 +753,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
   __shared__ __align__(8) uint64_t rbar[kStepRing];
   __shared__ __align__(16) float sPn[2 * (kMaxTy + 1) * kPnPitch];
   __shared__ __align__(16) float sV[3 * kMaxTy * kXT];
-  __shared__ float s_co[kMaxCoef];
+  __shared__ __align__(16) PmlTab Q;
   __shared__ unsigned char s_fl[kMaxZc + 1];  // planes kfirst ..: 1 q, 2 f entries, 4 closed cells
   __shared__ __align__(16) SolveDev S;  // the solve descriptor, read in the hot loop
   const int4 item = p.items[blockIdx.x];
@@ -700,8 +768,6 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
     const int* src = reinterpret_cast<const int*>(&G);
     int* dst = reinterpret_cast<int*>(&S);
     for (int w = tid; w < (int)(sizeof(SolveDev) / 4); w += nthr) dst[w] = src[w];
-    const int ncoef = 8 * G.npml + 4;
-    for (int w = tid; w < ncoef; w += nthr) s_co[w] = G.coef[w];
     const int kfirst = item.z > 0 ? item.z - 1 : 0;
     if (tid < item.w - kfirst) {
       const int* tp = G.tp_off + ((long long)(item.y & 0xFFFF) * G.nz + kfirst + tid) * 4;
@@ -711,6 +777,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
         f |= 4;
       s_fl[tid] = (unsigned char)f;
     }
+    pml_table(G, Q, item, it, kfirst, tid, nthr);
     if (tid == 0) {
       for (int q = 0; q < kStepRing; ++q) mbar_init(smem_u32(rbar + q), 1);
       fence_mbar_init();
@@ -722,9 +789,9 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
   pdl_trigger();  // after the wait: one step's kernels start ahead, not a chain of them
   __syncthreads();
   if (S.flags & SF_FP32)
-    step_item<float>(p, S, item, it, sPn, sV, s_co, ring, s_fl, rbar);
+    step_item<float>(S, Q, item, it, sPn, sV, ring, s_fl, rbar);
   else
-    step_item<double>(p, S, item, it, sPn, sV, s_co, ring, s_fl, rbar);
+    step_item<double>(S, Q, item, it, sPn, sV, ring, s_fl, rbar);
 }
 
 // closed[x tile][y tile][plane] = 1 where a cell of the tile's plane, its halo
