@@ -18,8 +18,8 @@
 // exchange of the new P, Float64 arithmetic) runs in each; what bounds them is
 // that chain and the instructions around it, not HBM.  With the stage read
 // through shared-space addresses, on different banks, and the entries' code out
-// of the plane loop, a launch of 8 x 256^3 takes 0.82 ms without boundaries
-// (0.89 before) and 1.42 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
+// of the plane loop, a launch of 8 x 256^3 takes 0.77 ms without boundaries
+// (0.89 before) and 1.31 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
 // The plane loop's code has to stay small: a masked form of the plain update and
 // one with the x slab's memory each made it slower (1.57 and 1.66 ms).
 //
@@ -123,7 +123,7 @@ static_assert(offsetof(PmlTab, xpa) % 16 == 0 && offsetof(PmlTab, xpb) % 16 == 0
 struct Quad {
   // cell e: bit e P updated (x <= nx-2), 4+e Vx updated (1 <= x < nx), 8+e in the
   // grid (x < nx), 12+e P has x-slab memory, 16+e Vx has; bit 20: cells in both x
-  // slabs (narrow grids)
+  // slabs (narrow grids); 21 the quad lies in the grid, 22 and is stored by the thread
   uint32_t bits;
   int j, x0, r;
   int px, vx;  // x-slab memory of plane 0
@@ -159,7 +159,7 @@ template <typename R>
 __device__ __forceinline__ float4 p_update_quad(const SolveDev& S, const PmlTab& Q, const Quad& q,
                                                 const Sc<R>& g, bool pcpml, int k, int u, bool owned,
                                                 float4 P4, float4 X4, float X5, float4 Y0, float4 Y1,
-                                                float4 Z0, float4 Z1, uint32_t nib) {
+                                                float4 Z0, float4 Z1, uint32_t nib, float4 mx) {
   using A = Arith<R>;
   const bool rigid_y = q.j == S.ny - 1, rigid_z = k == S.nz - 1;
   // rigid planes use update_p! (-2V/d at the wall, no CPML, no mask); the
@@ -184,7 +184,7 @@ __device__ __forceinline__ float4 p_update_quad(const SolveDev& S, const PmlTab&
                           q.bits >> 12, owned, a, b);
       } else {
         const int o = q.px + k * Q.stride[0];
-        const float4 t = ld4(Q.rd[0] + o);
+        const float4 t = mx;
         float m[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e)
@@ -203,7 +203,7 @@ __device__ __forceinline__ float4 p_update_quad(const SolveDev& S, const PmlTab&
         if ((up >> e) & 1u) cpml_apply<R>(dy[e], m[e], a, b);
       if (owned) st4(Q.wr[1] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
-    if (Q.zp[u] >= 0) {
+    if (Q.zp[u] >= 0 && (q.bits & (1u << 21))) {
       const int o = Q.zp[u] + q.j * S.nxp + q.x0;
       const float4 t = ld4(Q.rd[2] + o);
       float m[4] = {t.x, t.y, t.z, t.w};
@@ -277,7 +277,7 @@ template <typename R>
 __device__ __forceinline__ void v_update_quad(const SolveDev& S, const PmlTab& Q, const Quad& q,
                                               const Sc<R>& g, bool vcpml, int k, int u, float4 Pc,
                                               float Pxm, float4 Pym, float4 Pzm, float4 VX, float4 VY,
-                                              float4 VZ, uint32_t nib, float4& vxo, float4& vyo,
+                                              float4 VZ, uint32_t nib, float4 mx, float4& vxo, float4& vyo,
                                               float4& vzo) {
   using A = Arith<R>;
   const uint32_t in = (q.bits >> 8) & 15u;
@@ -296,7 +296,7 @@ __device__ __forceinline__ void v_update_quad(const SolveDev& S, const PmlTab& Q
                           q.x0, q.bits >> 16, true, a, b);
       } else {
         const int o = q.vx + k * Q.stride[3];
-        const float4 t = ld4(Q.rd[3] + o);
+        const float4 t = mx;
         float m[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e)
@@ -314,7 +314,7 @@ __device__ __forceinline__ void v_update_quad(const SolveDev& S, const PmlTab& Q
         if ((in >> e) & 1u) cpml_apply<R>(dy[e], m[e], a, b);
       st4(Q.wr[4] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
-    if (Q.zv[u] >= 0) {
+    if (Q.zv[u] >= 0 && (q.bits & (1u << 22))) {
       const int o = Q.zv[u] + q.j * S.nxp + q.x0;
       const float4 t = ld4(Q.rd[5] + o);
       float m[4] = {t.x, t.y, t.z, t.w};
@@ -460,17 +460,17 @@ constexpr int kXT = 64;             // cells per x tile (4 warps)
 constexpr int kPnPitch = kStageW;   // shared new-P row: [3] = halo column, [4..] = cells
 constexpr int kStepThreads = 32 * kXT / 16;  // warps of 4 quads x 8 rows
 
-// One stage: P, Vx, Vy of a plane ([3][ty+2][kStageW]) and, from the next
+// One stage: P, Vx, Vy of a plane ([3][kMaxTy+2][kStageW]) and, from the next
 // 128-B boundary on (TMA destinations must be 128-B aligned), Vz of the next
-// plane ([ty+2][kStageW]).
-__host__ __device__ constexpr int stage_vz_offset(int cst) { return (3 * cst + 31) / 32 * 32; }
-constexpr int kStageFloats =
-    (stage_vz_offset((kMaxTy + 2) * kStageW) + (kMaxTy + 2) * kStageW + 31) / 32 * 32;
+// plane ([kMaxTy+2][kStageW]).  The rows are those of the tallest tile, so that
+// every offset in a stage is a constant.
+constexpr int kStageChan = (kMaxTy + 2) * kStageW;
+constexpr int kStageVz = (3 * kStageChan + 31) / 32 * 32;
+constexpr int kStageFloats = (kStageVz + kStageChan + 31) / 32 * 32;
 // Polls of a staged plane's bounded wait: a plane lands within microseconds,
 // so a limit far below kWaitLimit keeps a lost copy from stalling the GPU
 constexpr uint32_t kStepWaitLimit = 1u << 20;
 static_assert((kStageFloats * 4) % 128 == 0, "stages stay 128-B aligned");
-static_assert((stage_vz_offset(5 * kStageW) * 4) % 128 == 0, "Vz boxes start 128-B aligned");
 
 template <typename R>
 __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, int4 item, int it,
@@ -489,18 +489,14 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
   const int wq0 = 4 * wid, wnq = 4, wr0 = 0, wnr = kMaxTy + 1;
   const int j = j0 - 1 + r, x0 = xb + 4 * qx;
   const bool row_ok = r <= ty && j >= 0 && j < ny;
-  const bool act = row_ok && x0 < nxp;  // this thread updates a quad
+  // this thread's quad lies in the grid; the others compute on the stage's zeros
+  // (every shared address is valid) and touch no global memory
+  const bool act = row_ok && x0 < nxp;
   const bool vrow = act && r >= 1;      // ... and owns it (velocity update, stores)
   const int rb = (it - S.it_first) & 1, wb = rb ^ 1;
   const long long cs = S.chan_stride, plane = (long long)ny * nxp;
   float* fout = S.field + wb * S.buf_stride;
   const bool pcp = (S.flags & SF_PCPML) != 0, vcp = (S.flags & SF_VCPML) != 0;
-  Sc<R> g;
-  g.fq = Arith<R>::fq(S);
-  g.fv = Arith<R>::fv(S);
-  g.rdx = Arith<R>::rdx(S);
-  g.rdy = Arith<R>::rdy(S);
-  g.rdz = Arith<R>::rdz(S);
   Quad q;
   q.j = j;
   q.x0 = x0;
@@ -516,16 +512,18 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
       if (x <= nx - 2) q.bits |= 1u << e;
       if (x >= 1 && x < nx) q.bits |= 16u << e;
       if (x < nx) q.bits |= 256u << e;
-      if (pcp && x <= nx - 2 && (x < npml || x >= nx - npml)) {
+      if (act && pcp && x <= nx - 2 && (x < npml || x >= nx - npml)) {
         q.bits |= 4096u << e;
         seen |= x < npml ? 1 : 2;
       }
-      if (vcp && x >= 1 && x < nx && (x <= npml || x >= nx - npml - 1)) {
+      if (vrow && vcp && x >= 1 && x < nx && (x <= npml || x >= nx - npml - 1)) {
         q.bits |= 65536u << e;
         seen |= x <= npml ? 4 : 8;
       }
     }
     if ((seen & 3) == 3 || (seen & 12) == 12) q.bits |= 1u << 20;
+    if (act) q.bits |= 1u << 21;
+    if (vrow) q.bits |= 1u << 22;
     if (act && pcp) {
       q.px = j * S.npp + ((seen & 1) ? x0 : (int)S.psi_p_side[0] + x0 - S.xs1p);
       const int ys = j < npml ? 0 : (j >= ny - npml ? 1 : -1);
@@ -559,11 +557,10 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
   const int kfirst = z0 > 0 ? z0 - 1 : z0;
   // The stage of plane k, staged by TMA into a ring of kStepRing slots, holds
   // P, Vx, Vy of plane k and Vz of plane k+1 (channel slot 3; not loaded for
-  // k = nz-1, where the loop supplies the zeros itself), rows j0-1 .. j0+ty,
+  // k = nz-1, whose update does not read it), rows j0-1 .. j0+kMaxTy,
   // x = xb-4 .. xb+67, zero outside the grid.  Vz of plane k is carried in
   // registers from the previous stage.
-  const int cst = (ty + 2) * kStageW;         // channel stride in a stage
-  const int vzo = stage_vz_offset(cst);       // Vz of the next plane in a stage
+  constexpr int cst = kStageChan, vzo = kStageVz;
   const int so = r * kStageW + 4 + 4 * qx;    // this quad in a stage channel
   const char* maps = static_cast<const char*>(S.fmap) + rb * 256;  // {P,Vx,Vy box; Vz box}
   auto slot_of = [&](int k) { return (k - kfirst) % kStepRing; };
@@ -594,38 +591,50 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
     if (act) Z0 = ldg4(vz0);
     if (hcol) Zh = __ldg(vz0 - 1);
   }
+  // The x-slab memory of a quad is read ahead of its use: the p side's of plane
+  // k+1 during the velocity update of plane k, the v side's of plane k during its
+  // pressure update.  One warp of every x-end tile would otherwise wait for two
+  // more reads of global memory per plane than the other three (1.39 ms without
+  // this at 8 x 256^3 with CPML and a sphere, 1.31 with it).
+  const bool pxm = (q.bits & 0xF000u) && !(q.bits & (1u << 20));
+  const bool vxm = (q.bits & 0xF0000u) && !(q.bits & (1u << 20));
+  float4 mpx = make_float4(0.f, 0.f, 0.f, 0.f), mvx = mpx;
+  if (pxm) mpx = ld4(Q.rd[0] + q.px + kfirst * Q.stride[0]);
   for (int k = kfirst; k < z1; ++k) {
     const bool prologue = k < z0;
+    if (vxm) mvx = ld4(Q.rd[3] + q.vx + k * Q.stride[3]);
     const int u = k - kfirst;
     float* pn = sPn + (k & 1) * (kMaxTy + 1) * kPnPitch;
     const float* st = ring + slot_of(k) * kStageFloats;
     wait(k);
     const int fl = s_fl[u];
     const bool has_mask = (fl & 4) != 0;  // elsewhere every cell of the tile's plane is open
-    const bool pplane = k != nz - 1 && (!pcp || (k >= npml && k < nz - npml));
-    const bool vplane = k >= 1 && (!vcp || (k > npml && k < nz - npml - 1));
-    const bool wplain = wplain_rx && pplane && (prologue || vplane) && !has_mask;
-    float4 Pn = make_float4(0.f, 0.f, 0.f, 0.f), X4 = Pn, Y0 = Pn, Z1 = Pn;
+    const bool wplain = wplain_rx && (fl & 12) == 8;
     uint32_t nib = 0xFFFFu;
-    if (act) {
-      const float4 P4 = ld4(st + so);
-      X4 = ld4(st + cst + so);
-      Y0 = ld4(st + 2 * cst + so);
-      const float X5 = st[cst + so + 4];
-      const float4 Y1 = ld4(st + 2 * cst + so + kStageW);
-      Z1 = k + 1 < nz ? ld4(st + vzo + so) : Pn;
-      if (has_mask)
-        nib = (__ldg(S.mask_bits + ((long long)k * ny + j) * S.mw + (x0 >> 3)) >> ((x0 & 4) * 4)) &
-              0xFFFFu;
-      if (wplain)
-        Pn = p_plain_quad<R>(g, P4, X4, X5, Y0, Y1, Z0, Z1);
-      else
-        Pn = p_update_quad<R>(S, Q, q, g, pcp, k, u, vrow && !prologue, P4, X4, X5, Y0, Y1, Z0, Z1,
-                              nib);
-      st4(pn + pq, Pn);
-    }
+    Sc<R> g;  // (read again in each phase: registers are what the loop is short of)
+    g.fq = Arith<R>::fq(S);
+    g.fv = Arith<R>::fv(S);
+    g.rdx = Arith<R>::rdx(S);
+    g.rdy = Arith<R>::rdy(S);
+    g.rdz = Arith<R>::rdz(S);
+    const float4 P4 = ld4(st + so);
+    const float4 X4 = ld4(st + cst + so);
+    const float4 Y0 = ld4(st + 2 * cst + so);
+    const float X5 = st[cst + so + 4];
+    const float4 Y1 = ld4(st + 2 * cst + so + kStageW);
+    const float4 Z1 = ld4(st + vzo + so);
+    if (has_mask && act)
+      nib = (__ldg(S.mask_bits + ((long long)k * ny + j) * S.mw + (x0 >> 3)) >> ((x0 & 4) * 4)) &
+            0xFFFFu;
+    float4 Pn;
+    if (wplain)
+      Pn = p_plain_quad<R>(g, P4, X4, X5, Y0, Y1, Z0, Z1);
+    else
+      Pn = p_update_quad<R>(S, Q, q, g, pcp, k, u, vrow && !prologue, P4, X4, X5, Y0, Y1, Z0, Z1, nib,
+                            mpx);
+    st4(pn + pq, Pn);
     if (hcol) {
-      const float Zh1 = k + 1 < nz ? st[vzo + so - 1] : 0.f;
+      const float Zh1 = st[vzo + so - 1];
       if (wplain && hplain_x)
         pn[pq - 1] = p_plain<R>(st[so - 1], __fsub_rn(X4.x, st[cst + so - 1]),
                                 __fsub_rn(st[2 * cst + so - 1 + kStageW], st[2 * cst + so - 1]),
@@ -636,25 +645,29 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
       Zh = Zh1;
     }
     __syncthreads();
+    if (pxm && k + 1 < z1) mpx = ld4(Q.rd[0] + q.px + (k + 1) * Q.stride[0]);
     // every read of plane k's stage is done: refill its slot
     if (tid == 0 && k + kStepRing < z1) issue(k + kStepRing);
     // ---- q channel: inject/record on the new P (forward.jl:92) ----
     if (fl & 1) {
       apply_entries(S, T, k, 0, xb - 1, xb + kXT, xb, !prologue, it, pn + 4 - xb, kPnPitch);
       __syncthreads();
-      if (act) Pn = ld4(pn + pq);
+      Pn = ld4(pn + pq);
     }
     if (!prologue) {
-      float4 vx = Pn, vy = Pn, vz = Pn;
-      if (vrow) {
-        const float Pxm = pn[pq - 1];
-        const float4 Pym = ld4(pn + pq - kPnPitch);
-        if (wplain) {
-          v_plain_quad<R>(g, Pn, Pxm, Pym, Pzm, X4, Y0, Z0, vx, vy, vz);
-        } else {
-          v_update_quad<R>(S, Q, q, g, vcp, k, u, Pn, Pxm, Pym, Pzm, X4, Y0, Z0, nib, vx, vy, vz);
-        }
-      }
+      float4 vx, vy, vz;
+      Sc<R> g;
+      g.fq = Arith<R>::fq(S);
+      g.fv = Arith<R>::fv(S);
+      g.rdx = Arith<R>::rdx(S);
+      g.rdy = Arith<R>::rdy(S);
+      g.rdz = Arith<R>::rdz(S);
+      const float Pxm = pn[pq - 1];
+      const float4 Pym = ld4(pn + pq - kPnPitch);
+      if (wplain)
+        v_plain_quad<R>(g, Pn, Pxm, Pym, Pzm, X4, Y0, Z0, vx, vy, vz);
+      else
+        v_update_quad<R>(S, Q, q, g, vcp, k, u, Pn, Pxm, Pym, Pzm, X4, Y0, Z0, nib, mvx, vx, vy, vz);
       // ---- f channel: inject/record on the new V (forward.jl:111-115) ----
       if (fl & 2) {
         float* sVx = sV;
@@ -681,11 +694,16 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
         float* o = fout + k * plane + rowoff;
         stcs4(o, Pn);
         stcs4(o + cs, vx);
-        // rigid mirrors (forward.jl:134-137): Vy[:,1,:] = -Vy[:,2,:], Vz[:,:,1] = -Vz[:,:,2]
-        if (j != 0) stcs4(o + 2 * cs, vy);
-        if (j == 1) st4(o + 2 * cs - nxp, neg4(vy));
-        if (k != 0) stcs4(o + 3 * cs, vz);
-        if (k == 1) st4(o + 3 * cs - plane, neg4(vz));
+        if (wplain) {
+          stcs4(o + 2 * cs, vy);
+          stcs4(o + 3 * cs, vz);
+        } else {
+          // rigid mirrors (forward.jl:134-137): Vy[:,1,:] = -Vy[:,2,:], Vz[:,:,1] = -Vz[:,:,2]
+          if (j != 0) stcs4(o + 2 * cs, vy);
+          if (j == 1) st4(o + 2 * cs - nxp, neg4(vy));
+          if (k != 0) stcs4(o + 3 * cs, vz);
+          if (k == 1) st4(o + 3 * cs - plane, neg4(vz));
+        }
       }
     }
     Pzm = Pn;
@@ -751,10 +769,10 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
   // (an index, not a rounded pointer, so that the compiler keeps shared-space accesses)
   float* ring = dyn_smem + ((0u - smem_u32(dyn_smem)) & 127u) / 4u;
   __shared__ __align__(8) uint64_t rbar[kStepRing];
-  __shared__ __align__(16) float sPn[2 * (kMaxTy + 1) * kPnPitch];
+  __shared__ __align__(16) float sPn[(2 * (kMaxTy + 1) + 1) * kPnPitch];  // (a row before the first)
   __shared__ __align__(16) float sV[3 * kMaxTy * kXT];
   __shared__ __align__(16) PmlTab Q;
-  __shared__ unsigned char s_fl[kMaxZc + 1];  // planes kfirst ..: 1 q, 2 f entries, 4 closed cells
+  __shared__ unsigned char s_fl[kMaxZc + 1];  // planes kfirst ..: 1 q, 2 f entries, 4 closed cells, 8 plain
   __shared__ __align__(16) SolveDev S;  // the solve descriptor, read in the hot loop
   const int4 item = p.items[blockIdx.x];
   const SolveDev& G = p.solves[item.x];
@@ -775,6 +793,9 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
       if (G.closed && G.closed[((long long)(item.y >> 16) * G.nty + (item.y & 0xFFFF)) * G.nz +
                                kfirst + tid])
         f |= 4;
+      // planes without z-slab memory, mirror or rigid wall
+      const int zm = (G.flags & (SF_PCPML | SF_VCPML)) ? G.npml + 1 : 1, k = kfirst + tid;
+      if (k >= max(zm, 2) && k < G.nz - zm) f |= 8;
       s_fl[tid] = (unsigned char)f;
     }
     pml_table(G, Q, item, it, kfirst, tid, nthr);
@@ -789,9 +810,9 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
   pdl_trigger();  // after the wait: one step's kernels start ahead, not a chain of them
   __syncthreads();
   if (S.flags & SF_FP32)
-    step_item<float>(S, Q, item, it, sPn, sV, ring, s_fl, rbar);
+    step_item<float>(S, Q, item, it, sPn + kPnPitch, sV, ring, s_fl, rbar);
   else
-    step_item<double>(S, Q, item, it, sPn, sV, ring, s_fl, rbar);
+    step_item<double>(S, Q, item, it, sPn + kPnPitch, sV, ring, s_fl, rbar);
 }
 
 // closed[x tile][y tile][plane] = 1 where a cell of the tile's plane, its halo

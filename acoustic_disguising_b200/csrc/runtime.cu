@@ -247,8 +247,8 @@ template int* solve_dalloc<int>(Solve&, size_t, int&);
 template double* solve_dalloc<double>(Solve&, size_t, int&);
 
 // The step kernel's TMA descriptors of the two field buffers: 4D tiled maps
-// (x: nxp, y: ny, z: nz, channel: 4) with the staged boxes (kStageW, ty+2, 1, 3)
-// for P, Vx, Vy and (kStageW, ty+2, 1, 1) for Vz, zero fill outside the grid.  cuTensorMapEncodeTiled comes from the
+// (x: nxp, y: ny, z: nz, channel: 4) with the staged boxes (kStageW, max ty + 2, 1, 3)
+// for P, Vx, Vy and (kStageW, max ty + 2, 1, 1) for Vz, zero fill outside the grid.  cuTensorMapEncodeTiled comes from the
 // driver through the runtime's entry-point query (no link against libcuda).
 static int make_field_maps(Solve& s) {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
@@ -270,7 +270,7 @@ static int make_field_maps(Solve& s) {
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   for (int m4 = 0; m4 < 4; ++m4) {  // buffer b = m4 / 2; box of 3 channels or of Vz
     const int b = m4 / 2;
-    const cuuint32_t box[4] = {(cuuint32_t)kStageW, (cuuint32_t)(d.ty + 2), 1,
+    const cuuint32_t box[4] = {(cuuint32_t)kStageW, (cuuint32_t)(step_max_ty() + 2), 1,
                                (cuuint32_t)(m4 % 2 ? 1 : 3)};
     CUtensorMap* m = reinterpret_cast<CUtensorMap*>(s.fmap_host + 128 * m4);
     const CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, d.field + b * d.buf_stride,
