@@ -19,7 +19,7 @@
 // that chain and the instructions around it, not HBM.  With the stage read
 // through shared-space addresses, on different banks, and the entries' code out
 // of the plane loop, a launch of 8 x 256^3 takes 0.77 ms without boundaries
-// (0.89 before) and 1.31 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
+// (0.89 before) and 1.30 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
 // The plane loop's code has to stay small: a masked form of the plain update and
 // one with the x slab's memory each made it slower (1.57 and 1.66 ms).
 //
@@ -130,6 +130,14 @@ struct Quad {
   int py, vy;  // y-slab memory of plane 0, -1: none
 };
 
+// Memory of cells that are not updated stays as it was read.
+__device__ __forceinline__ void keep_rest(float (&m)[4], float4 t, uint32_t upd) {
+  if (!(upd & 1u)) m[0] = t.x;
+  if (!(upd & 2u)) m[1] = t.y;
+  if (!(upd & 4u)) m[2] = t.z;
+  if (!(upd & 8u)) m[3] = t.w;
+}
+
 // x-slab memory of a quad with cells in both slabs: cell by cell.
 template <typename R>
 __device__ __forceinline__ void x_slabs_narrow(R (&d)[4], const PmlTab& Q, int arr, int pitch,
@@ -199,8 +207,8 @@ __device__ __forceinline__ float4 p_update_quad(const SolveDev& S, const PmlTab&
       float m[4] = {t.x, t.y, t.z, t.w};
       const float a = Q.ypa[q.r], b = Q.ypb[q.r];
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if ((up >> e) & 1u) cpml_apply<R>(dy[e], m[e], a, b);
+      for (int e = 0; e < 4; ++e) cpml_apply<R>(dy[e], m[e], a, b);
+      if (up != 15u) keep_rest(m, t, up);
       if (owned) st4(Q.wr[1] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
     if (Q.zp[u] >= 0 && (q.bits & (1u << 21))) {
@@ -209,8 +217,8 @@ __device__ __forceinline__ float4 p_update_quad(const SolveDev& S, const PmlTab&
       float m[4] = {t.x, t.y, t.z, t.w};
       const float a = Q.zpa[u], b = Q.zpb[u];
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if ((up >> e) & 1u) cpml_apply<R>(dz[e], m[e], a, b);
+      for (int e = 0; e < 4; ++e) cpml_apply<R>(dz[e], m[e], a, b);
+      if (up != 15u) keep_rest(m, t, up);
       if (owned) st4(Q.wr[2] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
   }
@@ -310,8 +318,8 @@ __device__ __forceinline__ void v_update_quad(const SolveDev& S, const PmlTab& Q
       float m[4] = {t.x, t.y, t.z, t.w};
       const float a = Q.yva[q.r], b = Q.yvb[q.r];
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if ((in >> e) & 1u) cpml_apply<R>(dy[e], m[e], a, b);
+      for (int e = 0; e < 4; ++e) cpml_apply<R>(dy[e], m[e], a, b);
+      if (in != 15u) keep_rest(m, t, in);
       st4(Q.wr[4] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
     if (Q.zv[u] >= 0 && (q.bits & (1u << 22))) {
@@ -320,8 +328,8 @@ __device__ __forceinline__ void v_update_quad(const SolveDev& S, const PmlTab& Q
       float m[4] = {t.x, t.y, t.z, t.w};
       const float a = Q.zva[u], b = Q.zvb[u];
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if ((in >> e) & 1u) cpml_apply<R>(dz[e], m[e], a, b);
+      for (int e = 0; e < 4; ++e) cpml_apply<R>(dz[e], m[e], a, b);
+      if (in != 15u) keep_rest(m, t, in);
       st4(Q.wr[5] + o, make_float4(m[0], m[1], m[2], m[3]));
     }
   }
@@ -494,7 +502,8 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
   const bool act = row_ok && x0 < nxp;
   const bool vrow = act && r >= 1;      // ... and owns it (velocity update, stores)
   const int rb = (it - S.it_first) & 1, wb = rb ^ 1;
-  const long long cs = S.chan_stride, plane = (long long)ny * nxp;
+  const long long cs = S.chan_stride;
+  const int plane = ny * nxp;
   float* fout = S.field + wb * S.buf_stride;
   const bool pcp = (S.flags & SF_PCPML) != 0, vcp = (S.flags & SF_VCPML) != 0;
   Quad q;
@@ -551,7 +560,7 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
     wplain_rx = ok;
     hplain_x = xb - 1 >= p_xmin && xb - 1 <= p_xmax;  // the halo column's cells
   }
-  const long long rowoff = (long long)(row_ok ? j : 0) * nxp + x0;
+  const int rowoff = (row_ok ? j : 0) * nxp + x0;
   const int pq = r * kPnPitch + 4 + 4 * qx;  // this quad in a shared new-P plane
   const int z0 = item.z, z1 = item.w;
   const int kfirst = z0 > 0 ? z0 - 1 : z0;
@@ -587,7 +596,7 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
   const bool hcol = qx == 0 && r >= 1 && row_ok && xb > 0;
   float Zh = 0.f;
   {
-    const float* vz0 = S.field + rb * S.buf_stride + 3 * cs + kfirst * plane + rowoff;
+    const float* vz0 = S.field + rb * S.buf_stride + 3 * cs + (long long)kfirst * plane + rowoff;
     if (act) Z0 = ldg4(vz0);
     if (hcol) Zh = __ldg(vz0 - 1);
   }
@@ -606,7 +615,7 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
     const int u = k - kfirst;
     float* pn = sPn + (k & 1) * (kMaxTy + 1) * kPnPitch;
     const float* st = ring + slot_of(k) * kStageFloats;
-    wait(k);
+    if (!mbar_try_wait(smem_u32(rbar) + 8u * (u & 1), (uint32_t)(u >> 1) & 1u)) wait(k);
     const int fl = s_fl[u];
     const bool has_mask = (fl & 4) != 0;  // elsewhere every cell of the tile's plane is open
     const bool wplain = wplain_rx && (fl & 12) == 8;
@@ -691,7 +700,7 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
         }
       }
       if (vrow) {
-        float* o = fout + k * plane + rowoff;
+        float* o = fout + ((long long)k * plane + rowoff);
         stcs4(o, Pn);
         stcs4(o + cs, vx);
         if (wplain) {
