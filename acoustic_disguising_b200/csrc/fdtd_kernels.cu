@@ -29,6 +29,7 @@
 // difference is x*(1/dx) in place of x/dx.  Arith<float> is the all-Float32
 // variant.  Injection/recording (derivatives.jl:30-60) is pure Float32 with
 // separate multiply and add, as the reference computes it.
+#include <algorithm>
 #include <cstddef>
 
 #include "adf_internal.h"
@@ -861,42 +862,59 @@ cudaError_t launch_mask_tiles(const SolveDev& d, unsigned char* closed, cudaStre
 }
 
 // Per-step trace assembly (derivatives.jl:51-56 record sums in corner order,
-// v2vn! :85-90, vn2v! :92-97 into row it+1).
-__global__ void adf_fdtd_epilogue_kernel(const EpiParams p) {
+// v2vn! :85-90, vn2v! :92-97 into row it+1).  Four lanes per transceiver, one per
+// channel: the kernel does next to nothing and its time is the chain of its reads
+// (a thread per transceiver, through the descriptor in global memory and corner by
+// corner, took 9.9 us cold between a step and the next).  Places are looked up
+// before the wait for the step kernel; after it, one round of reads is left.
+constexpr int kEpiThreads = 128;
+__global__ void __launch_bounds__(kEpiThreads) adf_fdtd_epilogue_kernel(const EpiParams p) {
   pdl_trigger();
-  pdl_wait();
   const SolveDev& S = p.solves[blockIdx.y];
+  const int c = threadIdx.x & 3, tx = (int)(blockIdx.x * kEpiThreads + threadIdx.x) >> 2;
+  const int ntx = S.ntx, nt = S.nt, stop = S.it_stop;
+  const bool on = tx < ntx;
+  float* const rec = S.rec[c];
+  float* const vn_rec = S.vn_rec;
+  const float* const vn_src = S.vn_src;
+  float* const src = S.src[c];
+  const float4* const cb = reinterpret_cast<const float4*>(S.contrib + ((long long)c * ntx + tx) * 8);
+  const bool inb = on && S.inb[c * ntx + tx];
+  const float d = on ? S.dir[4 * tx + c] : 0.0f;
+  // vn2v into row it+1; a GF solve's driven columns get it when the
+  // extrapolation has written their vn_src (gf_finish)
+  const bool v2 = on && c > 0 && vn_src && (!(S.flags & SF_GF) || S.gf_col[tx] == 0);
+  pdl_wait();
   const int it = S.it_base + p.step;
-  if (it > S.it_stop) return;
-  const int ntx = S.ntx;
-  const bool gf = (S.flags & SF_GF) != 0;
-  for (int tx = blockIdx.x * blockDim.x + threadIdx.x; tx < ntx; tx += gridDim.x * blockDim.x) {
-    const long long row = (long long)(it - 1) * ntx + tx;
-    float r[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      // a record buffer that is not kept starts every row at zero, as the
-      // reference's freshly packed rec (= src*0) does
-      r[c] = S.rec[c] ? S.rec[c][row] : 0.0f;
-      if (S.inb[c * ntx + tx]) {
-        const float* cb = S.contrib + ((long long)c * ntx + tx) * 8;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) r[c] = __fadd_rn(r[c], cb[k]);
-        if (S.rec[c]) S.rec[c][row] = r[c];
-      }
-    }
-    const float* d = S.dir + 4 * tx;
-    S.vn_rec[row] =
-        __fadd_rn(__fadd_rn(__fmul_rn(r[1], d[1]), __fmul_rn(r[2], d[2])), __fmul_rn(r[3], d[3]));
-    // vn2v! into row it+1; a GF solve's driven columns get it when the
-    // extrapolation has written their vn_src (gf_finish)
-    if (S.vn_src && it < S.nt && (!gf || S.gf_col[tx] == 0)) {
-      const long long nr = row + ntx;
-      const float vs = S.vn_src[nr];
-#pragma unroll
-      for (int c = 1; c <= 3; ++c) S.src[c][nr] = __fadd_rn(S.src[c][nr], __fmul_rn(vs, d[c]));
-    }
+  if (it > stop) return;
+  const long long row = (long long)(it - 1) * ntx + tx;
+  // a record buffer that is not kept starts every row at zero, as the
+  // reference's freshly packed rec (= src*0) does
+  float r = on && rec ? rec[row] : 0.0f;
+  float vs = 0.0f, sv = 0.0f;
+  if (v2 && it < nt) {
+    vs = vn_src[row + ntx];
+    sv = src[row + ntx];
   }
+  if (inb) {
+    const float4 lo = cb[0], hi = cb[1];
+    r = __fadd_rn(r, lo.x);
+    r = __fadd_rn(r, lo.y);
+    r = __fadd_rn(r, lo.z);
+    r = __fadd_rn(r, lo.w);
+    r = __fadd_rn(r, hi.x);
+    r = __fadd_rn(r, hi.y);
+    r = __fadd_rn(r, hi.z);
+    r = __fadd_rn(r, hi.w);
+    if (rec) rec[row] = r;
+  }
+  // vn = rec1 d1 + rec2 d2 + rec3 d3, in that order
+  const float m = __fmul_rn(r, d);
+  const float m1 = __shfl_sync(0xffffffffu, m, (threadIdx.x & 28) + 1);
+  const float m2 = __shfl_sync(0xffffffffu, m, (threadIdx.x & 28) + 2);
+  const float m3 = __shfl_sync(0xffffffffu, m, (threadIdx.x & 28) + 3);
+  if (on && c == 0) vn_rec[row] = __fadd_rn(__fadd_rn(m1, m2), m3);
+  if (v2 && it < nt) src[row + ntx] = __fadd_rn(sv, __fmul_rn(vs, d));
 }
 
 // Advances it_base of every solve by `by` steps: the last node of a captured
@@ -1318,11 +1336,9 @@ cudaError_t launch_gf_far(const EpiParams& p, int max_blocks, int max_nsrc, cuda
 }
 
 cudaError_t launch_epilogue(const EpiParams& p, int max_ntx, bool overlap, cudaStream_t s) {
-  int threads = 128;
-  int gx = (max_ntx + threads - 1) / threads;
-  if (gx < 1) gx = 1;
-  return launch_overlapped(adf_fdtd_epilogue_kernel, dim3(gx, p.n_solves), dim3(threads), 0, overlap,
-                           s, p);
+  const int gx = std::max(1, (4 * max_ntx + kEpiThreads - 1) / kEpiThreads);
+  return launch_overlapped(adf_fdtd_epilogue_kernel, dim3(gx, p.n_solves), dim3(kEpiThreads), 0,
+                           overlap, s, p);
 }
 
 }  // namespace adf
