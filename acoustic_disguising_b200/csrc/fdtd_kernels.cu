@@ -31,6 +31,7 @@
 // separate multiply and add, as the reference computes it.
 #include <algorithm>
 #include <cstddef>
+#include <type_traits>
 
 #include "adf_internal.h"
 #include "ptx_util.h"
@@ -1121,14 +1122,41 @@ __global__ void __launch_bounds__(256, 4) adf_gf_extrapolate_kernel(const EpiPar
 // (T_b = min(it0+b, ngf)).  Lags b+1 .. T_b-1 read input-history rows
 // it0-1+b-lag <= it0-2, all complete before the block starts, so they are
 // summed here once for the whole block: a contraction over (receiver, lag)
-// of the block's 32 steps x 32 sources, which reads each tensor slice once
+// of the block's 32 steps x 64 sources, which reads each tensor slice once
 // per block instead of once per step.  Lags 0..b, whose rows appear during
 // the block, stay in adf_gf_extrapolate_kernel.  FP64 fused multiply-adds;
 // one partial per (source, receiver split, step), added in split order by
-// adf_gf_reduce_kernel.  Input-history kinds only.
+// adf_gf_far_combine_kernel.  Input-history kinds only.
+//
+// Block: 64 sources; two groups of four warps, each with half of the block's
+// receivers.  A thread holds 2 sources x 8 steps x 2 tensors, so
+// that one staged lag costs it 4 tensor values and one new history value for 32
+// FMAs (the 8 steps' history values are one window that moves by a row per lag):
+// with 4 steps a thread the shared loads, not the FP64 pipe, were the bound, and
+// nothing read the next chunk while one was summed.  256 x 256 x 256 map, lags to
+// 255, cold: 245 us a block before, 128 here, 64 at the FP64 pipe's rate.
 constexpr int kGfLC = 32;  // lags per staged chunk
 constexpr int kGfOT = 64;  // sources per tile (two per thread)
-__global__ void __launch_bounds__(256) adf_gf_far_kernel(const EpiParams p) {
+constexpr int kGfGroup = 128;
+struct GfFarStage {  // a chunk of one receiver
+  float g[2][kGfLC][kGfOT + 1];  // the two tensors, lag-major, padded against conflicts
+  double h[kGfLC + kGfBlock];    // history rows
+};
+// asynchronous copies of 4 and 8 bytes, zeros where !in
+__device__ __forceinline__ void copy4(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src),
+               "r"(in ? 4 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void copy8(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src),
+               "r"(in ? 8 : 0)
+               : "memory");
+}
+constexpr size_t kGfFarSmem = 4 * sizeof(GfFarStage);  // two groups, two buffers each
+static_assert(kGfFarSmem >= 32 * kGfGroup * sizeof(double), "the groups' exchange");
+static_assert(sizeof(GfFarStage) % 16 == 0 && offsetof(GfFarStage, h) % 8 == 0, "aligned copies");
+__global__ void __launch_bounds__(2 * kGfGroup, 2) adf_gf_far_kernel(const EpiParams p) {
   const SolveDev& S = p.solves[blockIdx.y];
   const int it0 = S.it_base + p.step;
   if (S.gf_rs <= 0 || it0 > S.it_stop || it0 >= S.nt || !(S.flags & SF_GF) || (S.flags & SF_GF_TC))
@@ -1138,78 +1166,115 @@ __global__ void __launch_bounds__(256) adf_gf_far_kernel(const EpiParams p) {
   if (ot * kGfOT >= nout) return;
   const int nt = S.nt, ngf = S.gf_nt, n1 = S.gf_n1, nin = S.gf_nin;
   const bool pv = S.gf_kind == ADF_GF_PV_FROM_PIN_;
-  const int r0 = (int)((long long)nin * rsi / rsn), r1 = (int)((long long)nin * (rsi + 1) / rsn);
-  // thread: sources ol and ol+32 of the tile, steps b = bg + 8q of the block
-  const int ol = (int)threadIdx.x & 31, bg = (int)threadIdx.x >> 5;
-  __shared__ double sG[2][kGfLC][kGfOT + 1];   // lag-major, Float64, padded against conflicts
-  __shared__ double sH[kGfLC + kGfBlock - 1];  // history rows of the chunk
-  double acc[2][2][4];
+  const int grp = (int)threadIdx.x / kGfGroup, tid = (int)threadIdx.x % kGfGroup;
+  // this group's half of the block's receivers
+  const int r0 = (int)((long long)nin * (2 * rsi + grp) / (2 * rsn));
+  const int r1 = (int)((long long)nin * (2 * rsi + grp + 1) / (2 * rsn));
+  const int ol = tid & 31, b0 = 8 * (tid >> 5);  // sources ol and ol+32, steps b0 .. b0+7
+  extern __shared__ __align__(16) unsigned char gf_smem[];
+  GfFarStage* const stage = reinterpret_cast<GfFarStage*>(gf_smem) + 2 * grp;  // [buffer]
+  double acc[2][2][8];  // tensor, source, step
 #pragma unroll
   for (int t = 0; t < 2; ++t)
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[t][h][q] = 0.0;
+      for (int q = 0; q < 8; ++q) acc[t][h][q] = 0.0;
   const int lag_hi = min(it0 + kGfBlock - 1, ngf) - 1;  // largest lag any step of the block uses
-  for (int r = r0; r < r1; ++r) {
-    const double* hist = S.gf_pin + (long long)r * nt;
-    for (int l0 = 1; l0 <= lag_hi; l0 += kGfLC) {
-      __syncthreads();  // the previous chunk has been used
-      for (int i = threadIdx.x; i < kGfOT * kGfLC; i += blockDim.x) {
-        const int oo = i / kGfLC, ll = i - oo * kGfLC;  // lag fastest: coalesced reads
-        const int lag = l0 + ll, og = ot * kGfOT + oo;
-        float v0 = 0.f, v1 = 0.f;
-        if (lag <= lag_hi && og < nout) {
-          const long long col = pv ? (long long)ngf * (og + (long long)n1 * r)
-                                   : (long long)ngf * (r + (long long)n1 * og);
-          v0 = S.gf_t[0][col + lag];
-          v1 = S.gf_t[1][col + lag];
-        }
-        sG[0][ll][oo] = (double)v0;
-        sG[1][ll][oo] = (double)v1;
-      }
-      // rows it0-1+b-lag of this chunk lie in [hlo, hlo + kGfLC + kGfBlock - 2]
-      const int hlo = it0 - l0 - kGfLC;
-      for (int i = threadIdx.x; i < kGfLC + kGfBlock - 1; i += blockDim.x) {
-        const int row = hlo + i;
-        sH[i] = (row >= 0 && row < nt) ? hist[row] : 0.0;
-      }
-      __syncthreads();
-      const bool full = l0 >= kGfBlock && l0 + kGfLC <= min(it0, ngf);
-      for (int ll = 0; ll < kGfLC; ++ll) {
-        const int lag = l0 + ll;
-        const double g00 = sG[0][ll][ol], g01 = sG[0][ll][ol + 32];
-        const double g10 = sG[1][ll][ol], g11 = sG[1][ll][ol + 32];
+  const int nch = (lag_hi + kGfLC - 1) / kGfLC;         // chunks of lags 1 .. lag_hi
+  const int total = (r1 - r0) * nch;
+  // chunk i: receiver r0 + i / nch, lags 1 + 32 (i % nch) ..; copied a chunk ahead,
+  // the lane the lag, so that a source's 32 values are one coalesced row
+  const int ll = tid & 31, ow = tid >> 5;
+  auto fetch = [&](int i) {
+    GfFarStage& d = stage[i & 1];
+    const int r = r0 + i / nch, l0 = 1 + (i % nch) * kGfLC, lag = l0 + ll;
+    const long long step = 4ll * (pv ? (long long)ngf : (long long)ngf * n1);
+    long long g = lag + (pv ? (long long)ngf * (ot * kGfOT + ow + (long long)n1 * r)
+                            : (long long)ngf * (r + (long long)n1 * (ot * kGfOT + ow)));
+#pragma unroll 4
+    for (int s = 0; s < kGfOT / 4; ++s, g += step) {
+      const bool in = lag <= lag_hi && ot * kGfOT + ow + 4 * s < nout;
+      copy4(&d.g[0][ll][ow + 4 * s], S.gf_t[0] + (in ? g : 0), in);
+      copy4(&d.g[1][ll][ow + 4 * s], S.gf_t[1] + (in ? g : 0), in);
+    }
+    // rows it0-1+b-lag of this chunk lie in [it0 - l0 - kGfLC, + kGfLC + kGfBlock - 2]
+    if (tid < kGfLC + kGfBlock) {
+      const int row = it0 - l0 - kGfLC + tid;
+      const bool in = row >= 0 && row < nt;
+      copy8(&d.h[tid], S.gf_pin + (in ? (long long)r * nt + row : 0), in);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // the groups' barriers are their own: their halves may differ by a receiver
+  auto sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(kGfGroup) : "memory"); };
+  if (total > 0) fetch(0);
+  for (int i = 0; i < total; ++i) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    sync();  // chunk i has landed for all, chunk i-1 has been used by all
+    if (i + 1 < total) fetch(i + 1);
+    const GfFarStage& d = stage[i & 1];
+    const int l0 = 1 + (i % nch) * kGfLC;
+    // past every step of the block and below every step's T, or checked
+    const bool full = l0 >= kGfBlock && l0 + kGfLC <= min(it0, ngf);
+    double h[8];  // rows of steps b0 .. b0+7 at the current lag
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int b = bg + 8 * q;
-          // past every step of the block and below every step's T, or checked
-          if (full || (lag > b && lag < min(it0 + b, ngf))) {
-            const double h = sH[b + kGfLC - 1 - ll];
-            acc[0][0][q] = __fma_rn(g00, h, acc[0][0][q]);
-            acc[0][1][q] = __fma_rn(g01, h, acc[0][1][q]);
-            acc[1][0][q] = __fma_rn(g10, h, acc[1][0][q]);
-            acc[1][1][q] = __fma_rn(g11, h, acc[1][1][q]);
+    for (int q = 0; q < 8; ++q) h[q] = d.h[b0 + q + kGfLC - 1];
+    auto lags = [&](auto checked) {
+#pragma unroll 8
+      for (int k = 0; k < kGfLC; ++k) {
+        const double a0 = d.g[0][k][ol], a1 = d.g[0][k][ol + 32], c0 = d.g[1][k][ol],
+                     c1 = d.g[1][k][ol + 32];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int lag = l0 + k, b = b0 + q;
+          if (!decltype(checked)::value || (lag > b && lag < min(it0 + b, ngf))) {
+            acc[0][0][q] = __fma_rn(a0, h[q], acc[0][0][q]);
+            acc[0][1][q] = __fma_rn(a1, h[q], acc[0][1][q]);
+            acc[1][0][q] = __fma_rn(c0, h[q], acc[1][0][q]);
+            acc[1][1][q] = __fma_rn(c1, h[q], acc[1][1][q]);
           }
         }
+#pragma unroll
+        for (int q = 7; q > 0; --q) h[q] = h[q - 1];
+        h[0] = d.h[max(b0 + kGfLC - 2 - k, 0)];
       }
-    }
+    };
+    if (full)
+      lags(std::false_type());
+    else
+      lags(std::true_type());
   }
+  // the second group's sums are added to the first's
+  __syncthreads();  // every group is done with its stages
+  double* const other = reinterpret_cast<double*>(gf_smem) + tid;  // [32][kGfGroup]
+  if (grp == 1) {
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) other[((t * 2 + h) * 8 + q) * kGfGroup] = acc[t][h][q];
+  }
+  __syncthreads();
+  if (grp == 1) return;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int o = ot * kGfOT + ol + 32 * h;
     if (o >= nout) continue;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      double* pp = S.gf_far + (((long long)o * rsn + rsi) * kGfBlock + bg + 8 * q) * 2;
-      pp[0] = acc[0][h][q];
-      pp[1] = acc[1][h][q];
+    for (int q = 0; q < 8; ++q) {
+      double* pp = S.gf_far + (((long long)o * rsn + rsi) * kGfBlock + b0 + q) * 2;
+      pp[0] = __dadd_rn(acc[0][h][q], other[(h * 8 + q) * kGfGroup]);
+      pp[1] = __dadd_rn(acc[1][h][q], other[((2 + h) * 8 + q) * kGfGroup]);
     }
   }
 }
 
 // Sums the far-lag partials of each (source, step of the block) over the
-// receiver splits, in split order, into split 0's slot.
+// receiver splits, in split order, into split 0's slot.  Eight splits' loads in
+// flight and small blocks: a chain of dependent adds over strided reads, 18.7 us for
+// 256 sources of 64 splits (20.4 for 74, one load at a time in 256-thread blocks).
 __global__ void adf_gf_far_combine_kernel(const EpiParams p) {
   const SolveDev& S = p.solves[blockIdx.y];
   const int it0 = S.it_base + p.step;
@@ -1218,6 +1283,7 @@ __global__ void adf_gf_far_combine_kernel(const EpiParams p) {
   if (i >= S.gf_nout * kGfBlock) return;
   const int o = i / kGfBlock, b = i - o * kGfBlock;
   double sa = 0.0, sb = 0.0;
+#pragma unroll 8
   for (int k = 0; k < S.gf_rs; ++k) {
     const double* pp = S.gf_far + (((long long)o * S.gf_rs + k) * kGfBlock + b) * 2;
     sa = __dadd_rn(sa, pp[0]);
@@ -1327,11 +1393,14 @@ cudaError_t launch_gf_near_pack(const SolveDev& d, float* near, cudaStream_t s) 
 
 cudaError_t launch_gf_far(const EpiParams& p, int max_blocks, int max_nsrc, cudaStream_t s) {
   if (max_blocks > 0) {  // 0: every blocked solve of the batch is on the tensor cores
-    adf_gf_far_kernel<<<dim3(max_blocks, p.n_solves), 256, 0, s>>>(p);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = cudaFuncSetAttribute((const void*)adf_gf_far_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGfFarSmem);
+    if (e != cudaSuccess) return e;
+    adf_gf_far_kernel<<<dim3(max_blocks, p.n_solves), 2 * kGfGroup, kGfFarSmem, s>>>(p);
+    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  adf_gf_far_combine_kernel<<<dim3((max_nsrc * kGfBlock + 255) / 256, p.n_solves), 256, 0, s>>>(p);
+  adf_gf_far_combine_kernel<<<dim3((max_nsrc * kGfBlock + 63) / 64, p.n_solves), 64, 0, s>>>(p);
   return cudaGetLastError();
 }
 

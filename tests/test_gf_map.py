@@ -154,6 +154,44 @@ def test_gf_map_tensor_core_contraction(adf, oracle, ctx, kind, nt_gf):
         assert np.linalg.norm(a - b) <= tol * max(np.linalg.norm(b), 1e-30)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["PVFromPin", "PFromPin"])
+@pytest.mark.parametrize("nt_gf,n_src,n_rec", [
+    (33, 1, 1),     # one source, one receiver: half of a block has none; one lag chunk
+    (34, 64, 2),    # a full source tile; the second lag chunk holds one lag
+    (32, 33, 5),    # a map no longer than a block
+    (97, 65, 37),   # a second tile of one source, halves of unequal receivers
+    (66, 130, 150),  # three tiles, more receivers than splits
+])
+def test_gf_map_far_lags_at_tile_edges(adf, oracle, ctx, kind, nt_gf, n_src, n_rec):
+    """The Float64 far-lag kernel at the edges of its tiles (64 sources, 32 lags,
+    receivers split over half blocks).  Its sums are Float64 with an order of their
+    own, so the Float32 samples agree to 1e-6, as for the other Float64 maps."""
+    steps = 110
+    d, o, g, cp, mask, field = make_case(adf, oracle, 40, 36, 32, steps=steps, npml=5,
+                                         shape="sphere", seed=10, n_rec=300)
+    i_rec = np.arange(3, 3 + n_rec, dtype=np.int64)
+    i_src = np.arange(160, 160 + n_src, dtype=np.int64)
+    assert i_src.max() <= g.dir.shape[1]
+    shape = (nt_gf, n_src, n_rec) if kind == "PVFromPin" else (nt_gf, n_rec, n_src)
+    rng = np.random.default_rng(12)
+    scale = 4e-2 / np.sqrt(nt_gf * n_src * n_rec)
+    ts = [(rng.standard_normal(shape) * scale).astype(np.float32, order="F") for _ in range(2)]
+    gg = to_adf_grid(adf, g)
+    pc = _Cp(adf, cp)
+    f_gpu = field.copy(order="F")
+    adf.run_fdtd(d, f_gpu, gg, pc, mask, gf_map=adf.GfMap(kind, tuple(ts), i_src, i_rec, False))
+    f_cpu = field.copy(order="F")
+    go, co = g.copy(), cp.copy()
+    oracle.run_fdtd_gf(o, f_cpu, go, co, mask, kind, ts, i_src, i_rec, o.z0, discard=False)
+    assert_parity((f_gpu, gg, pc), (f_cpu, go, co), 1e-6)
+    for k in i_src - 1:
+        for a, b in ((gg.src[0][:, k], go.src[0][:, k]), (gg.vn_src[:, k], go.vn_src[:, k])):
+            b = b.astype(np.float64)
+            assert np.abs(b[40:]).max() > 0  # the later blocks are driven
+            assert np.linalg.norm(a - b) <= 1e-6 * np.linalg.norm(b)
+
+
 def test_gf_map_unknown_contraction(adf):
     ts, isr, irc = gf_inputs(40, "PVFromPin")
     with pytest.raises(KeyError):
