@@ -2,8 +2,8 @@
 //
 // For one grid size, runs a short batch of synthetic impulsive GF solves
 // (CPML, a centred rigid sphere, a point source and a receiver shell: the
-// work mix of the serving stream) once per candidate (tile rows, z-chunk
-// depth), times the fused step kernel with per-launch CUDA events, and stores
+// work mix of the serving stream) once per candidate (tile rows, most planes
+// of a work item), times the fused step kernel with per-launch CUDA events, and stores
 // the fastest shape in the tune table that later solves of that size read.
 #include <cmath>
 #include <cstring>

@@ -91,7 +91,7 @@ void choose_tiles(int nx, int ny, int nz, int& nxp, int& ty, int& nzc, int& mw) 
   if (ty < 2) ty = 2;
   if (ty > step_max_ty()) ty = step_max_ty();
   if (ty > ny) ty = ny;
-  if (nzc == 0) return;  // chosen for the batch
+  if (nzc == 0) return;  // no bound of its own
   if (nzc < 2) nzc = 2;
   if (nzc > kMaxZc) nzc = kMaxZc;
   if (nzc > nz) nzc = nz;
@@ -399,46 +399,112 @@ int solve_finalize(adf_ctx* ctx, Solve& s, const float* const idx[4], const floa
   return ADF_OK;
 }
 
-// Work items {solve, y tile | x tile << 16, z0, z1}: z chunks outer, then y
-// tiles, x tiles inner, so that tiles sharing halo rows run together and the
-// halo hits L2.
+// Work items {solve, y tile | x tile << 16, z0, z1}.  The items of one z chunk stand
+// together, y tiles outer, x tiles inner, so that tiles sharing halo rows run together
+// and the halo hits L2.
 long long Solve::columns() const {
   const int xt = step_x_tile();
   return (long long)((dev.nxp + xt - 1) / xt) * dev.nty;
 }
-void Solve::add_items(int depth, std::vector<int4>& out) const {
-  const int xt = step_x_tile(), nxt = (dev.nxp + xt - 1) / xt;
-  if (nzc > 0) depth = nzc;
-  // as many chunks as that depth gives, of equal depth
-  const int chunks = (dev.nz + depth - 1) / depth;
-  depth = (dev.nz + chunks - 1) / chunks;
-  for (int z0 = 0; z0 < dev.nz; z0 += depth)
-    for (int t = 0; t < dev.nty; ++t)
-      for (int x = 0; x < nxt; ++x)
-        out.push_back(make_int4(0, t | (x << 16), z0, std::min(z0 + depth, dev.nz)));
+void Solve::add_chunk(int solve, int z0, int z1, std::vector<int4>& out) const {
+  const int nxt = (int)(columns() / dev.nty);
+  for (int t = 0; t < dev.nty; ++t)
+    for (int x = 0; x < nxt; ++x) out.push_back(make_int4(solve, t | (x << 16), z0, z1));
 }
 
-// Planes per work item of the batch's solves that have no tuned depth.  A CTA
-// walks its planes one after the other and recomputes one plane before them:
-// deep items waste least, shallow ones spread a small batch over the GPU.  When
-// a batch fits the GPU's resident CTAs at a depth of at most 12, the shallowest
-// such depth is taken (96^3: 73 us a step at 16 planes, 31 at 4; 40^3: 81 and
-// 22 at 3); otherwise the deepest of 24, 12 and 8 that leaves two CTAs for each
-// resident one, so that the last ones even out (2 x 256^3: 467 us at 32 planes,
-// 432 at 24, 445 at 16; 224^3: 212, 184 and 197 us at 24, 12 and 8).
-int batch_depth(const std::vector<Solve*>& list, long long resident) {
-  auto items = [&](int depth) {
-    long long n = 0;
-    for (const Solve* s : list)
-      n += s->columns() * ((s->dev.nz + (s->nzc > 0 ? s->nzc : depth) - 1) /
-                           (s->nzc > 0 ? s->nzc : depth));
-    return n;
+// The z chunks of a batch's solves, as work items in launch order.  A CTA walks its
+// item's planes one after the other and recomputes one plane before them, so deep items
+// waste least and shallow ones spread the work; `resident` CTAs run at once.
+//
+// When every solve fits the resident CTAs at one depth of at most 7, the shallowest
+// such depth is taken: one wave of equal chunks (96^3: 73 us a step at 16 planes, 31 at
+// 4).  The items of several solves alternate, so that each SM gets its share of the
+// chunks inside the z slabs (4 x 64^3: 39 us, 42 one solve after the other).  Above 7
+// planes two and more waves are as fast or faster (2 x 96^3, depth 7: 48.5 and 47.4 us;
+// 8 x 64^3, depth 8: 79 and 65; 128^3, depth 7: 43 and 46).
+//
+// Otherwise the CTAs take items as they finish, and what matters is that they end
+// together: a chunk holds at most the planes that are left per resident CTA, so that the
+// chunks become shallower towards the end, down to 3 planes, and the outer chunks, whose
+// planes lie in the z slabs and take longer (counted as 1.5), come first.  No chunk is
+// more than 0.6 of what a resident CTA gets in all: the first ones would outlast all
+// others (224^3: 166 us without that bound, 142 with it).  Step kernel, against equal
+// chunks of 24, 12 or 8 planes from the bottom up: 256^3 203 -> 177 us, 2 x 256^3
+// 351 -> 328, 8 x 256^3 1263 -> 1231, 512^3 1038 -> 1018, 192^3 120 -> 101, 224^3
+// 159 -> 142, 160^3 92 -> 79, 8 x 96^3 162 -> 145, 30 x 40^3 126 -> 100.  Over 20 batches
+// the time was on average 1.01 times the best of 30 settings of these numbers, 1.16
+// times before.
+void cut_items(const std::vector<Solve*>& list, long long resident, std::vector<int4>& out) {
+  const int ns = (int)list.size();
+  auto cap = [](const Solve* s) { return s->nzc > 0 ? std::min(s->nzc, kMaxZc) : kMaxZc; };
+  auto chunks = [&](const Solve* s, int depth) {
+    return (s->dev.nz + std::min(depth, cap(s)) - 1) / std::min(depth, cap(s));
   };
-  for (int depth = 2; depth <= 12; ++depth)
-    if (items(depth) <= resident) return depth;
-  for (int depth : {24, 12})
-    if (items(depth) >= 2 * resident) return depth;
-  return 8;
+  for (int depth = 2; depth <= 7; ++depth) {
+    long long n = 0;
+    for (const Solve* s : list) n += s->columns() * chunks(s, depth);
+    if (n > resident) continue;
+    std::vector<std::vector<int4>> own(ns);
+    for (int i = 0; i < ns; ++i) {
+      // as many chunks as that depth gives, of equal depth
+      const int nz = list[i]->dev.nz, k = chunks(list[i], depth), d = (nz + k - 1) / k;
+      for (int z = 0; z < nz; z += d) list[i]->add_chunk(i, z, std::min(z + d, nz), own[i]);
+    }
+    // a few consecutive items per solve keep neighbouring tiles together
+    size_t longest = 0;
+    for (const auto& o : own) longest = std::max(longest, o.size());
+    for (size_t pos = 0; pos < longest; pos += 8)
+      for (const auto& o : own)
+        for (size_t k = pos; k < pos + 8 && k < o.size(); ++k) out.push_back(o[k]);
+    return;
+  }
+  auto cost = [](const Solve* s, int z) {
+    const int n = s->dev.npml;
+    return n > 0 && (z <= n || z >= s->dev.nz - n - 1) ? 1.5 : 1.0;
+  };
+  struct Rest {
+    int lo, hi;          // planes not yet in an item
+    double all, left;    // their cost: at the start, now
+    bool top;            // the next chunk comes from the upper end
+  };
+  std::vector<Rest> rest(ns);
+  double left = 0;
+  for (int i = 0; i < ns; ++i) {
+    const Solve* s = list[i];
+    rest[i] = Rest{0, s->dev.nz, 0.0, 0.0, false};
+    for (int z = 0; z < s->dev.nz; ++z) rest[i].all += cost(s, z);
+    rest[i].left = rest[i].all;
+    left += rest[i].all * (double)s->columns();
+  }
+  const double most = 0.6 * left / (double)resident;
+  for (;;) {
+    int i = -1;  // the solve with the largest part of it left: all end together
+    for (int k = 0; k < ns; ++k)
+      if (rest[k].lo < rest[k].hi &&
+          (i < 0 || rest[k].left / rest[k].all > rest[i].left / rest[i].all))
+        i = k;
+    if (i < 0) break;
+    const Solve* s = list[i];
+    Rest& r = rest[i];
+    const int planes = r.hi - r.lo;
+    const double bound = std::min(most, left / (double)resident);
+    double c = 0;
+    int d = 0;
+    while (d < planes && d < cap(s)) {
+      c += cost(s, r.top ? r.hi - 1 - d : r.lo + d);
+      if (d >= 3 && c > bound) break;
+      ++d;
+    }
+    if (planes > d && planes < 2 * d) d = (planes + 1) / 2;
+    const int z0 = r.top ? r.hi - d : r.lo;
+    (r.top ? r.hi : r.lo) += r.top ? -d : d;
+    r.top = !r.top;
+    for (int z = z0; z < z0 + d; ++z) {
+      r.left -= cost(s, z);
+      left -= cost(s, z) * (double)s->columns();
+    }
+    s->add_chunk(i, z0, z0 + d, out);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -485,26 +551,7 @@ int Batch::setup(adf_ctx* ctx, const std::vector<Solve*>& list) {
     max_ty = std::max(max_ty, d.ty);
     max_ntx = std::max(max_ntx, d.ntx);
   }
-  // interleave items of different solves so the batch stays balanced
-  {
-    const int depth = batch_depth(list, ctx->step_ctas);
-    std::vector<std::vector<int4>> own(ns);
-    for (int i = 0; i < ns; ++i) list[i]->add_items(depth, own[i]);
-    std::vector<size_t> pos(ns, 0);
-    bool any = true;
-    while (any) {
-      any = false;
-      for (int i = 0; i < ns; ++i) {
-        // a few consecutive items per solve keep neighbouring tiles together
-        for (int k = 0; k < 8 && pos[i] < own[i].size(); ++k) {
-          int4 it = own[i][pos[i]++];
-          it.x = i;
-          items.push_back(it);
-          any = true;
-        }
-      }
-    }
-  }
+  cut_items(list, ctx->step_ctas, items);
   n_items = (int)items.size();
   if (ns > cap_solves || n_items > cap_items) {
     release();

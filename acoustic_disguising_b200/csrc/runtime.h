@@ -74,7 +74,7 @@ struct Solve {
   unsigned char fmap_host[4 * 128];  // the tensor maps of dev.fmap (copied to the device)
   std::vector<void*> allocs;
   size_t bytes = 0;
-  int nzc = 0;             // planes per work item, 0: chosen for the batch
+  int nzc = 0;             // planes per work item, at most; 0: kMaxZc
   uint32_t* mask_bits = nullptr;
   float* coef_dev = nullptr;
   float* dir_dev = nullptr;
@@ -85,7 +85,8 @@ struct Solve {
   cudaStream_t alloc_stream = nullptr;  // stream-ordered allocation from alloc_pool when set
   cudaMemPool_t alloc_pool = nullptr;
   long long columns() const;                                // x tiles x y tiles
-  void add_items(int depth, std::vector<int4>& out) const;  // {0, y tile | x tile << 16, z0, z1}
+  // its work items of the planes [z0, z1): {solve, y tile | x tile << 16, z0, z1}
+  void add_chunk(int solve, int z0, int z1, std::vector<int4>& out) const;
   ~Solve();
   void release();
 };
@@ -123,7 +124,8 @@ struct Batch {
 };
 
 void choose_tiles(int nx, int ny, int nz, int& nxp, int& ty, int& nzc, int& mw);
-int batch_depth(const std::vector<Solve*>& list, long long resident);
+// the batch's work items in launch order, for `resident` CTAs at once
+void cut_items(const std::vector<Solve*>& list, long long resident, std::vector<int4>& out);
 size_t solve_bytes_estimate(int64_t nx, int64_t ny, int64_t nz, int64_t npml, int64_t ntx,
                             int64_t nt, bool mask);
 int solve_alloc(adf_ctx* ctx, Solve& s, const hm::Dom& dom, int npml, bool has_mask, int arith,

@@ -1,7 +1,7 @@
 // tune.cpp -- tile-shape table for the step kernel.
 //
 // The fused step kernel's tile has `ty` rows (plus one recomputed halo row)
-// and streams `nzc` planes per work item.  adf_autotune (autotune.cu) times
+// and streams at most `nzc` planes per work item.  adf_autotune (autotune.cu) times
 // candidate shapes per grid size and stores the fastest in tune_table.json
 // next to the library; lookups fall back to a size-based default.
 #include <cstdio>
@@ -56,7 +56,7 @@ static Tune default_tune(int nx, int ny, int nz) {
   // plus the recomputed halo row) and recompute the fewest halo rows.
   t.ty = 7;
   (void)nx;
-  t.nzc = 0;  // the batch's choice (batch_depth)
+  t.nzc = 0;  // the batch's choice (cut_items)
   (void)ny;
   return t;
 }

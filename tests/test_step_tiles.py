@@ -61,3 +61,33 @@ def test_depth_of_a_batch_changes_nothing(adf, ctx):
     for a, b in zip(batch, alone):
         assert np.abs(a.p).max() > 0
         assert np.array_equal(a.p, b.p) and np.array_equal(a.vn, b.vn)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile", [None, "7,1", "7,2", "5,9", "7,32"])
+def test_chunks_of_a_mixed_batch_change_nothing(adf, ctx, tile, monkeypatch):
+    """Solves of unequal sizes and layer widths (none, and layers that leave few
+    planes between them) in one batch: the chunks shrink towards the end, come from
+    both ends in turn and keep to a tile's depth where one is given.  Every plane is
+    stepped once: the traces are bit for bit those of each solve alone, and those of
+    solves cut into equal chunks."""
+    from test_fdtd_parity import C0, DT, DX, RHO
+
+    def request(n, npml, k):
+        d = adf.Domain(tmax=19.5 * DT, xmax=(n - 1) * DX / 2, nx=n, c0=C0, r0=RHO, cf=0.5)
+        tf, _ = adf.impulsive_wavelet(d, 9000.0)
+        rp, rn = adf.fibonacci_sphere(30, 0.4 * d.xmax)
+        return adf.GfRequest(d, [0.35 * d.xmax, 0.01 * k * d.xmax, 0.0], [1.0, 0, 0, 0], tf, rp,
+                             rn, npml=npml, pml_fc=2000.0, scatterer="sphere",
+                             scatterer_kw=dict(radius=0.25 * d.xmax))
+    sizes = [(96, 10), (30, 13), (101, 0), (64, 5), (33, 1), (110, 12), (96, 10), (47, 8), (83, 20)]
+    if tile:
+        monkeypatch.setenv("ADF_TILE", tile)
+    batch = [request(n, npml, k) for k, (n, npml) in enumerate(sizes)]
+    adf.gf_solve_batch(batch, batched=True)
+    monkeypatch.setenv("ADF_TILE", "7,4")
+    alone = [request(n, npml, k) for k, (n, npml) in enumerate(sizes)]
+    adf.gf_solve_batch(alone, batched=False)
+    for a, b in zip(batch, alone):
+        assert np.abs(a.p).max() > 0
+        assert np.array_equal(a.p, b.p) and np.array_equal(a.vn, b.vn)
