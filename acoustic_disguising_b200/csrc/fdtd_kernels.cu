@@ -482,6 +482,16 @@ constexpr int kStageFloats = (kStageVz + kStageChan + 31) / 32 * 32;
 constexpr uint32_t kStepWaitLimit = 1u << 20;
 static_assert((kStageFloats * 4) % 128 == 0, "stages stay 128-B aligned");
 
+// One thread: the copies of plane k's stage into a free slot.
+__device__ __forceinline__ void stage_plane(const char* maps, float* slot, uint64_t* bar, int xb,
+                                            int j0, int k, int nz) {
+  const uint32_t b = smem_u32(bar);
+  const bool vz = k + 1 < nz;
+  mbar_expect_tx(b, (uint32_t)((vz ? 16 : 12) * kStageChan));
+  tma_load_4d(smem_u32(slot), maps, xb - 4, j0 - 1, k, 0, b);
+  if (vz) tma_load_4d(smem_u32(slot + kStageVz), maps + 128, xb - 4, j0 - 1, k + 1, 3, b);
+}
+
 template <typename R>
 __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, int4 item, int it,
                                           float* sPn, float* sV, float* ring,
@@ -571,6 +581,7 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
   // k = nz-1, whose update does not read it), rows j0-1 .. j0+kMaxTy,
   // x = xb-4 .. xb+67, zero outside the grid.  Vz of plane k is carried in
   // registers from the previous stage.
+  // (The kernel has issued the item's first planes.)
   constexpr int cst = kStageChan, vzo = kStageVz;
   const int so = r * kStageW + 4 + 4 * qx;    // this quad in a stage channel
   const char* maps = static_cast<const char*>(S.fmap) + rb * 256;  // {P,Vx,Vy box; Vz box}
@@ -578,20 +589,13 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
   auto issue = [&](int k) {  // one thread
     const int sl = slot_of(k);
     fence_proxy_async_smem();  // the slot was last read through the generic proxy
-    const uint32_t bar = smem_u32(rbar + sl);
-    const bool vz = k + 1 < nz;
-    mbar_expect_tx(bar, (uint32_t)((vz ? 16 : 12) * cst));
-    float* dst = ring + sl * kStageFloats;
-    tma_load_4d(smem_u32(dst), maps, xb - 4, j0 - 1, k, 0, bar);
-    if (vz) tma_load_4d(smem_u32(dst + vzo), maps + 128, xb - 4, j0 - 1, k + 1, 3, bar);
+    stage_plane(maps, ring + sl * kStageFloats, rbar + sl, xb, j0, k, nz);
   };
   auto wait = [&](int k) {
     const int u = k - kfirst;
     if (!mbar_wait(smem_u32(rbar + u % kStepRing), (uint32_t)(u / kStepRing) & 1u, kStepWaitLimit))
       atomicOr(S.err, 4);  // reported as ADF_E_TIMEOUT; the values read are wrong
   };
-  if (tid == 0)
-    for (int k = kfirst; k < min(z1, kfirst + kStepRing); ++k) issue(k);
   // Vz of plane kfirst (the stages carry the next plane's), and of the halo
   // column for its single-cell update
   float4 Z0 = make_float4(0.f, 0.f, 0.f, 0.f), Pzm = Z0;
@@ -745,22 +749,33 @@ __device__ __forceinline__ void pml_table(const SolveDev& G, PmlTab& Q, int4 ite
   auto cv = [&](int x, int m) {
     return x < 0 || x >= m ? -1 : x <= n ? 2 * n + x : (x >= m - n - 1 ? 3 * n + 1 + x - (m - n - 1) : -1);
   };
-  auto fill = [&](float* pa, float* pb, float* va, float* vb, int i, int x, int m) {
-    const int p = cp(x, m), v = cv(x, m);
-    if (p >= 0) pa[i] = co[p], pb[i] = co[nb + p];
-    if (v >= 0) va[i] = co[v], vb[i] = co[nb + v];
-  };
-  const int xb = (item.y >> 16) * kXT, j0 = (item.y & 0xFFFF) * G.ty;
-  for (int i = 3 + tid; i < 68; i += nthr) fill(Q.xpa, Q.xpb, Q.xva, Q.xvb, i, xb + i - 4, G.nx);
-  for (int i = tid; i < 8; i += nthr) fill(Q.ypa, Q.ypb, Q.yva, Q.yvb, i, j0 - 1 + i, G.ny);
-  for (int u = tid; u < item.w - kfirst; u += nthr) {
-    const int k = kfirst + u, p = cp(k, G.nz), v = k >= 1 ? cv(k, G.nz) : -1;
-    fill(Q.zpa, Q.zpb, Q.zva, Q.zvb, u, k, G.nz);
-    const int pl = G.ny * G.nxp;
-    Q.zp[u] = p < 0 ? -1 : (p >= n ? (int)G.psi_p_side[2] : 0) + (p >= n ? p - n : p) * pl;
-    Q.zv[u] = v < 0 ? -1
-                    : (v >= 3 * n + 1 ? (int)G.psi_v_side[2] : 0) +
-                          (v >= 3 * n + 1 ? v - 3 * n - 1 : v - 2 * n) * pl;
+  // the halo column's and the tile's 65 columns, 8 rows and the item's planes, one to
+  // a thread, so that their reads go out together
+  const int xb = (item.y >> 16) * kXT, j0 = (item.y & 0xFFFF) * G.ty, np = item.w - kfirst;
+  for (int i = tid; i < 73 + np; i += nthr) {
+    int x, m, e;
+    float *pa, *pb, *va, *vb;
+    if (i < 65) {
+      x = xb - 1 + i, m = G.nx, e = 3 + i;
+      pa = Q.xpa, pb = Q.xpb, va = Q.xva, vb = Q.xvb;
+    } else if (i < 73) {
+      e = i - 65, x = j0 - 1 + e, m = G.ny;
+      pa = Q.ypa, pb = Q.ypb, va = Q.yva, vb = Q.yvb;
+    } else {
+      e = i - 73, x = kfirst + e, m = G.nz;
+      pa = Q.zpa, pb = Q.zpb, va = Q.zva, vb = Q.zvb;
+    }
+    const int c = cp(x, m), v = i >= 73 && x < 1 ? -1 : cv(x, m);
+    const int c0 = max(c, 0), v0 = max(v, 0);
+    const float ca = co[c0], cb = co[nb + c0], wa = co[v0], wb = co[nb + v0];
+    if (i >= 73) {
+      const int pl = G.ny * G.nxp;
+      Q.zp[e] = c < 0 ? -1 : (c >= n ? (int)G.psi_p_side[2] : 0) + (c >= n ? c - n : c) * pl;
+      Q.zv[e] = v < 0 ? -1
+                      : (v >= 3 * n + 1 ? (int)G.psi_v_side[2] : 0) +
+                            (v >= 3 * n + 1 ? v - 3 * n - 1 : v - 2 * n) * pl;
+    }
+    pa[e] = ca, pb[e] = cb, va[e] = wa, vb[e] = wb;
   }
 }
 
@@ -792,30 +807,39 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
     pdl_wait();  // this kernel is not over before those it depends on
     return;
   }
-  const int tid = threadIdx.y * 32 + threadIdx.x, nthr = blockDim.x * blockDim.y;
-  {
+  // The first warp's first thread starts the copies of the item's first planes as soon
+  // as it has their place; the other warps read the item's tables meanwhile.
+  const int tid = threadIdx.y * 32 + threadIdx.x, kfirst = item.z > 0 ? item.z - 1 : 0;
+  if (tid == 0) {
+    for (int q = 0; q < kStepRing; ++q) mbar_init(smem_u32(rbar + q), 1);
+    fence_mbar_init();
+    const char* maps = static_cast<const char*>(G.fmap) + ((it - G.it_first) & 1) * 256;
+    prefetch_tensormap(maps);
+    prefetch_tensormap(maps + 128);
+    const int j0 = (item.y & 0xFFFF) * G.ty, nz = G.nz;
+    pdl_wait();
+    for (int k = kfirst; k < min(item.w, kfirst + kStepRing); ++k)
+      stage_plane(maps, ring + (k - kfirst) * kStageFloats, rbar + (k - kfirst), (item.y >> 16) * kXT,
+                  j0, k, nz);
+  } else if (tid >= 32) {
+    const int t = tid - 32, nthr = kStepThreads - 32;
     const int* src = reinterpret_cast<const int*>(&G);
     int* dst = reinterpret_cast<int*>(&S);
-    for (int w = tid; w < (int)(sizeof(SolveDev) / 4); w += nthr) dst[w] = src[w];
-    const int kfirst = item.z > 0 ? item.z - 1 : 0;
-    if (tid < item.w - kfirst) {
-      const int* tp = G.tp_off + ((long long)(item.y & 0xFFFF) * G.nz + kfirst + tid) * 4;
+    for (int w = t; w < (int)(sizeof(SolveDev) / 4); w += nthr) dst[w] = src[w];
+    if (t < item.w - kfirst) {
+      const int* tp = G.tp_off + ((long long)(item.y & 0xFFFF) * G.nz + kfirst + t) * 4;
       int f = (tp[0] < tp[1] ? 1 : 0) | (tp[1] < tp[4] ? 2 : 0);
-      if (G.closed && G.closed[((long long)(item.y >> 16) * G.nty + (item.y & 0xFFFF)) * G.nz +
-                               kfirst + tid])
+      if (G.closed &&
+          G.closed[((long long)(item.y >> 16) * G.nty + (item.y & 0xFFFF)) * G.nz + kfirst + t])
         f |= 4;
       // planes without z-slab memory, mirror or rigid wall
-      const int zm = (G.flags & (SF_PCPML | SF_VCPML)) ? G.npml + 1 : 1, k = kfirst + tid;
+      const int zm = (G.flags & (SF_PCPML | SF_VCPML)) ? G.npml + 1 : 1, k = kfirst + t;
       if (k >= max(zm, 2) && k < G.nz - zm) f |= 8;
-      s_fl[tid] = (unsigned char)f;
+      s_fl[t] = (unsigned char)f;
     }
-    pml_table(G, Q, item, it, kfirst, tid, nthr);
-    if (tid == 0) {
-      for (int q = 0; q < kStepRing; ++q) mbar_init(smem_u32(rbar + q), 1);
-      fence_mbar_init();
-    }
+    pml_table(G, Q, item, it, kfirst, t, nthr);
   }
-  // Up to here only the descriptors and tables of the set-up were read.  The field,
+  // Up to the wait only the descriptors and tables of the set-up are read.  The field,
   // the sources and the records belong to the kernels before.
   pdl_wait();
   pdl_trigger();  // after the wait: one step's kernels start ahead, not a chain of them
