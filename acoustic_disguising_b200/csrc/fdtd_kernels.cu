@@ -482,6 +482,53 @@ constexpr int kStageFloats = (kStageVz + kStageChan + 31) / 32 * 32;
 constexpr uint32_t kStepWaitLimit = 1u << 20;
 static_assert((kStageFloats * 4) % 128 == 0, "stages stay 128-B aligned");
 
+// Fetches plane k's slab memory of the item into L2, a warp to a plane: lane = tile row +
+// 8 x array (p y, v y, p z, v z; the v arrays have no halo row, whose lanes take the x
+// slabs' rows, one contiguous piece each).  A boundary warp waits for reads of slab
+// memory that nothing has touched since the last step, and its length sets its CTA's
+// pace.  On grids whose memory stays in L2 there is nothing to gain (128^3: 39 us
+// without this, 41 with it; 192^3: 89.4 and 86.7), so it is for grids from 2^22 cells on:
+// 8 x 256^3 with CPML 1.108 -> 1.044 ms, with a sphere 1.252 -> 1.209, 2 x 256^3
+// 314 -> 294 us, 512^3 1.003 -> 0.968 ms.  The x slabs are read a phase ahead anyway and
+// pay from 2^24 cells on (192^3 86.7 without them, 88.5 with; 256^3 157.0, 157.5;
+// 8 x 256^3 with CPML 1.061, 1.044).  A prefetch a quad in place of a row took 28.6 us at
+// 96^3 (26.7) and 0.768 ms at 8 x 256^3 without CPML (0.750).  Out of line, as
+// apply_entries is.
+constexpr long long kFetchCells = 1 << 22, kFetchXCells = 1 << 24;
+__device__ __noinline__ void fetch_slabs(const SolveDev& S, const PmlTab& Q, int4 item, int kfirst,
+                                         int k) {
+  const int lane = threadIdx.x, row = lane & 7, arr = lane >> 3, n = S.npml;
+  const int j = (item.y & 0xFFFF) * S.ty - 1 + row, X = item.y >> 16, xb = X * kXT;
+  if (k >= item.w || j >= S.ny || row > S.ty) return;
+  const bool v = arr & 1;
+  constexpr int line = 32;  // floats
+  if (v && row == 0) {
+    const bool lo = X == 0, hi = (X + 1) * kXT >= S.nxp, xv = arr == 3;
+    if ((!lo && !hi) || S.chan_stride < kFetchXCells) return;
+    const int pitch = xv ? S.nvp : S.npp, j0 = max(j, 0), j1 = min(j + S.ty + 1, S.ny);
+    const int side = lo ? 0 : (int)(xv ? S.psi_v_side[0] : S.psi_p_side[0]);
+    const float* p = Q.rd[xv ? 3 : 0] + (side + (k * S.ny + j0) * pitch);
+    for (int i = 0; i < (j1 - j0) * pitch; i += line) prefetch_l2(p + i);
+    return;
+  }
+  if (j < 0) return;
+  int o;
+  if (arr < 2) {
+    const int m = n + (v ? 1 : 0);  // layers
+    if (j >= m && j < S.ny - m) return;
+    o = (j < m ? 0 : (int)(v ? S.psi_v_side[1] : S.psi_p_side[1])) +
+        (k * m + (j < m ? j : j - (S.ny - m))) * S.nxp;
+  } else {
+    o = v ? Q.zv[k - kfirst] : Q.zp[k - kfirst];
+    if (o < 0) return;
+    o += j * S.nxp;
+  }
+  const float* p = Q.rd[(arr < 2 ? 1 : 2) + (v ? 3 : 0)] + (o + xb);
+#pragma unroll
+  for (int i = 0; i < kXT; i += line)
+    if (i < S.nxp - xb) prefetch_l2(p + i);
+}
+
 // One thread: the copies of plane k's stage into a free slot.
 __device__ __forceinline__ void stage_plane(const char* maps, float* slot, uint64_t* bar, int xb,
                                             int j0, int k, int nz) {
@@ -721,6 +768,7 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
         }
       }
     }
+    if (fl & 16) fetch_slabs(S, Q, item, kfirst, k + 1 + wid);
     Pzm = Pn;
     Z0 = Z1;
   }
@@ -798,7 +846,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
   __shared__ __align__(16) float sPn[(2 * (kMaxTy + 1) + 1) * kPnPitch];  // (a row before the first)
   __shared__ __align__(16) float sV[3 * kMaxTy * kXT];
   __shared__ __align__(16) PmlTab Q;
-  __shared__ unsigned char s_fl[kMaxZc + 1];  // planes kfirst ..: 1 q, 2 f entries, 4 closed cells, 8 plain
+  __shared__ unsigned char s_fl[kMaxZc + 1];  // planes kfirst ..: 1 q, 2 f entries, 4 closed cells, 8 plain, 16 fetch_slabs
   __shared__ __align__(16) SolveDev S;  // the solve descriptor, read in the hot loop
   const int4 item = p.items[blockIdx.x];
   const SolveDev& G = p.solves[item.x];
@@ -835,6 +883,13 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
       // planes without z-slab memory, mirror or rigid wall
       const int zm = (G.flags & (SF_PCPML | SF_VCPML)) ? G.npml + 1 : 1, k = kfirst + t;
       if (k >= max(zm, 2) && k < G.nz - zm) f |= 8;
+      // every fourth plane: do the next four have slab memory to fetch?
+      if ((t & 3) == 0 && G.npml > 0 && G.chan_stride >= kFetchCells) {
+        const int X = item.y >> 16, j0 = (item.y & 0xFFFF) * G.ty;
+        if (j0 - 1 < zm || j0 + G.ty > G.ny - zm || k + 1 < zm || k + 4 >= G.nz - zm ||
+            (G.chan_stride >= kFetchXCells && (X == 0 || (X + 1) * kXT >= G.nxp)))
+          f |= 16;
+      }
       s_fl[t] = (unsigned char)f;
     }
     pml_table(G, Q, item, it, kfirst, t, nthr);

@@ -62,6 +62,9 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, int x
       "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(c), "r"(mbar)
       : "memory");
 }
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
 __device__ __forceinline__ void prefetch_tensormap(const void* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }

@@ -91,3 +91,17 @@ def test_chunks_of_a_mixed_batch_change_nothing(adf, ctx, tile, monkeypatch):
     for a, b in zip(batch, alone):
         assert np.abs(a.p).max() > 0
         assert np.array_equal(a.p, b.p) and np.array_equal(a.vn, b.vn)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,nz,npml", [
+    (163, 162, 161, 7),   # just above the size from which slab memory is fetched ahead
+    (257, 260, 255, 9),   # ... and the x slabs' too, the right one in the last two x tiles
+    (270, 141, 442, 1),   # one layer: velocity memory of two
+])
+def test_fetched_slab_memory(adf, oracle, ctx, nx, ny, nz, npml):
+    """Grids whose slab memory is fetched into L2 ahead, of odd sizes: the fetches
+    change nothing and stay inside the memory."""
+    case = make_case(adf, oracle, nx, ny, nz, steps=8, npml=npml, shape="none", seed=nx, n_rec=6)
+    gpu, cpu = run_both(adf, oracle, case)
+    assert_parity(gpu, cpu, 1e-6)
