@@ -30,9 +30,11 @@ enum : int {
   SF_GF_TC = 64,    // its far lags on the tensor cores (TF32 split, gf_tc)
 };
 
-// Steps per block of the in-loop GF extrapolation: lags older than the block
-// are summed once per block, the rest step by step.
+// Steps per block of the in-loop GF extrapolation: lags older than the block are
+// summed once per block, those older than a sub-block once per sub-block, the rest
+// step by step.
 constexpr int kGfBlock = 32;
+constexpr int kGfSub = 8;
 constexpr int kGfRing = 64;  // input-history rows kept receiver-major (>= kGfBlock + 1)
 
 // GF map kinds, as ADF_GF_* in include/adfdtd.h
@@ -57,8 +59,8 @@ struct SolveDev {
   float fqf, fvf, rdxf, rdyf, rdzf;
   float* field;
   // four CUtensorMaps (128 B each) over the field: per buffer 0, 1 one with
-  // box (kStageW, ty + 2, 1, 3) (P, Vx, Vy of a plane) and one with box
-  // (kStageW, ty + 2, 1, 1) (Vz); 4D (x: nxp, y: ny, z: nz, channel: 4),
+  // box (kStageW, max ty + 2, 1, 3) (P, Vx, Vy of a plane) and one with box
+  // (kStageW, max ty + 2, 1, 1) (Vz); 4D (x: nxp, y: ny, z: nz, channel: 4),
   // zero fill outside the grid
   const void* fmap;
   long long buf_stride;   // floats per field buffer (4*nz*ny*nxp)
@@ -145,6 +147,8 @@ cudaError_t launch_gf_extrapolate(const EpiParams& p, int max_blocks, int max_ns
 // that starts at launch-step p.step
 cudaError_t launch_gf_near_pack(const SolveDev& d, float* near, cudaStream_t s);
 cudaError_t launch_gf_far(const EpiParams& p, int max_blocks, int max_nsrc, cudaStream_t s);
+// the block's rows for the sub-block of kGfSub steps that starts at launch-step p.step
+cudaError_t launch_gf_mid(const EpiParams& p, int max_nsrc, bool overlap, cudaStream_t s);
 // the same on the tensor cores for SF_GF_TC solves (gf_tc_kernel.cu): blocks =
 // 128-source tiles x gf_rs; launch_gf_far's combine step then adds the splits
 cudaError_t launch_gf_far_tc(const EpiParams& p, int max_blocks, cudaStream_t s);

@@ -18,8 +18,8 @@
 // exchange of the new P, Float64 arithmetic) runs in each; what bounds them is
 // that chain and the instructions around it, not HBM.  With the stage read
 // through shared-space addresses, on different banks, and the entries' code out
-// of the plane loop, a launch of 8 x 256^3 takes 0.77 ms without boundaries
-// (0.89 before) and 1.30 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
+// of the plane loop, a launch of 8 x 256^3 takes 0.75 ms without boundaries
+// (0.89 before) and 1.21 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
 // The plane loop's code has to stay small: a masked form of the plain update and
 // one with the x slab's memory each made it slower (1.57 and 1.66 ms).
 //
@@ -93,7 +93,7 @@ __device__ __forceinline__ void stcs4(float* p, float4 v) { __stcs(reinterpret_c
 __device__ __forceinline__ float4 neg4(float4 v) { return make_float4(-v.x, -v.y, -v.z, -v.w); }
 
 template <typename R>
-struct Sc {  // per-solve update scalars in registers
+struct Sc {  // per-solve update scalars
   R fq, fv, rdx, rdy, rdz;
 };
 
@@ -829,7 +829,7 @@ __device__ __forceinline__ void pml_table(const SolveDev& G, PmlTab& Q, int4 ite
 
 // Shared memory: the staged-plane ring (dynamic, kStepRing * kStageFloats
 // floats) plus the new-P planes, the f-channel staging and the descriptor:
-// 33.4 KB per CTA; five CTAs per SM (the register budget: 102 per thread,
+// 34.3 KB per CTA; five CTAs per SM (the register budget: 102 per thread,
 // no spills; six CTAs at 80 registers spill and measured slower).
 #ifndef ADF_STEP_CTAS_PER_SM
 #define ADF_STEP_CTAS_PER_SM 5
@@ -1056,9 +1056,10 @@ __global__ void __launch_bounds__(256, 4) adf_gf_extrapolate_kernel(const EpiPar
   if (o >= S.gf_nout) return;
   const int nt = S.nt, ntx = S.ntx, ngf = S.gf_nt, n1 = S.gf_n1, nin = S.gf_nin;
   const int kind = S.gf_kind;
-  // lags 0..T-1 (T = min(it, ngf)); with blocking only 0..b, b = this step's
-  // place in its block, the older lags coming from adf_gf_far_kernel
-  const int T = S.gf_rs > 0 ? min(min(it, ngf), p.step % kGfBlock + 1) : min(it, ngf);
+  // lags 0..T-1 (T = min(it, ngf)); with blocking only 0..b, b = this step's place
+  // in its sub-block, the older lags coming from adf_gf_mid_kernel and
+  // adf_gf_far_kernel
+  const int T = S.gf_rs > 0 ? min(min(it, ngf), p.step % kGfSub + 1) : min(it, ngf);
   const int t0 = it - T;  // 0-based row of tt = 1
   const long long cur = (long long)(it - 1) * ntx;
   auto pin_now = [&](int r) {
@@ -1195,6 +1196,80 @@ __global__ void __launch_bounds__(256, 4) adf_gf_extrapolate_kernel(const EpiPar
   }
 }
 
+// The same split inside a block: at the first step it0 of a sub-block of kGfSub steps
+// (not the block's first), the sb rows that the block has filed so far, for the
+// sub-block's steps it0 .. it0+kGfSub-1.  Step it0+q reads row it0-1-i with lag q+i,
+// i = 1 .. sb; lags 0..q stay in adf_gf_extrapolate_kernel.  The sums go on top of the
+// far lags' (gf_finish adds them).  One block per source, threads over receivers; each
+// walks the rows from the newest back, the 8 steps' tensor values one window that moves
+// by a lag per row, so a lag is read once for 8 steps and not at each: the near-lag
+// copy, up to 58 MB of a 512 x 448 map, is what a step's sum is bound by (L2).
+// With all 32 lags in the step's sum it took 11.4 us on a 256 x 256 map and 17.3 on a
+// 512 x 448 one, cold, now 9.3 and 12.2, plus 17 and 32 every 8 steps here.
+constexpr int kGfMidThreads = 128;
+__global__ void __launch_bounds__(kGfMidThreads) adf_gf_mid_kernel(const EpiParams p) {
+  pdl_trigger();
+  pdl_wait();
+  const SolveDev& S = p.solves[blockIdx.y];
+  const int it0 = S.it_base + p.step, o = blockIdx.x;
+  if (S.gf_rs <= 0 || it0 > S.it_stop || it0 >= S.nt || !(S.flags & SF_GF) || o >= S.gf_nout) return;
+  const int sb = p.step % kGfBlock, nl = S.gf_nl, nin = S.gf_nin;
+  const float* const g0 = S.gf_near + (long long)o * nl * nin;
+  const float* const g1 = g0 + (long long)S.gf_nout * nl * nin;
+  double acc[2][kGfSub];
+#pragma unroll
+  for (int q = 0; q < kGfSub; ++q) acc[0][q] = acc[1][q] = 0.0;
+  for (int r = threadIdx.x; r < nin; r += kGfMidThreads) {
+    float w0[kGfSub], w1[kGfSub];  // lags i .. i+7 at row i; past the map unused
+#pragma unroll
+    for (int q = 0; q < kGfSub - 1; ++q) {
+      const bool in = q + 1 < nl;
+      w0[q + 1] = in ? g0[(long long)(q + 1) * nin + r] : 0.f;
+      w1[q + 1] = in ? g1[(long long)(q + 1) * nin + r] : 0.f;
+    }
+    auto rows = [&](auto checked) {
+#pragma unroll 4
+      for (int i = 1; i <= sb; ++i) {
+        const double h = S.gf_ring[(long long)((it0 - 1 - i) % kGfRing) * nin + r];
+#pragma unroll
+        for (int q = 0; q < kGfSub - 1; ++q) w0[q] = w0[q + 1], w1[q] = w1[q + 1];
+        const int lag = i + kGfSub - 1;
+        if (!decltype(checked)::value || lag < nl) {
+          w0[kGfSub - 1] = g0[(long long)lag * nin + r];
+          w1[kGfSub - 1] = g1[(long long)lag * nin + r];
+        }
+#pragma unroll
+        for (int q = 0; q < kGfSub; ++q)
+          if (!decltype(checked)::value || i + q < nl) {
+            acc[0][q] = __fma_rn((double)w0[q], h, acc[0][q]);
+            acc[1][q] = __fma_rn((double)w1[q], h, acc[1][q]);
+          }
+      }
+    };
+    if (sb + kGfSub <= nl)
+      rows(std::false_type());
+    else
+      rows(std::true_type());
+  }
+  __shared__ double red[2][kGfSub][kGfMidThreads / 32];
+#pragma unroll
+  for (int t = 0; t < 2; ++t)
+#pragma unroll
+    for (int q = 0; q < kGfSub; ++q) {
+      double a = acc[t][q];
+#pragma unroll
+      for (int w = 16; w > 0; w >>= 1) a = __dadd_rn(a, __shfl_down_sync(0xffffffffu, a, w));
+      if ((threadIdx.x & 31) == 0) red[t][q][threadIdx.x >> 5] = a;
+    }
+  __syncthreads();
+  if (threadIdx.x >= 2 * kGfSub) return;
+  const int t = threadIdx.x & 1, q = threadIdx.x >> 1;
+  double a = 0.0;
+  for (int w = 0; w < kGfMidThreads / 32; ++w) a = __dadd_rn(a, red[t][q][w]);
+  double* pp = S.gf_far + ((long long)o * S.gf_rs * kGfBlock + sb + q) * 2 + t;
+  *pp = __dadd_rn(*pp, a);
+}
+
 // Far-lag part of the in-loop GF extrapolation (extrapolation.jl:139-170),
 // block-causal form.  For the block of kGfBlock steps it0 .. it0+B-1 that
 // starts at this launch-step, step it0+b needs lags 0 .. T_b-1 of the map
@@ -1203,7 +1278,7 @@ __global__ void __launch_bounds__(256, 4) adf_gf_extrapolate_kernel(const EpiPar
 // summed here once for the whole block: a contraction over (receiver, lag)
 // of the block's 32 steps x 64 sources, which reads each tensor slice once
 // per block instead of once per step.  Lags 0..b, whose rows appear during
-// the block, stay in adf_gf_extrapolate_kernel.  FP64 fused multiply-adds;
+// the block, stay in the kernels above.  FP64 fused multiply-adds;
 // one partial per (source, receiver split, step), added in split order by
 // adf_gf_far_combine_kernel.  Input-history kinds only.
 //
@@ -1481,6 +1556,11 @@ cudaError_t launch_gf_far(const EpiParams& p, int max_blocks, int max_nsrc, cuda
   }
   adf_gf_far_combine_kernel<<<dim3((max_nsrc * kGfBlock + 63) / 64, p.n_solves), 64, 0, s>>>(p);
   return cudaGetLastError();
+}
+
+cudaError_t launch_gf_mid(const EpiParams& p, int max_nsrc, bool overlap, cudaStream_t s) {
+  return launch_overlapped(adf_gf_mid_kernel, dim3(max_nsrc, p.n_solves), dim3(kGfMidThreads), 0,
+                           overlap, s, p);
 }
 
 cudaError_t launch_epilogue(const EpiParams& p, int max_ntx, bool overlap, cudaStream_t s) {

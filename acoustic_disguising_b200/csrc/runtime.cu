@@ -627,6 +627,10 @@ int Batch::launch_step(adf_ctx* ctx, int step) {
     if ((max_gf_far_blocks > 0 || max_gf_tc_blocks > 0) && step % kGfBlock == 0 &&
         (e2 = launch_gf_far(ep, max_gf_far_blocks, max_gf_nsrc, ctx->stream)) != cudaSuccess)
       return fail(ADF_E_DEVICE, std::string("GF launch failed: ") + cudaGetErrorString(e2));
+    if ((max_gf_far_blocks > 0 || max_gf_tc_blocks > 0) && step % kGfBlock != 0 &&
+        step % kGfSub == 0 &&
+        (e2 = launch_gf_mid(ep, max_gf_nsrc, overlap, ctx->stream)) != cudaSuccess)
+      return fail(ADF_E_DEVICE, std::string("GF launch failed: ") + cudaGetErrorString(e2));
     if ((e2 = launch_gf_extrapolate(ep, max_gf_blocks, max_gf_nsrc, gf_reduce, overlap,
                                     ctx->stream)) !=
         cudaSuccess)

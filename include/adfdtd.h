@@ -269,7 +269,7 @@ int adf_gf_solve_batch(adf_ctx* ctx, int64_t n, adf_gf_request* reqs, int batche
 /* Autotuner of the fused step kernel's tile shape for one grid size; no
  * counterpart in the reference.  Times n_solves synthetic GF solves of
  * `steps` steps (CPML npml, centred rigid sphere, point source, receiver
- * shell) for each candidate (tile rows, z-chunk depth), keeps the fastest
+ * shell) for each candidate (tile rows, most planes of an item), keeps the fastest
  * in the tune table next to the library (or $ADF_TUNE_TABLE) that later
  * solves of this size use, and returns it with its mean step-kernel time.  */
 int adf_autotune(adf_ctx* ctx, int64_t nx, int64_t ny, int64_t nz, int64_t npml, int n_solves,
@@ -284,8 +284,8 @@ int adf_server_start(adf_ctx* ctx, size_t hbm_budget, int max_resident, adf_serv
 /* The request's pointers (src_tf, points, outputs) must stay valid until the
  * request completes.  *id receives a request id.                          */
 /* Admission by work, with no reference counterpart: a queued request joins
- * only while the resident solves' step-kernel work items (CTAs per step
- * launch) stay within max_items, so that each step launch keeps the GPU
+ * only while the resident solves' step-kernel work items (of 16 planes, or of
+ * the tuned depth) stay within max_items, so that each step launch keeps the GPU
  * full without spreading it over more solves than that needs; one solve is
  * always admitted.  0 (the default) = HBM budget and slot count only.
  * adf_step_resident_ctas gives the CTAs the GPU runs at once (one wave).  */

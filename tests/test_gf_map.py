@@ -192,6 +192,21 @@ def test_gf_map_far_lags_at_tile_edges(adf, oracle, ctx, kind, nt_gf, n_src, n_r
             assert np.linalg.norm(a - b) <= 1e-6 * np.linalg.norm(b)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["PVFromPin", "PFromPin"])
+@pytest.mark.parametrize("nt_gf,n_src,n_rec", [
+    (1, 3, 5),      # no lag older than the step's own row
+    (8, 2, 127),    # lags of one sub-block of 8 steps, a thread without a receiver
+    (9, 2, 129),    # one more lag, one more receiver than threads
+    (24, 5, 40),    # the map ends where the last sub-block's window does not
+    (31, 1, 140),   # one lag short of a block
+])
+def test_gf_map_lags_inside_a_block(adf, oracle, ctx, kind, nt_gf, n_src, n_rec):
+    """The sums of a block's own rows over sub-blocks of 8 steps, for maps shorter
+    than a block and receiver counts around its 128 threads: as above, 1e-6."""
+    test_gf_map_far_lags_at_tile_edges(adf, oracle, ctx, kind, nt_gf, n_src, n_rec)
+
+
 def test_gf_map_unknown_contraction(adf):
     ts, isr, irc = gf_inputs(40, "PVFromPin")
     with pytest.raises(KeyError):
