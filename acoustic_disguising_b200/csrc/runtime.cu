@@ -13,6 +13,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <queue>
 #include <string>
 #include <vector>
 
@@ -477,13 +478,12 @@ void cut_items(const std::vector<Solve*>& list, long long resident, std::vector<
     left += rest[i].all * (double)s->columns();
   }
   const double most = 0.6 * left / (double)resident;
-  for (;;) {
-    int i = -1;  // the solve with the largest part of it left: all end together
-    for (int k = 0; k < ns; ++k)
-      if (rest[k].lo < rest[k].hi &&
-          (i < 0 || rest[k].left / rest[k].all > rest[i].left / rest[i].all))
-        i = k;
-    if (i < 0) break;
+  // next: the solve with the largest part of it left, so that all end together
+  std::priority_queue<std::pair<double, int>> next;  // {part left, -index}
+  for (int i = 0; i < ns; ++i) next.push({1.0, -i});
+  while (!next.empty()) {
+    const int i = -next.top().second;
+    next.pop();
     const Solve* s = list[i];
     Rest& r = rest[i];
     const int planes = r.hi - r.lo;
@@ -504,6 +504,7 @@ void cut_items(const std::vector<Solve*>& list, long long resident, std::vector<
       left -= cost(s, z) * (double)s->columns();
     }
     s->add_chunk(i, z0, z0 + d, out);
+    if (r.lo < r.hi) next.push({r.left / r.all, -i});
   }
 }
 
