@@ -568,8 +568,7 @@ def serving_section(A, ctx, n_req, max_resident=0, waves=2.0, load=4.0):
                        "capacity; 120 GB HBM budget; both arms served in real time")
     small = serve_stream(A, ctx, 64, lambda n, sd: serving_requests(A, n, sd, sizes=(96, 128)),
                          max_resident, waves, load, seed=20261205)
-    small["workload"] = ("64 requests of the same stream restricted to 96^3 and 128^3 grids "
-                         "(one solve fills 23-41 % of the GPU's resident CTAs)")
+    small["workload"] = "64 requests of the same stream restricted to 96^3 and 128^3 grids"
     out["small_grids"] = small
     return out
 
