@@ -85,7 +85,9 @@ __device__ __forceinline__ void cpml_apply(R& dv, float& m, float a, float b) {
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+// (The kernels of a step start while their predecessors run, so the read-only path,
+// __ldg, is for what the set-up wrote alone: what a predecessor still writes has to be
+// read with ordinary loads, after the wait.)
 // field stores: evict-first (the next step reads them back from HBM, and the
 // halo rows that neighbouring tiles re-read are loads, which keep normal
 // priority)
@@ -381,14 +383,14 @@ __device__ __noinline__ void apply_entries(const SolveDev& S, int T, int k, int 
     if (cnt == 1) {
       const float w = __int_as_float(sg.y);
       if (rec && sg.z >= 0) S.contrib[sg.z] = __fmul_rn(w, v);
-      if (sg.w >= 0) v = __fadd_rn(v, __fmul_rn(w, __ldg(src + sg.w)));
+      if (sg.w >= 0) v = __fadd_rn(v, __fmul_rn(w, src[sg.w]));
     } else {
       for (int kk = sg.y; kk < sg.y + cnt; ++kk) {
         const float w = __ldg(S.ent_w + kk);
         const int slot = __ldg(S.ent_slot + kk);
         if (rec && slot >= 0) S.contrib[slot] = __fmul_rn(w, v);
         const int col = __ldg(S.ent_tx + kk);
-        if (col >= 0) v = __fadd_rn(v, __fmul_rn(w, __ldg(src + col)));  // receivers: src == 0
+        if (col >= 0) v = __fadd_rn(v, __fmul_rn(w, src[col]));  // receivers: src == 0
       }
     }
     *c = v;
@@ -650,8 +652,8 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
   float Zh = 0.f;
   {
     const float* vz0 = S.field + rb * S.buf_stride + 3 * cs + (long long)kfirst * plane + rowoff;
-    if (act) Z0 = ldg4(vz0);
-    if (hcol) Zh = __ldg(vz0 - 1);
+    if (act) Z0 = ld4(vz0);
+    if (hcol) Zh = vz0[-1];
   }
   // The x-slab memory of a quad is read ahead of its use: the p side's of plane
   // k+1 during the velocity update of plane k, the v side's of plane k during its

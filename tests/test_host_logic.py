@@ -182,3 +182,17 @@ def test_illumination_helpers(adf, oracle):
     for inj in (False, True):
         assert np.allclose(adf.ricker_wavelet(d, 2000.0, inj), oracle.ricker_wavelet(o, 2000.0, inj),
                            rtol=1e-13, atol=1e-13)
+
+
+def test_read_only_loads_are_of_set_up_tables():
+    """The kernels of a step overlap the end of those before them (programmatic
+    dependent launch), and __ldg is defined for memory that nobody writes while its
+    kernel runs: only what the set-up wrote may be read with it, not the field, the
+    sources or the records."""
+    csrc = os.path.join(ROOT, "acoustic_disguising_b200", "csrc")
+    tables = {"tp", "S.seg", "S.ent_w", "S.ent_slot", "S.ent_tx", "S.mask_bits"}
+    for name in ("fdtd_kernels.cu", "gf_tc_kernel.cu"):
+        txt = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        read = {m.strip() for m in re.findall(r"\b\w*ldg\w*\(\s*([^)+\-\[]+)", txt)}
+        assert read <= tables, (name, read - tables)
+        assert "ld.global.nc" not in txt and "__restrict__" not in txt, name
