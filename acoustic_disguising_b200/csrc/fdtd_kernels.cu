@@ -35,6 +35,7 @@
 
 #include "adf_internal.h"
 #include "ptx_util.h"
+#include "slab_index.h"
 
 namespace adf {
 
@@ -102,21 +103,23 @@ struct Sc {  // per-solve update scalars
 // What the CPML updates of a work item need, in shared memory: per array (p x,
 // y, z, v x, y, z) the buffer read, the one written and, for the x and y slabs,
 // the plane stride; the coefficients of the tile's columns ([3] is the halo
-// column's), rows and planes; and where the z slabs' layers lie (-1: none).
-// (Element offsets are 32-bit: a buffer holds at most 4 x 512 x 512 x 68.)  A
+// column's), rows and planes; and where the z slabs' layers lie (kNoSlab: none).
+// Places are counted in quads (slab_index.h), which hold any buffer in 32 bits; in
+// floats x-slab memory passes 2^31 at 128 x 4100 x 4100 cells and 63 layers.  A
 // boundary warp's length sets its CTA's pace, so what does not change from plane
-// to plane is worked out once per item: 8 x 256^3 with CPML 1.36 -> 1.28 ms.
+// to plane is worked out once per item.
 struct PmlTab {
-  const float* rd[6];
-  float* wr[6];
-  int stride[6];
+  const float4* rd[6];
+  float4* wr[6];
+  uint32_t stride[6];
+  uint32_t hx;  // the halo column's cell, the last of its quad, in row 0 of the p side; or kNoSlab
   alignas(16) float xpa[68];  // (read four at a time)
   alignas(16) float xpb[68];
   alignas(16) float xva[68];
   alignas(16) float xvb[68];
   float ypa[8], ypb[8], yva[8], yvb[8];
   float zpa[kMaxZc + 1], zpb[kMaxZc + 1], zva[kMaxZc + 1], zvb[kMaxZc + 1];
-  int zp[kMaxZc + 1], zv[kMaxZc + 1];
+  uint32_t zp[kMaxZc + 1], zv[kMaxZc + 1];
 };
 
 static_assert(offsetof(PmlTab, xpa) % 16 == 0 && offsetof(PmlTab, xpb) % 16 == 0 &&
@@ -130,9 +133,14 @@ struct Quad {
   // slabs (narrow grids); 21 the quad lies in the grid, 22 and is stored by the thread
   uint32_t bits;
   int j, x0, r;
-  int px, vx;  // x-slab memory of plane 0
-  int py, vy;  // y-slab memory of plane 0, -1: none
+  uint32_t px, vx;  // x-slab memory of plane 0 (quads, as in PmlTab)
+  uint32_t py, vy;  // y-slab memory of plane 0, kNoSlab: none
 };
+
+// Cell e of a quad of slab memory.
+__device__ __forceinline__ const float* slab_cell(const float4* base, uint32_t quad, int e) {
+  return reinterpret_cast<const float*>(base + quad) + e;
+}
 
 // Memory of cells that are not updated stays as it was read.
 __device__ __forceinline__ void keep_rest(float (&m)[4], float4 t, uint32_t upd) {
@@ -145,16 +153,17 @@ __device__ __forceinline__ void keep_rest(float (&m)[4], float4 t, uint32_t upd)
 // x-slab memory of a quad with cells in both slabs: cell by cell.
 template <typename R>
 __device__ __forceinline__ void x_slabs_narrow(R (&d)[4], const PmlTab& Q, int arr, int pitch,
-                                               int side1, int first1, int row, int x0, uint32_t in,
-                                               bool store, const float* a, const float* b) {
+                                               long long side, int xs1, int first1, int row, int x0,
+                                               uint32_t in, bool store, const float* a,
+                                               const float* b) {
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     if (!((in >> e) & 1u)) continue;
-    const int x = x0 + e;
-    const int o = row * pitch + (x < first1 ? x : x + side1);
-    float m = Q.rd[arr][o];
+    const int right = x0 + e >= first1;
+    const uint32_t o = slab_quad(side, right, row, pitch, right ? x0 - xs1 : x0);
+    float m = *slab_cell(Q.rd[arr], o, e);
     cpml_apply<R>(d[e], m, a[e], b[e]);
-    if (store) Q.wr[arr][o] = m;
+    if (store) reinterpret_cast<float*>(Q.wr[arr] + o)[e] = m;
   }
 }
 
@@ -192,38 +201,38 @@ __device__ __forceinline__ float4 p_update_quad(const SolveDev& S, const PmlTab&
       const float4 a4 = ld4(Q.xpa + 4 + 4 * (q.x0 / 4 % 16)), b4 = ld4(Q.xpb + 4 + 4 * (q.x0 / 4 % 16));
       const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
       if (q.bits & (1u << 20)) {
-        x_slabs_narrow<R>(dx, Q, 0, S.npp, (int)S.psi_p_side[0] - S.xs1p, S.npml, k * S.ny + q.j, q.x0,
+        x_slabs_narrow<R>(dx, Q, 0, S.npp, S.psi_p_side[0], S.xs1p, S.npml, k * S.ny + q.j, q.x0,
                           q.bits >> 12, owned, a, b);
       } else {
-        const int o = q.px + k * Q.stride[0];
+        const uint32_t o = q.px + k * Q.stride[0];
         const float4 t = mx;
         float m[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e)
           if ((q.bits >> (12 + e)) & 1u) cpml_apply<R>(dx[e], m[e], a[e], b[e]);
         // cells outside the slab or not updated write back what they read
-        if (owned) st4(Q.wr[0] + o, make_float4(m[0], m[1], m[2], m[3]));
+        if (owned) Q.wr[0][o] = make_float4(m[0], m[1], m[2], m[3]);
       }
     }
-    if (q.py >= 0) {  // y slab: the whole quad, cells that are not updated keep their memory
-      const int o = q.py + k * Q.stride[1];
-      const float4 t = ld4(Q.rd[1] + o);
+    if (q.py != kNoSlab) {  // y slab: the whole quad, cells that are not updated keep their memory
+      const uint32_t o = q.py + k * Q.stride[1];
+      const float4 t = Q.rd[1][o];
       float m[4] = {t.x, t.y, t.z, t.w};
       const float a = Q.ypa[q.r], b = Q.ypb[q.r];
 #pragma unroll
       for (int e = 0; e < 4; ++e) cpml_apply<R>(dy[e], m[e], a, b);
       if (up != 15u) keep_rest(m, t, up);
-      if (owned) st4(Q.wr[1] + o, make_float4(m[0], m[1], m[2], m[3]));
+      if (owned) Q.wr[1][o] = make_float4(m[0], m[1], m[2], m[3]);
     }
-    if (Q.zp[u] >= 0 && (q.bits & (1u << 21))) {
-      const int o = Q.zp[u] + q.j * S.nxp + q.x0;
-      const float4 t = ld4(Q.rd[2] + o);
+    if (Q.zp[u] != kNoSlab && (q.bits & (1u << 21))) {
+      const uint32_t o = Q.zp[u] + ((uint32_t)(q.j * S.nxp + q.x0) >> 2);
+      const float4 t = Q.rd[2][o];
       float m[4] = {t.x, t.y, t.z, t.w};
       const float a = Q.zpa[u], b = Q.zpb[u];
 #pragma unroll
       for (int e = 0; e < 4; ++e) cpml_apply<R>(dz[e], m[e], a, b);
       if (up != 15u) keep_rest(m, t, up);
-      if (owned) st4(Q.wr[2] + o, make_float4(m[0], m[1], m[2], m[3]));
+      if (owned) Q.wr[2][o] = make_float4(m[0], m[1], m[2], m[3]);
     }
   }
   const float Pv[4] = {P4.x, P4.y, P4.z, P4.w};
@@ -236,15 +245,16 @@ __device__ __forceinline__ float4 p_update_quad(const SolveDev& S, const PmlTab&
   return make_float4(o[0], o[1], o[2], o[3]);
 }
 
-// The same update for one cell (the halo column x = xb-1 of an x tile), from
-// the staged plane `st` (P, Vx, Vy of plane k; `c` the cell's offset in a
-// channel, `cst` the channel stride) and Vz of planes k and k+1 (Z0, Z1).
+// The same update for the cell before a tile's first quad q (the halo column
+// x = xb-1 of an x tile), from the staged plane `st` (P, Vx, Vy of plane k; `c` the
+// cell's offset in a channel, `cst` the channel stride) and Vz of planes k and k+1
+// (Z0, Z1).  Its y and z slab memory lies one float before the quad's.
 template <typename R>
-__device__ __forceinline__ float p_update_cell(const SolveDev& S, const PmlTab& Q, const Sc<R>& g,
-                                               bool pcpml, const float* st, float Z0, float Z1, int c,
-                                               int cst, int x, int j, int r, int k, int u, bool masked) {
+__device__ __forceinline__ float p_update_cell(const SolveDev& S, const PmlTab& Q, const Quad& q,
+                                               const Sc<R>& g, bool pcpml, const float* st, float Z0,
+                                               float Z1, int c, int cst, int k, int u, bool masked) {
   using A = Arith<R>;
-  const int nx = S.nx, ny = S.ny, nz = S.nz, npml = S.npml, nxp = S.nxp;
+  const int nx = S.nx, ny = S.ny, nz = S.nz, x = q.x0 - 1, j = q.j, r = q.r;
   const bool rigid_y = j == ny - 1, rigid_z = k == nz - 1;
   const bool plain_rigid = rigid_y || rigid_z;
   const bool upd = x <= nx - 2 && !(rigid_y && rigid_z);
@@ -261,17 +271,16 @@ __device__ __forceinline__ float p_update_cell(const SolveDev& S, const PmlTab& 
   if (!plain_rigid) {
     if (masked) open = (S.mask_bits[((long long)k * ny + j) * S.mw + (x >> 3)] >> (4 * (x & 7))) & 1u;
     if (pcpml) {
-      if (x < npml || x >= nx - npml) {
-        float m = Q.rd[0][(k * ny + j) * S.npp + (x < npml ? x : (int)S.psi_p_side[0] + x - S.xs1p)];
+      if (Q.hx != kNoSlab) {
+        float m = *slab_cell(Q.rd[0], Q.hx + slab_quad(0, 0, k * ny + j, S.npp, 0), 3);
         cpml_apply<R>(dvx, m, Q.xpa[3], Q.xpb[3]);
       }
-      if (j < npml || j >= ny - npml) {
-        float m = Q.rd[1][(j < npml ? 0 : (int)S.psi_p_side[1]) +
-                          (k * npml + (j < npml ? j : j - (ny - npml))) * nxp + x];
+      if (q.py != kNoSlab) {
+        float m = *slab_cell(Q.rd[1], q.py + k * Q.stride[1], -1);
         cpml_apply<R>(dvy, m, Q.ypa[r], Q.ypb[r]);
       }
-      if (Q.zp[u] >= 0) {
-        float m = Q.rd[2][Q.zp[u] + j * nxp + x];
+      if (Q.zp[u] != kNoSlab) {
+        float m = *slab_cell(Q.rd[2], Q.zp[u] + ((uint32_t)(j * S.nxp + q.x0) >> 2), -1);
         cpml_apply<R>(dvz, m, Q.zpa[u], Q.zpb[u]);
       }
     }
@@ -304,37 +313,37 @@ __device__ __forceinline__ void v_update_quad(const SolveDev& S, const PmlTab& Q
       const float4 a4 = ld4(Q.xva + 4 + 4 * (q.x0 / 4 % 16)), b4 = ld4(Q.xvb + 4 + 4 * (q.x0 / 4 % 16));
       const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
       if (q.bits & (1u << 20)) {
-        x_slabs_narrow<R>(dx, Q, 3, S.nvp, (int)S.psi_v_side[0] - S.xs1v, S.npml + 1, k * S.ny + q.j,
-                          q.x0, q.bits >> 16, true, a, b);
+        x_slabs_narrow<R>(dx, Q, 3, S.nvp, S.psi_v_side[0], S.xs1v, S.npml + 1, k * S.ny + q.j, q.x0,
+                          q.bits >> 16, true, a, b);
       } else {
-        const int o = q.vx + k * Q.stride[3];
+        const uint32_t o = q.vx + k * Q.stride[3];
         const float4 t = mx;
         float m[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e)
           if ((q.bits >> (16 + e)) & 1u) cpml_apply<R>(dx[e], m[e], a[e], b[e]);
-        st4(Q.wr[3] + o, make_float4(m[0], m[1], m[2], m[3]));
+        Q.wr[3][o] = make_float4(m[0], m[1], m[2], m[3]);
       }
     }
-    if (q.vy >= 0) {
-      const int o = q.vy + k * Q.stride[4];
-      const float4 t = ld4(Q.rd[4] + o);
+    if (q.vy != kNoSlab) {
+      const uint32_t o = q.vy + k * Q.stride[4];
+      const float4 t = Q.rd[4][o];
       float m[4] = {t.x, t.y, t.z, t.w};
       const float a = Q.yva[q.r], b = Q.yvb[q.r];
 #pragma unroll
       for (int e = 0; e < 4; ++e) cpml_apply<R>(dy[e], m[e], a, b);
       if (in != 15u) keep_rest(m, t, in);
-      st4(Q.wr[4] + o, make_float4(m[0], m[1], m[2], m[3]));
+      Q.wr[4][o] = make_float4(m[0], m[1], m[2], m[3]);
     }
-    if (Q.zv[u] >= 0 && (q.bits & (1u << 22))) {
-      const int o = Q.zv[u] + q.j * S.nxp + q.x0;
-      const float4 t = ld4(Q.rd[5] + o);
+    if (Q.zv[u] != kNoSlab && (q.bits & (1u << 22))) {
+      const uint32_t o = Q.zv[u] + ((uint32_t)(q.j * S.nxp + q.x0) >> 2);
+      const float4 t = Q.rd[5][o];
       float m[4] = {t.x, t.y, t.z, t.w};
       const float a = Q.zva[u], b = Q.zvb[u];
 #pragma unroll
       for (int e = 0; e < 4; ++e) cpml_apply<R>(dz[e], m[e], a, b);
       if (in != 15u) keep_rest(m, t, in);
-      st4(Q.wr[5] + o, make_float4(m[0], m[1], m[2], m[3]));
+      Q.wr[5][o] = make_float4(m[0], m[1], m[2], m[3]);
     }
   }
   const uint32_t ux = (q.bits >> 4) & 15u, uy = q.j >= 1 ? in : 0u, uz = k >= 1 ? in : 0u;
@@ -508,24 +517,25 @@ __device__ __noinline__ void fetch_slabs(const SolveDev& S, const PmlTab& Q, int
     const bool lo = X == 0, hi = (X + 1) * kXT >= S.nxp, xv = arr == 3;
     if ((!lo && !hi) || S.chan_stride < kFetchXCells) return;
     const int pitch = xv ? S.nvp : S.npp, j0 = max(j, 0), j1 = min(j + S.ty + 1, S.ny);
-    const int side = lo ? 0 : (int)(xv ? S.psi_v_side[0] : S.psi_p_side[0]);
-    const float* p = Q.rd[xv ? 3 : 0] + (side + (k * S.ny + j0) * pitch);
+    const float* p = slab_cell(Q.rd[xv ? 3 : 0],
+                               slab_quad(xv ? S.psi_v_side[0] : S.psi_p_side[0], !lo, k * S.ny + j0,
+                                         pitch, 0), 0);
     for (int i = 0; i < (j1 - j0) * pitch; i += line) prefetch_l2(p + i);
     return;
   }
   if (j < 0) return;
-  int o;
+  uint32_t o;
   if (arr < 2) {
-    const int m = n + (v ? 1 : 0);  // layers
-    if (j >= m && j < S.ny - m) return;
-    o = (j < m ? 0 : (int)(v ? S.psi_v_side[1] : S.psi_p_side[1])) +
-        (k * m + (j < m ? j : j - (S.ny - m))) * S.nxp;
+    const int m = n + (v ? 1 : 0), right = j >= m;  // layers
+    if (right && j < S.ny - m) return;
+    o = slab_quad(v ? S.psi_v_side[1] : S.psi_p_side[1], right,
+                  k * m + (right ? j - (S.ny - m) : j), S.nxp, xb);
   } else {
     o = v ? Q.zv[k - kfirst] : Q.zp[k - kfirst];
-    if (o < 0) return;
-    o += j * S.nxp;
+    if (o == kNoSlab) return;
+    o += slab_quad(0, 0, j, S.nxp, xb);
   }
-  const float* p = Q.rd[(arr < 2 ? 1 : 2) + (v ? 3 : 0)] + (o + xb);
+  const float* p = slab_cell(Q.rd[(arr < 2 ? 1 : 2) + (v ? 3 : 0)], o, 0);
 #pragma unroll
   for (int i = 0; i < kXT; i += line)
     if (i < S.nxp - xb) prefetch_l2(p + i);
@@ -573,7 +583,7 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
   q.r = r;
   q.bits = 0;
   q.px = q.vx = 0;
-  q.py = q.vy = -1;
+  q.py = q.vy = kNoSlab;
   {
     int seen = 0;  // x slabs that the quad's cells lie in: 1 left, 2 right
 #pragma unroll
@@ -595,14 +605,16 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
     if (act) q.bits |= 1u << 21;
     if (vrow) q.bits |= 1u << 22;
     if (act && pcp) {
-      q.px = j * S.npp + ((seen & 1) ? x0 : (int)S.psi_p_side[0] + x0 - S.xs1p);
+      const int right = !(seen & 1);
+      q.px = slab_quad(S.psi_p_side[0], right, j, S.npp, right ? x0 - S.xs1p : x0);
       const int ys = j < npml ? 0 : (j >= ny - npml ? 1 : -1);
-      if (ys >= 0) q.py = ys * (int)S.psi_p_side[1] + (ys == 0 ? j : j - (ny - npml)) * nxp + x0;
+      if (ys >= 0) q.py = slab_quad(S.psi_p_side[1], ys, ys == 0 ? j : j - (ny - npml), nxp, x0);
     }
     if (vrow && vcp) {
-      q.vx = j * S.nvp + ((seen & 4) ? x0 : (int)S.psi_v_side[0] + x0 - S.xs1v);
+      const int right = !(seen & 4);
+      q.vx = slab_quad(S.psi_v_side[0], right, j, S.nvp, right ? x0 - S.xs1v : x0);
       const int ys = j < 1 ? -1 : (j <= npml ? 0 : (j >= ny - npml - 1 ? 1 : -1));
-      if (ys >= 0) q.vy = ys * (int)S.psi_v_side[1] + (ys == 0 ? j : j - (ny - npml - 1)) * nxp + x0;
+      if (ys >= 0) q.vy = slab_quad(S.psi_v_side[1], ys, ys == 0 ? j : j - (ny - npml - 1), nxp, x0);
     }
   }
   // warp-uniform: do all of the warp's rows and x cells take the plain P
@@ -663,10 +675,10 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
   const bool pxm = (q.bits & 0xF000u) && !(q.bits & (1u << 20));
   const bool vxm = (q.bits & 0xF0000u) && !(q.bits & (1u << 20));
   float4 mpx = make_float4(0.f, 0.f, 0.f, 0.f), mvx = mpx;
-  if (pxm) mpx = ld4(Q.rd[0] + q.px + kfirst * Q.stride[0]);
+  if (pxm) mpx = Q.rd[0][q.px + kfirst * Q.stride[0]];
   for (int k = kfirst; k < z1; ++k) {
     const bool prologue = k < z0;
-    if (vxm) mvx = ld4(Q.rd[3] + q.vx + k * Q.stride[3]);
+    if (vxm) mvx = Q.rd[3][q.vx + k * Q.stride[3]];
     const int u = k - kfirst;
     float* pn = sPn + (k & 1) * (kMaxTy + 1) * kPnPitch;
     const float* st = ring + slot_of(k) * kStageFloats;
@@ -704,12 +716,11 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
                                 __fsub_rn(st[2 * cst + so - 1 + kStageW], st[2 * cst + so - 1]),
                                 __fsub_rn(Zh1, Zh), g);
       else
-        pn[pq - 1] = p_update_cell<R>(S, Q, g, pcp, st, Zh, Zh1, so - 1, cst, xb - 1, j, r, k, u,
-                                      has_mask);
+        pn[pq - 1] = p_update_cell<R>(S, Q, q, g, pcp, st, Zh, Zh1, so - 1, cst, k, u, has_mask);
       Zh = Zh1;
     }
     __syncthreads();
-    if (pxm && k + 1 < z1) mpx = ld4(Q.rd[0] + q.px + (k + 1) * Q.stride[0]);
+    if (pxm && k + 1 < z1) mpx = Q.rd[0][q.px + (k + 1) * Q.stride[0]];
     // every read of plane k's stage is done: refill its slot
     if (tid == 0 && k + kStepRing < z1) issue(k + kStepRing);
     // ---- q channel: inject/record on the new P (forward.jl:92) ----
@@ -781,7 +792,7 @@ __device__ __forceinline__ void pml_table(const SolveDev& G, PmlTab& Q, int4 ite
                                           int tid, int nthr) {
   const int n = G.npml, nb = 4 * n + 2;
   if (n == 0) {
-    for (int u = tid; u < item.w - kfirst; u += nthr) Q.zp[u] = Q.zv[u] = -1;
+    for (int u = tid; u < item.w - kfirst; u += nthr) Q.zp[u] = Q.zv[u] = kNoSlab;
     return;
   }
   const float* co = G.coef;
@@ -790,9 +801,16 @@ __device__ __forceinline__ void pml_table(const SolveDev& G, PmlTab& Q, int4 ite
     const bool v = tid >= 3;
     float* base = v ? G.psi_v[a] : G.psi_p[a];
     const long long buf = v ? G.psi_v_buf[a] : G.psi_p_buf[a];
-    Q.rd[tid] = base + rb * buf;
-    Q.wr[tid] = base + (rb ^ 1) * buf;
-    Q.stride[tid] = a == 0 ? G.ny * (v ? G.nvp : G.npp) : (n + (v ? 1 : 0)) * G.nxp;
+    Q.rd[tid] = reinterpret_cast<const float4*>(base + rb * buf);
+    Q.wr[tid] = reinterpret_cast<float4*>(base + (rb ^ 1) * buf);
+    Q.stride[tid] = a == 0 ? slab_quad(0, 0, G.ny, v ? G.nvp : G.npp, 0)
+                           : slab_quad(0, 0, n + (v ? 1 : 0), G.nxp, 0);
+  }
+  if (tid == 6) {
+    const int x = (item.y >> 16) * kXT - 1, right = x >= n;
+    Q.hx = x < 0 || (right && x < G.nx - n) ? kNoSlab
+                                            : slab_quad(G.psi_p_side[0], right, 0, G.npp,
+                                                        right ? x - G.xs1p : x);
   }
   // index of the coefficient of cell x of an axis of m cells, -1: no slab
   auto cp = [&](int x, int m) { return x < 0 || x >= m ? -1 : x < n ? x : (x >= m - n ? n + x - (m - n) : -1); };
@@ -819,11 +837,12 @@ __device__ __forceinline__ void pml_table(const SolveDev& G, PmlTab& Q, int4 ite
     const int c0 = max(c, 0), v0 = max(v, 0);
     const float ca = co[c0], cb = co[nb + c0], wa = co[v0], wb = co[nb + v0];
     if (i >= 73) {
-      const int pl = G.ny * G.nxp;
-      Q.zp[e] = c < 0 ? -1 : (c >= n ? (int)G.psi_p_side[2] : 0) + (c >= n ? c - n : c) * pl;
-      Q.zv[e] = v < 0 ? -1
-                      : (v >= 3 * n + 1 ? (int)G.psi_v_side[2] : 0) +
-                            (v >= 3 * n + 1 ? v - 3 * n - 1 : v - 2 * n) * pl;
+      const int top = c >= n, vtop = v >= 3 * n + 1;
+      Q.zp[e] = c < 0 ? kNoSlab
+                      : slab_quad(G.psi_p_side[2], top, (top ? c - n : c) * G.ny, G.nxp, 0);
+      Q.zv[e] = v < 0 ? kNoSlab
+                      : slab_quad(G.psi_v_side[2], vtop, (vtop ? v - 3 * n - 1 : v - 2 * n) * G.ny,
+                                  G.nxp, 0);
     }
     pa[e] = ca, pb[e] = cb, va[e] = wa, vb[e] = wb;
   }

@@ -24,6 +24,7 @@
 #include <cudaTypedefs.h>
 
 #include "runtime.h"
+#include "slab_index.h"
 
 namespace adf {
 cudaError_t launch_cpml_profiles(int n, double vel_max, double dt, double rcoef, double thickness,
@@ -341,6 +342,8 @@ int solve_alloc(adf_ctx* ctx, Solve& s, const hm::Dom& dom, int npml, bool has_m
   const long long ps[3] = {nz * ny * d.npp, nz * n * nxp, n * ny * nxp};
   const long long vs[3] = {nz * ny * d.nvp, nz * nm * nxp, nm * ny * nxp};
   for (int a = 0; a < 3; ++a) {
+    if (ps[a] >= kMaxSideFloats || vs[a] >= kMaxSideFloats)
+      return fail(ADF_E_ARG, "CPML memory of a side past 2^33 floats is not supported");
     d.psi_p_side[a] = ps[a];
     d.psi_p_buf[a] = 2 * ps[a];
     d.psi_v_side[a] = vs[a];
