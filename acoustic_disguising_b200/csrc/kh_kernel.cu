@@ -73,6 +73,7 @@ constexpr KhT kKhT[3] = {{17, 1.0}, {13, 0.811}, {7, 0.492}};  // measured, 592 
 struct KhParams {
   int ns, nr, nt;
   int t_base;       // first output sample of this launch
+  int t_len;        // and how many of the trace it covers
   int splits;       // parts of the surface, one per blockIdx.z
   int group;        // points summed before each compensated add, a power of two
   int sc;           // surface points per chunk
@@ -96,7 +97,7 @@ struct KhParams {
                         // the pair of sample t at 2 (pad + t)
   const float* cs_f;    // running sum of in_f, same layout (velocity output)
   float* out;           // (nt, nr)
-  float2* part;         // splits > 1: [splits][nr][nt] {sum, compensation} instead
+  float2* part;         // splits > 1: [splits][nr][t_len] {sum, compensation} instead
   int* err;
   unsigned wait_limit;  // polls of a chunk's bounded wait (kWaitLimit)
   int skip_chunk;       // test hook: chunk whose copies are not issued (-1: none)
@@ -373,7 +374,7 @@ __global__ void __launch_bounds__(KH_THREADS, 1) adf_kh_pressure_kernel(KhParams
     if (r >= p.nr) continue;
     const int t0 = tb + T * lane;
     float* o = p.out + (size_t)r * p.nt + t0;
-    float2* q = p.part + ((size_t)blockIdx.z * p.nr + r) * p.nt + t0;
+    float2* q = p.part + ((size_t)blockIdx.z * p.nr + r) * p.t_len + (t0 - p.t_base);
 #pragma unroll
     for (int j = 0; j < T; ++j) {
       if (t0 + j >= p.nt) continue;
@@ -385,19 +386,19 @@ __global__ void __launch_bounds__(KH_THREADS, 1) adf_kh_pressure_kernel(KhParams
   }
 }
 
-// Adds the surface parts of output samples t0 .. t1-1, in part order, in Float64.
+// Adds the surface parts of output samples t0 .. t0+len-1, in part order, in Float64.
 __global__ void adf_kh_combine_kernel(const float2* __restrict__ part, float* __restrict__ out,
-                                      int nr, int nt, int t0, int t1, int splits) {
-  const long long n = (long long)nr * nt;
+                                      int nr, int nt, int t0, int len, int splits) {
+  const long long n = (long long)nr * len;
   for (int r = blockIdx.x; r < nr; r += gridDim.x)
-    for (int t = t0 + (int)threadIdx.x; t < t1; t += blockDim.x) {
-      const long long i = (long long)r * nt + t;
+    for (int t = (int)threadIdx.x; t < len; t += blockDim.x) {
+      const float2* p = part + (long long)r * len + t;
       double a = 0.0;
       for (int z = 0; z < splits; ++z) {
-        const float2 v = part[z * n + i];
+        const float2 v = p[z * n];
         a += (double)v.x - (double)v.y;
       }
-      out[i] = (float)a;
+      out[(long long)r * nt + t0 + t] = (float)a;
     }
 }
 
@@ -511,6 +512,7 @@ __global__ void adf_kh_gather_kernel(const float* q, const float* f, int ntx, in
 // partial sums.  Estimated in us from the measured time of a surface point.
 // 200 points -> 48 targets x 700 samples: 283 us in one part, 49 in 16 or more;
 // 2048 -> 4096 x 500: 6.95 and 6.16 ms.
+// A part's sums take 8 bytes a target and sample, 256 MB in all at most.
 static int kh_splits(int nsm, long long ctas, int ns, int nr, int samples, double point_us) {
   int best = 1;
   double best_us = 1e300;
@@ -574,7 +576,7 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
   // Time blocks: whole blocks of the longest T, and a last one of the shortest
   // that holds the rest (2048 samples: 3 x 544 + 416, none padded)
   struct Launch {
-    int t, nb, t_base;  // kKhT index, blocks, first sample
+    int t, nb, t_base, t_len;  // kKhT index, blocks, first sample, samples of the trace
     int rowpad, sc, splits;
     size_t smem;
   };
@@ -585,8 +587,8 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
     for (int t = 1; t < 3; ++t)
       if (rest <= 32 * kKhT[t].T) last = t;
     if (rest > 0 && last == 0) ++whole;
-    if (whole > 0) runs.push_back({0, whole, 0, 0, 0, 1, 0});
-    if (rest > 0 && last > 0) runs.push_back({last, 1, nt - rest, 0, 0, 1, 0});
+    if (whole > 0) runs.push_back({0, whole, 0, 0, 0, 0, 1, 0});
+    if (rest > 0 && last > 0) runs.push_back({last, 1, nt - rest, 0, 0, 0, 1, 0});
   }
   const int ntiles = (nr + KH_RT - 1) / KH_RT;
   std::vector<int2> tlo((size_t)ntiles);
@@ -633,12 +635,13 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
   // the tail covers the last time block's window end.
   const int pad = (lo_all + lm + 4 + 3) / 4 * 4;
   const long long pitch = ((long long)pad + t_end + lo_all + 16 + 3) / 4 * 4;
-  int splits = 1;  // the most of any launch
+  size_t parts = 0;  // of the launch with the most; the next one reuses them
   for (Launch& l : runs) {
+    l.t_len = std::min(nt - l.t_base, l.nb * 32 * kKhT[l.t].T);
     if (ctx->kh_skip_chunk < 0)
-      l.splits = kh_splits(ctx->nsm, (long long)ntiles * l.nb, ns, nr, std::min(nt - l.t_base, l.nb * 32 * kKhT[l.t].T),
+      l.splits = kh_splits(ctx->nsm, (long long)ntiles * l.nb, ns, nr, l.t_len,
                            1.7 * kKhT[l.t].cost * lm / 16.0);
-    splits = std::max(splits, l.splits);
+    if (l.splits > 1) parts = std::max(parts, (size_t)l.splits * l.t_len * nr);
   }
 
   // scratch from the context's pool: after the first call of a size the
@@ -652,10 +655,11 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
       !dq.alloc((size_t)pitch * ns) || !df.alloc((size_t)pitch * ns) ||
       !dqf.alloc((size_t)2 * pitch * ns) ||
       !dout.alloc((size_t)nt * nr) ||
-      (splits > 1 && !dpart.alloc((size_t)splits * nt * nr)) ||
       !dtlo.alloc((size_t)ntiles) || !derr.alloc(1) ||
       (kind && (!drn.alloc((size_t)3 * nr) || !dc.alloc((size_t)pitch * ns))))
     return fail(ADF_E_NOMEM, "adf_kh_pressure: device allocation failed");
+  if (parts > 0 && !dpart.alloc(parts))  // no room for parts: one
+    for (Launch& l : runs) l.splits = 1;
   std::vector<float> csum;
   if (kind) {  // running sum of in_f per surface point, in Float64, stored Float32
     csum.resize((size_t)nt * ns);
@@ -738,6 +742,7 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
     e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
     if (e != cudaSuccess) return fail(ADF_E_DEVICE, std::string("kh smem: ") + cudaGetErrorString(e));
     p.t_base = l.t_base;
+    p.t_len = l.t_len;
     p.splits = l.splits;
     // (parts sum their points in another order than one pass does: groups half as
     // long keep their error below its, at 1 % of the time)
@@ -748,7 +753,7 @@ static int kh_run(adf_ctx* ctx, const adf_kh_desc* d, const float* in_q, const f
     e = cudaGetLastError();
     if (e == cudaSuccess && l.splits > 1) {
       adf_kh_combine_kernel<<<std::min(nr, ctx->nsm * 8), 256, 0, st>>>(
-          dpart.p, dout.p, nr, nt, l.t_base, std::min(nt, l.t_base + l.nb * 32 * kKhT[l.t].T), l.splits);
+          dpart.p, dout.p, nr, nt, l.t_base, l.t_len, l.splits);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) return fail(ADF_E_DEVICE, std::string("kh launch: ") + cudaGetErrorString(e));

@@ -193,3 +193,33 @@ def test_kh_parts_and_time_blocks(adf, oracle, ctx, ns, nr, nt):
     assert rel_l2(out, ref) <= 1e-6
     if nt > 544:
         assert np.abs(ref[544:]).max() > 0 and rel_l2(out[544:], ref[544:]) <= 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ns,blocks", [
+    (512, 20),  # the last block of 10 samples in 12 parts, the others in one
+    (256, 8),   # the last block in 7 parts, the others in two
+])
+def test_kh_parts_take_the_memory_of_their_launch(adf, oracle, ns, blocks):
+    """A long trace whose short last block is summed in many parts takes, besides its
+    inputs and result, the 256 MB that parts may take at most (2.5 GB for the first
+    case's whole trace in 12 parts), and every launch's parts are added up."""
+    import torch
+
+    nr, nt = 2400, blocks * 544 + 10
+    c = case(ns, nr, nt, 5e-6, 0.25, 0.35)
+    own = adf.Context(0)
+    args = (c["dt"], c["sigma"], C0, c["aq"], c["af"])
+    adf.kh_pressure(c["sp"][:40], c["sn"][:40], c["rp"][:20], c["q"][:100, :40], c["f"][:100, :40],
+                    *args, ctx=own)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    out = adf.kh_pressure(c["sp"], c["sn"], c["rp"], c["q"], c["f"], *args, ctx=own)
+    used = free - torch.cuda.mem_get_info()[0]  # a context's pool keeps what a KH call took
+    columns = 4 * 4 * ns * (nt + 1000)          # q, f and their pairs, padded
+    assert used <= columns + 4 * nt * nr + 256e6 + 64e6  # (the pool grows in steps)
+    pick = np.r_[0:3, nr - 3:nr]
+    ref = oracle.kh_pressure(c["sp"], c["sn"], c["rp"][pick], c["q"], c["f"], *args)
+    for part in (slice(0, nt - 10), slice(nt - 10, nt)):
+        assert np.abs(ref[part]).max() > 0
+        assert rel_l2(out[part][:, pick], ref[part]) <= 1e-6
