@@ -131,8 +131,9 @@ struct EpiParams {
 // (programmatic dependent launch); not after anything that writes the descriptors
 cudaError_t launch_step(const StepParams& p, int grid, int max_ty, bool overlap, cudaStream_t s);
 // layout conversions of a call's arrays (runtime.cu): src[c][r] -> dst[r][c] over
-// cols x rows, and rows of `width` floats from one pitch to another
-cudaError_t launch_transpose(const float* src, float* dst, int rows, int cols, cudaStream_t s);
+// cols x rows, and rows of `width` floats, each from one pitch to another
+cudaError_t launch_transpose(const float* src, long long src_pitch, float* dst, long long dst_pitch,
+                             int rows, int cols, cudaStream_t s);
 cudaError_t launch_repitch(const float* src, long long src_pitch, float* dst, long long dst_pitch,
                            int width, long long rows, cudaStream_t s);
 // fills SolveDev.closed from the mask bits (set-up)

@@ -407,24 +407,27 @@ cudaError_t launch_gf_postprocess(int ncol, int n, int nt_out, double t_in0, dou
 // samples in and eight out took 180 ms of a 192^3 run).
 // src[c][r] -> dst[r][c]: 32 x 32 tiles through shared memory.
 __global__ void __launch_bounds__(256) adf_transpose_kernel(const float* __restrict__ src,
-                                                            float* __restrict__ dst, int rows,
-                                                            int cols) {
+                                                            long long src_pitch,
+                                                            float* __restrict__ dst,
+                                                            long long dst_pitch, int rows, int cols) {
   __shared__ float tile[32][33];
   const int tr = (rows + 31) / 32;
   const int r0 = (int)(blockIdx.x % tr) * 32, c0 = (int)(blockIdx.x / tr) * 32;
   for (int i = threadIdx.y; i < 32; i += 8)
     if (c0 + i < cols && r0 + (int)threadIdx.x < rows)
-      tile[i][threadIdx.x] = src[(long long)(c0 + i) * rows + r0 + threadIdx.x];
+      tile[i][threadIdx.x] = src[(c0 + i) * src_pitch + r0 + threadIdx.x];
   __syncthreads();
   for (int i = threadIdx.y; i < 32; i += 8)
     if (r0 + i < rows && c0 + (int)threadIdx.x < cols)
-      dst[(long long)(r0 + i) * cols + c0 + threadIdx.x] = tile[threadIdx.x][i];
+      dst[(r0 + i) * dst_pitch + c0 + threadIdx.x] = tile[threadIdx.x][i];
 }
 
-cudaError_t launch_transpose(const float* src, float* dst, int rows, int cols, cudaStream_t s) {
+cudaError_t launch_transpose(const float* src, long long src_pitch, float* dst, long long dst_pitch,
+                             int rows, int cols, cudaStream_t s) {
   const long long tiles = (long long)((rows + 31) / 32) * ((cols + 31) / 32);
   if (tiles == 0) return cudaSuccess;
-  adf_transpose_kernel<<<(unsigned)tiles, dim3(32, 8), 0, s>>>(src, dst, rows, cols);
+  adf_transpose_kernel<<<(unsigned)tiles, dim3(32, 8), 0, s>>>(src, src_pitch, dst, dst_pitch, rows,
+                                                               cols);
   return cudaGetLastError();
 }
 

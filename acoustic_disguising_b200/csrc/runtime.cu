@@ -104,16 +104,14 @@ size_t solve_bytes_estimate(int64_t nx, int64_t ny, int64_t nz, int64_t npml, in
   int nxp, ty, nzc, mw;
   choose_tiles((int)nx, (int)ny, (int)nz, nxp, ty, nzc, mw);
   size_t b = 2ull * 4 * nz * ny * nxp * 4;
-  if (mask) {  // the bits, and a byte per tile and plane
-    b += (size_t)mw * ny * nz * 4;
-    b += (size_t)((nxp + step_x_tile() - 1) / step_x_tile()) * ((ny + ty - 1) / ty) * nz;
-  }
+  if (mask) b += (size_t)mw * ny * nz * 4;
   size_t n = npml;
   b += 2ull * 2 * 4 * (nz * ny * n + nz * n * nxp + n * ny * nxp);
   b += 2ull * 2 * 4 * (nz * ny * (n + 1) + nz * (n + 1) * nxp + (n + 1) * ny * nxp);
   b += 10ull * nt * ntx * 4;
   b += (size_t)ntx * 4 * 8 * 4 * 3;  // contributions + entries
   b += (size_t)((ny + ty - 1) / ty) * nz * 4 * 4;
+  // small tables; a mask's byte per tile and plane (1 MiB per 15 GB of field)
   return b + (1 << 20);
 }
 
@@ -771,19 +769,47 @@ using namespace adf;
 // ---------------------------------------------------------------------------
 // layout helpers
 // ---------------------------------------------------------------------------
-// Each array crosses as the caller holds it, through a device buffer `stage`
-// that the next one reuses in stream order; kernels convert the layout.  A
-// pageable source is staged before cudaMemcpyAsync returns, and a copy to
-// pageable memory has arrived when it returns.
+// Each array crosses as the caller holds it, through device memory that the next
+// piece reuses in stream order; kernels convert the layout.  That memory is the
+// field buffer that no step reads or writes at the time (buffer 1 before the first
+// step, the last step's input after it), so that a run needs no more than its
+// solve; a grid below kStageMin, whose buffer would cut the arrays into very small
+// pieces, has a buffer of its own, within the estimate's last MiB.  A pageable
+// source is staged before cudaMemcpyAsync returns, and a copy to pageable memory
+// has arrived when it returns.
+constexpr size_t kStageMin = (size_t)1 << 18;  // floats
+struct Stage {
+  float* p;
+  size_t floats;
+};
+
+// Pieces {first column, columns, first sample, samples} of an (nt, ntx) array,
+// each contiguous in it and no larger than `room`: whole columns, or parts of one.
+template <typename F>
+static cudaError_t trace_pieces(size_t nt, size_t ntx, size_t room, F&& piece) {
+  const size_t dt = std::min(nt, room), dc = nt <= room ? room / nt : 1;
+  for (size_t c = 0; c < ntx; c += dc)
+    for (size_t t = 0; t < nt; t += dt) {
+      const cudaError_t e = piece(c, std::min(dc, ntx - c), t, std::min(dt, nt - t));
+      if (e != cudaSuccess) return e;
+    }
+  return cudaSuccess;
+}
 
 // Julia (nt, ntx) time-fastest -> device [nt][ntx] transceiver-fastest
-static cudaError_t upload_traces(Solve& s, const adf_txgrid* txs, float* stage, cudaStream_t st) {
+static cudaError_t upload_traces(Solve& s, const adf_txgrid* txs, Stage stage, cudaStream_t st) {
   SolveDev& d = s.dev;
-  const size_t bytes = (size_t)d.nt * d.ntx * 4;
+  const size_t nt = d.nt, ntx = d.ntx;
   cudaError_t e = cudaSuccess;
   auto up = [&](const float* jl, float* dst) {
-    if (e == cudaSuccess) e = cudaMemcpyAsync(stage, jl, bytes, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = launch_transpose(stage, dst, d.nt, d.ntx, st);
+    if (e != cudaSuccess) return;
+    e = trace_pieces(nt, ntx, stage.floats, [&](size_t c, size_t nc, size_t t, size_t n) {
+      const cudaError_t ce =
+          cudaMemcpyAsync(stage.p, jl + c * nt + t, nc * n * 4, cudaMemcpyHostToDevice, st);
+      return ce != cudaSuccess ? ce
+                               : launch_transpose(stage.p, (long long)n, dst + t * ntx + c,
+                                                  (long long)ntx, (int)n, (int)nc, st);
+    });
   };
   for (int c = 0; c < 4; ++c) {
     up(txs->src[c], d.src[c]);
@@ -799,14 +825,20 @@ static cudaError_t upload_traces(Solve& s, const adf_txgrid* txs, float* stage, 
 // Device (step-major) traces -> the caller's Julia (nt, ntx) arrays; with
 // `sources` also p_src and vn_src, which the GF extrapolation writes.  Stops at
 // the first failed copy and returns its error.
-static cudaError_t download_traces(Solve& s, adf_txgrid* txs, bool sources, float* stage,
+static cudaError_t download_traces(Solve& s, adf_txgrid* txs, bool sources, Stage stage,
                                    cudaStream_t st) {
   SolveDev& d = s.dev;
-  const size_t bytes = (size_t)d.nt * d.ntx * 4;
+  const size_t nt = d.nt, ntx = d.ntx;
   cudaError_t e = cudaSuccess;
   auto down = [&](const float* src, float* jl) {
-    if (e == cudaSuccess) e = launch_transpose(src, stage, d.ntx, d.nt, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(jl, stage, bytes, cudaMemcpyDeviceToHost, st);
+    if (e != cudaSuccess) return;
+    e = trace_pieces(nt, ntx, stage.floats, [&](size_t c, size_t nc, size_t t, size_t n) {
+      const cudaError_t ce = launch_transpose(src + t * ntx + c, (long long)ntx, stage.p,
+                                              (long long)n, (int)nc, (int)n, st);
+      return ce != cudaSuccess ? ce
+                               : cudaMemcpyAsync(jl + c * nt + t, stage.p, nc * n * 4,
+                                                 cudaMemcpyDeviceToHost, st);
+    });
   };
   for (int c = 0; c < 4; ++c) {
     down(d.rec[c], txs->rec[c]);
@@ -822,42 +854,40 @@ static cudaError_t download_traces(Solve& s, adf_txgrid* txs, bool sources, floa
 
 // psi: Julia (npml,ny,nz,2) / (nx,npml,nz,2) / (nx,ny,npml,2) <-> device.  An
 // upload fills both buffers, a download takes the one given.
-static size_t psi_floats(const SolveDev& d, int axis, bool vside) {
-  const size_t n = vside ? d.npml + 1 : d.npml;
-  const size_t nx = d.nx, ny = d.ny, nz = d.nz;
-  return 2 * n * (axis == 0 ? ny * nz : axis == 1 ? nx * nz : nx * ny);
-}
 static cudaError_t psi_copy(Solve& s, int axis, bool vside, float* host, bool upload, int buffer,
-                            float* stage, cudaStream_t st) {
+                            Stage stage, cudaStream_t st) {
   SolveDev& d = s.dev;
   const long long n = vside ? d.npml + 1 : d.npml;
   float* base = vside ? d.psi_v[axis] : d.psi_p[axis];
   const long long side = vside ? d.psi_v_side[axis] : d.psi_p_side[axis];
-  const size_t bytes = psi_floats(d, axis, vside) * 4;
-  // a block of rows of `width` floats: its place in a device buffer, in the host array
-  auto move = [&](float* dev, long long pitch, float* st_rows, int width, long long rows) {
-    return upload ? launch_repitch(st_rows, width, dev, pitch, width, rows, st)
-                  : launch_repitch(dev, pitch, st_rows, width, width, rows, st);
-  };
-  cudaError_t e = cudaSuccess;
-  if (upload) e = cudaMemcpyAsync(stage, host, bytes, cudaMemcpyHostToDevice, st);
-  for (int b = upload ? 0 : buffer; b <= (upload ? 1 : buffer); ++b) {
-    float* dev = base + (long long)b * 2 * side;
-    if (axis == 0) {  // rows of n values per side; device pitch npp / nvp, side 1 offset
-      const long long rows = (long long)d.ny * d.nz;
-      const long long first1 = vside ? d.nx - d.npml - 1 : d.nx - d.npml;  // side 1's first cell
-      // (a grid narrower than npml+1 cells never uses side 1: any in-row offset does)
-      const long long off1 = first1 < 0 ? 0 : first1 - (vside ? d.xs1v : d.xs1p);
-      for (int sd = 0; sd < 2 && e == cudaSuccess; ++sd)
-        e = move(dev + sd * side + (sd ? off1 : 0), vside ? d.nvp : d.npp, stage + sd * rows * n,
-                 (int)n, rows);
-    } else if (e == cudaSuccess) {
-      e = move(dev, d.nxp, stage, d.nx, axis == 1 ? n * d.nz * 2 : d.ny * n * 2);
+  // rows of `width` floats, contiguous on the host: pieces of them through the stage
+  auto move = [&](float* dev, long long pitch, float* rows_host, int width, long long rows) {
+    const long long most = std::max<long long>(1, (long long)stage.floats / width);
+    cudaError_t e = cudaSuccess;
+    for (long long r = 0; r < rows && e == cudaSuccess; r += most) {
+      const long long m = std::min(most, rows - r);
+      float* h = rows_host + r * width;
+      const size_t bytes = (size_t)m * width * 4;
+      if (upload) {
+        e = cudaMemcpyAsync(stage.p, h, bytes, cudaMemcpyHostToDevice, st);
+        for (int b = 0; b < 2 && e == cudaSuccess; ++b)
+          e = launch_repitch(stage.p, width, dev + b * 2 * side + r * pitch, pitch, width, m, st);
+      } else {
+        e = launch_repitch(dev + buffer * 2 * side + r * pitch, pitch, stage.p, width, width, m, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h, stage.p, bytes, cudaMemcpyDeviceToHost, st);
+      }
     }
-  }
-  if (!upload && e == cudaSuccess)
-    e = cudaMemcpyAsync(host, stage, bytes, cudaMemcpyDeviceToHost, st);
-  return e;
+    return e;
+  };
+  if (axis > 0) return move(base, d.nxp, host, d.nx, axis == 1 ? n * d.nz * 2 : d.ny * n * 2);
+  // rows of n values per side; device pitch npp / nvp, side 1 offset
+  const long long rows = (long long)d.ny * d.nz;
+  const long long first1 = vside ? d.nx - d.npml - 1 : d.nx - d.npml;  // side 1's first cell
+  // (a grid narrower than npml+1 cells never uses side 1: any in-row offset does)
+  const long long off1 = first1 < 0 ? 0 : first1 - (vside ? d.xs1v : d.xs1p);
+  const long long pitch = vside ? d.nvp : d.npp;
+  const cudaError_t e = move(base, pitch, host, (int)n, rows);
+  return e != cudaSuccess ? e : move(base + side + off1, pitch, host + rows * n, (int)n, rows);
 }
 
 // The context's pool after a run that took its memory from it: back to what it
@@ -1169,11 +1199,6 @@ static int run_fdtd_impl(adf_ctx* ctx, const adf_domain* d, float* field, adf_tx
               (size_t)8 * kGfRing * gf->n_rec;
     if (use_tc) need += sizeof(float) * gf_tc_packed_floats(gf->nt_gf, gf->n_src, gf->n_rec);
   }
-  // the layout conversions' buffer: the largest of a trace and a CPML array
-  const size_t n1 = (size_t)npml + 1, face = (size_t)std::max(
-      {d->ny * d->nz, d->nx * d->nz, d->nx * d->ny});
-  const size_t stage_floats = std::max((size_t)d->nt * txs->ntx, npml > 0 ? 2 * n1 * face : 0);
-  need += 4 * stage_floats;
   if (need > ctx->budget) return fail(ADF_E_BUDGET, "solve exceeds the context's HBM budget");
   PoolTrim trim(ctx);  // (before the solve and the batch, which return their memory first)
   auto s = std::make_unique<Solve>();
@@ -1182,7 +1207,9 @@ static int run_fdtd_impl(adf_ctx* ctx, const adf_domain* d, float* field, adf_tx
   const hm::Dom dom = to_dom(*d);
   int rc = solve_alloc(ctx, *s, dom, (int)npml, mask != nullptr, flags, (int)txs->ntx);
   if (!rc) rc = solve_alloc_traces(*s);
-  float* stage = rc ? nullptr : solve_dalloc<float>(*s, stage_floats, rc);
+  Stage stage{s->dev.field + s->dev.buf_stride, (size_t)s->dev.buf_stride};
+  const bool own_stage = stage.floats < kStageMin;
+  if (own_stage && !rc) stage = Stage{solve_dalloc<float>(*s, kStageMin, rc), kStageMin};
   if (rc) return rc;
   // Every upload below is a stream-ordered copy on the context stream: the
   // zeroing above, the copies, the set-up kernels and the steps run in that
@@ -1220,6 +1247,11 @@ static int run_fdtd_impl(adf_ctx* ctx, const adf_domain* d, float* field, adf_tx
     }
   }
   up(upload_traces(*s, txs, stage, st));
+  if (!own_stage) {  // a fresh solve's buffer 1 is zero
+    const size_t psi = 2 * ((size_t)npml + 1) * std::max({d->ny * d->nz, d->nx * d->nz, d->nx * d->ny});
+    const size_t used = std::min(stage.floats, std::max((size_t)d->nt * txs->ntx, psi));
+    up(cudaMemsetAsync(stage.p, 0, used * 4, st));
+  }
   if (use_gf) {  // GF tensors, 0-based columns, Float64 pin history
     const size_t ng = (size_t)gf->nt_gf * gf->n1 * gf->n2;
     for (int k = 0; k < ntens && !rc; ++k) {
@@ -1397,6 +1429,7 @@ static int run_fdtd_impl(adf_ctx* ctx, const adf_domain* d, float* field, adf_tx
   // output buffer of the last executed step
   const int fb = (int)((stop_step - start_step + 1) & 1);
   const float* last = sd.field + (size_t)fb * sd.buf_stride;
+  if (!own_stage) stage.p = sd.field + (size_t)(1 - fb) * sd.buf_stride;
   cudaError_t e =
       sd.nxp == sd.nx
           ? cudaMemcpyAsync(field, last, field_rows * sd.nx * 4, cudaMemcpyDeviceToHost, st)

@@ -82,10 +82,7 @@ static size_t gf_bytes(const adf_gf_request& r) {
   const size_t nx = r.dom.nx, ny = r.dom.ny, nz = r.dom.nz, n = r.npml, nt = r.dom.nt;
   const size_t ntx = 1 + r.n_rec;
   size_t b = 2ull * 4 * nz * ny * nxp * 4;
-  if (r.shape != ADF_SHAPE_NONE) {  // the bits, and a byte per tile and plane
-    b += (size_t)mw * ny * nz * 4;
-    b += (size_t)((nxp + step_x_tile() - 1) / step_x_tile()) * ((ny + ty - 1) / ty) * nz;
-  }
+  if (r.shape != ADF_SHAPE_NONE) b += (size_t)mw * ny * nz * 4;
   b += 2ull * 2 * 4 * (nz * ny * n + nz * n * nxp + n * ny * nxp);
   b += 2ull * 2 * 4 * (nz * ny * (n + 1) + nz * (n + 1) * nxp + (n + 1) * ny * nxp);
   b += 2ull * nt * ntx * 4 + 4ull * nt * 4;  // p/vn records + source columns
