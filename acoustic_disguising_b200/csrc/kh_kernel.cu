@@ -396,7 +396,8 @@ __global__ void adf_kh_combine_kernel(const float2* __restrict__ part, float* __
       double a = 0.0;
       for (int z = 0; z < splits; ++z) {
         const float2 v = p[z * n];
-        a += (double)v.x - (double)v.y;
+        // (an infinite sum's compensation is infinite or NaN)
+        a += isinf(v.x) ? (double)v.x : (double)v.x - (double)v.y;
       }
       out[(long long)r * nt + t0 + t] = (float)a;
     }

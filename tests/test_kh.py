@@ -223,3 +223,31 @@ def test_kh_parts_take_the_memory_of_their_launch(adf, oracle, ns, blocks):
     for part in (slice(0, nt - 10), slice(nt - 10, nt)):
         assert np.abs(ref[part]).max() > 0
         assert rel_l2(out[part][:, pick], ref[part]) <= 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["pressure", "velocity"])
+def test_kh_parts_keep_infinite_samples(adf, oracle, ctx, kind):
+    """Samples past Float32 in the last surface point's group are infinite whether the
+    surface is summed in one part (many targets) or in several (few), and the others
+    are what they are without them."""
+    ns, nt = 200, 700
+    c = case(ns, 2368, nt, 5e-6, 0.25, 0.35)
+    c["q"][:, :] = 0
+    c["f"][:, :] = 0
+    c["f"][40, ns - 1] = 1e30     # one sample: no two products meet in a sum
+    fn = adf.kh_pressure if kind == "pressure" else adf.kh_velocity
+    rn = c["rp"] / np.linalg.norm(c["rp"], axis=1, keepdims=True)
+
+    def run(nr, af):
+        rp = np.asfortranarray(c["rp"][:nr])
+        extra = () if kind == "pressure" else (np.asfortranarray(rn[:nr]),)
+        return fn(c["sp"], c["sn"], rp, *extra, c["q"], c["f"], c["dt"], c["sigma"], C0, 0.0, af,
+                  rho=RHO)
+    small = run(2368, 1.0)
+    scale = 1e9 * 3.4e38 / float(np.abs(small).max())
+    assert np.isfinite(small).all() and np.isfinite(scale)
+    one, parts = run(2368, scale)[:, :48], run(48, scale)
+    assert np.isinf(one).any() and not np.isnan(one).any()
+    assert np.array_equal(np.isinf(one), np.isinf(parts)) and not np.isnan(parts).any()
+    assert np.array_equal(one[np.isinf(one)], parts[np.isinf(one)])
