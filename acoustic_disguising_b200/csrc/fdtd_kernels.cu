@@ -682,7 +682,7 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
     const int u = k - kfirst;
     float* pn = sPn + (k & 1) * (kMaxTy + 1) * kPnPitch;
     const float* st = ring + slot_of(k) * kStageFloats;
-    if (!mbar_try_wait(smem_u32(rbar) + 8u * (u & 1), (uint32_t)(u >> 1) & 1u)) wait(k);
+    if (!mbar_try_wait(smem_u32(rbar + (uint32_t)u % kStepRing), (uint32_t)u / kStepRing & 1u)) wait(k);
     const int fl = s_fl[u];
     const bool has_mask = (fl & 4) != 0;  // elsewhere every cell of the tile's plane is open
     const bool wplain = wplain_rx && (fl & 12) == 8;
