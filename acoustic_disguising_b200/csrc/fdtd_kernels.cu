@@ -493,9 +493,8 @@ constexpr int kStageFloats = (kStageVz + kStageChan + 31) / 32 * 32;
 constexpr uint32_t kStepWaitLimit = 1u << 20;
 static_assert((kStageFloats * 4) % 128 == 0, "stages stay 128-B aligned");
 
-// Fetches plane k's slab memory of the item into L2, a warp to a plane: lane = tile row +
-// 8 x array (p y, v y, p z, v z; the v arrays have no halo row, whose lanes take the x
-// slabs' rows, one contiguous piece each).  A boundary warp waits for reads of slab
+// Fetches plane k's slab memory of the item into L2, a warp to a plane (slab_piece says
+// what each lane takes).  A boundary warp waits for reads of slab
 // memory that nothing has touched since the last step, and its length sets its CTA's
 // pace.  On grids whose memory stays in L2 there is nothing to gain (128^3: 39 us
 // without this, 41 with it; 192^3: 89.4 and 86.7), so it is for grids from 2^22 cells on:
@@ -508,37 +507,12 @@ static_assert((kStageFloats * 4) % 128 == 0, "stages stay 128-B aligned");
 constexpr long long kFetchCells = 1 << 22, kFetchXCells = 1 << 24;
 __device__ __noinline__ void fetch_slabs(const SolveDev& S, const PmlTab& Q, int4 item, int kfirst,
                                          int k) {
-  const int lane = threadIdx.x, row = lane & 7, arr = lane >> 3, n = S.npml;
-  const int j = (item.y & 0xFFFF) * S.ty - 1 + row, X = item.y >> 16, xb = X * kXT;
-  if (k >= item.w || j >= S.ny || row > S.ty) return;
-  const bool v = arr & 1;
-  constexpr int line = 32;  // floats
-  if (v && row == 0) {
-    const bool lo = X == 0, hi = (X + 1) * kXT >= S.nxp, xv = arr == 3;
-    if ((!lo && !hi) || S.chan_stride < kFetchXCells) return;
-    const int pitch = xv ? S.nvp : S.npp, j0 = max(j, 0), j1 = min(j + S.ty + 1, S.ny);
-    const float* p = slab_cell(Q.rd[xv ? 3 : 0],
-                               slab_quad(xv ? S.psi_v_side[0] : S.psi_p_side[0], !lo, k * S.ny + j0,
-                                         pitch, 0), 0);
-    for (int i = 0; i < (j1 - j0) * pitch; i += line) prefetch_l2(p + i);
-    return;
-  }
-  if (j < 0) return;
-  uint32_t o;
-  if (arr < 2) {
-    const int m = n + (v ? 1 : 0), right = j >= m;  // layers
-    if (right && j < S.ny - m) return;
-    o = slab_quad(v ? S.psi_v_side[1] : S.psi_p_side[1], right,
-                  k * m + (right ? j - (S.ny - m) : j), S.nxp, xb);
-  } else {
-    o = v ? Q.zv[k - kfirst] : Q.zp[k - kfirst];
-    if (o == kNoSlab) return;
-    o += slab_quad(0, 0, j, S.nxp, xb);
-  }
-  const float* p = slab_cell(Q.rd[(arr < 2 ? 1 : 2) + (v ? 3 : 0)], o, 0);
-#pragma unroll
-  for (int i = 0; i < kXT; i += line)
-    if (i < S.nxp - xb) prefetch_l2(p + i);
+  if (k >= item.w) return;
+  const SlabPiece f = slab_piece(S, item.y >> 16, item.y & 0xFFFF, kXT, threadIdx.x, k,
+                                 S.chan_stride >= kFetchXCells, Q.zp[k - kfirst], Q.zv[k - kfirst]);
+  const float* p = slab_cell(Q.rd[f.array], f.quad, 0);
+#pragma unroll 2
+  for (int i = 0; i < f.floats; i += 32) prefetch_l2(p + i);  // a line each
 }
 
 // One thread: the copies of plane k's stage into a free slot.

@@ -69,6 +69,87 @@ int main(int argc, char** argv) {
 """
 
 
+# What the lanes of a warp fetch ahead of a plane of a tile, against the slab rows of
+# the tile, worked out cell by cell in 64 bits from the layout of solve_alloc.
+PIECES = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <algorithm>
+#include <set>
+#include <utility>
+#include "slab_index.h"
+using namespace adf;
+typedef long long ll;
+struct Grid {
+  int ny, ty, nxp, npml, npp, nvp;
+  ll psi_p_side[3], psi_v_side[3];
+};
+int main(int argc, char** argv) {
+  const int nx = atoi(argv[1]), ny = atoi(argv[2]), nz = atoi(argv[3]), n = atoi(argv[4]);
+  const int ty = atoi(argv[5]), xt = 64, nxp = (nx + 3) / 4 * 4;
+  auto pitch = [&](int m) { return std::max((m + 3) / 4 * 4, nxp - std::max(0, nx - m) / 4 * 4); };
+  Grid g{ny, ty, nxp, n, pitch(n), pitch(n + 1), {}, {}};
+  for (int v = 0; v < 2; ++v) {
+    const ll m = n + v, s[3] = {(ll)nz * ny * (v ? g.nvp : g.npp), nz * m * nxp, m * ny * nxp};
+    for (int a = 0; a < 3; ++a) (v ? g.psi_v_side : g.psi_p_side)[a] = s[a];
+  }
+  auto side = [&](int array) { return (array >= 3 ? g.psi_v_side : g.psi_p_side)[array % 3]; };
+  ll wrong = 0, fetched = 0;
+  for (int k = 0; k < nz; ++k) {
+    // (-1, m: the layer and its side; slab memory of the v side starts at plane 1)
+    auto layer = [&](int v) {
+      const int m = n + v;
+      if (k < v) return kNoSlab;
+      if (k < m) return slab_quad(g.psi_p_side[2], 0, (uint32_t)(k * ny), nxp, 0);
+      if (k >= nz - m)
+        return slab_quad(side(v ? 5 : 2), 1, (uint32_t)((k - (nz - m)) * ny), nxp, 0);
+      return kNoSlab;
+    };
+    for (int T = 0; T < (ny + ty - 1) / ty; ++T)
+      for (int X = 0; X < (nxp + xt - 1) / xt; ++X) {
+        const int xb = X * xt, xe = std::min(xb + xt, nxp);
+        std::set<std::pair<int, ll>> want, got;  // (array, float / 4)
+        for (int r = 0; r <= ty; ++r) {
+          const int j = T * ty - 1 + r;
+          if (j < 0 || j >= ny) continue;
+          for (int v = 0; v < 2; ++v) {
+            const ll m = n + v;
+            if (X == 0 || xe == nxp) {
+              const ll p = v ? g.nvp : g.npp, s = X == 0 ? 0 : 1;
+              for (ll x = 0; x < p; x += 4)
+                want.insert({3 * v, (s * side(3 * v) + ((ll)k * ny + j) * p + x) / 4});
+            }
+            if (v && r == 0) continue;  // the halo row has no velocity update
+            for (ll x = xb; x < xe; x += 4) {
+              if (j < m) want.insert({1 + 3 * v, ((k * m + j) * nxp + x) / 4});
+              else if (j >= ny - m)
+                want.insert({1 + 3 * v, (side(1 + 3 * v) + (k * m + j - (ny - m)) * nxp + x) / 4});
+              if (k >= v && k < m) want.insert({2 + 3 * v, (((ll)k * ny + j) * nxp + x) / 4});
+              else if (k >= nz - m)
+                want.insert({2 + 3 * v, (side(2 + 3 * v) + ((k - (nz - m)) * ny + j) * nxp + x) / 4});
+            }
+          }
+        }
+        for (int lane = 0; lane < 32; ++lane) {
+          const SlabPiece f = slab_piece(g, X, T, xt, lane, k, true, layer(0), layer(1));
+          for (int i = 0; i < f.floats; i += 4) {
+            const ll at = (ll)f.quad * 4 + i;
+            if (at < 0 || at + 4 > 2 * side(f.array)) ++wrong;
+            got.insert({f.array, at / 4});
+          }
+          const SlabPiece h = slab_piece(g, X, T, xt, lane, k, false, layer(0), layer(1));
+          if (h.floats != (f.array % 3 == 0 ? 0 : f.floats)) ++wrong;
+        }
+        if (got != want) ++wrong;
+        fetched += (ll)got.size();
+      }
+  }
+  std::printf("%lld %lld\n", wrong, fetched);
+  return 0;
+}
+"""
+
+
 def run_cpp(tmp_path, text, *args):
     gxx = shutil.which("g++")
     if gxx is None:
@@ -93,6 +174,20 @@ def test_slab_places(tmp_path, nx, ny, nz, npml, past):
     bad, top = map(int, run_cpp(tmp_path, PLACES, nx, ny, nz, npml).split())
     assert bad == 0
     assert top >= past
+
+
+@pytest.mark.parametrize("nx,ny,nz,npml,ty", [
+    (163, 30, 29, 7, 7),    # three x tiles, the last y tile of two rows
+    (129, 29, 21, 1, 7),    # one layer: velocity memory of two; an x tile of one quad
+    (70, 23, 25, 9, 5),     # the right x slab begins in the tile before the last
+    (40, 16, 18, 3, 7),     # one x tile with both slabs: the left one is fetched
+])
+def test_slab_pieces(tmp_path, nx, ny, nz, npml, ty):
+    """The memory fetched ahead of every plane of every tile is that of the tile's slab
+    rows, all of it, and lies inside its buffer."""
+    wrong, fetched = map(int, run_cpp(tmp_path, PIECES, nx, ny, nz, npml, ty).split())
+    assert wrong == 0
+    assert fetched > 0
 
 
 @pytest.mark.gpu
