@@ -295,7 +295,7 @@ __global__ void adf_gf_resample_kernel(int ncol, int n, int nt_out, double t_in0
 // it as the sequential recurrence does.)  The Thomas division by 4 - cpv[i-1] is
 // a product with cpv[i], its reciprocal.  2000 -> 700 samples x 4096 columns:
 // 1.25 ms as two kernels with a thread per column, whose 66 MB of coefficients
-// were written and read at a stride of a column; 0.19 ms here, bound by the
+// were written and read at a stride of a column; 0.16 ms here, bound by the
 // instructions of the sweeps (half the issue slots).
 constexpr int kGfWarm = 64;
 constexpr int kGfThreads = 128;

@@ -16,12 +16,12 @@
 // the halo row and column are recomputed, not exchanged.  Five such CTAs per
 // SM keep HBM busy while a plane's chain (stage loads, Float64 arithmetic,
 // exchange of the new P, Float64 arithmetic) runs in each; what bounds them is
-// that chain and the instructions around it, not HBM.  With the stage read
-// through shared-space addresses, on different banks, and the entries' code out
-// of the plane loop, a launch of 8 x 256^3 takes 0.75 ms without boundaries
-// (0.89 before) and 1.21 ms with 10-cell CPML, a sphere and 2048 receivers (1.82).
-// The plane loop's code has to stay small: a masked form of the plain update and
-// one with the x slab's memory each made it slower (1.57 and 1.66 ms).
+// that chain and the instructions around it, not HBM.  The stage is read through
+// shared-space addresses, on different banks, and the entries' code is out of the
+// plane loop.  A launch of 8 x 256^3 takes 0.75 ms without boundaries and, with
+// 10-cell CPML, a sphere and 2048 receivers, 1.21 ms in short runs and 1.25 over 2000
+// steps (under the power cap).  The plane loop's code has to stay small: a masked form
+// of the plain update made the second 2 % slower, one with the x slab's memory 6 %.
 //
 // Arithmetic: Arith<double> reproduces Julia's promotion (Float32 storage,
 // Float64 Domain scalars, src/kernels/updates.jl) with explicit round-to-
@@ -496,14 +496,14 @@ static_assert((kStageFloats * 4) % 128 == 0, "stages stay 128-B aligned");
 // Fetches plane k's slab memory of the item into L2, a warp to a plane (slab_piece says
 // what each lane takes).  A boundary warp waits for reads of slab
 // memory that nothing has touched since the last step, and its length sets its CTA's
-// pace.  On grids whose memory stays in L2 there is nothing to gain (128^3: 39 us
-// without this, 41 with it; 192^3: 89.4 and 86.7), so it is for grids from 2^22 cells on:
-// 8 x 256^3 with CPML 1.108 -> 1.044 ms, with a sphere 1.252 -> 1.209, 2 x 256^3
-// 314 -> 294 us, 512^3 1.003 -> 0.968 ms.  The x slabs are read a phase ahead anyway and
-// pay from 2^24 cells on (192^3 86.7 without them, 88.5 with; 256^3 157.0, 157.5;
-// 8 x 256^3 with CPML 1.061, 1.044).  A prefetch a quad in place of a row took 28.6 us at
-// 96^3 (26.7) and 0.768 ms at 8 x 256^3 without CPML (0.750).  Out of line, as
-// apply_entries is.
+// pace.  Launches in us, without this, with the y and z slabs, with the x slabs too:
+//   8 x 256^3, CPML 1109 1064 1040; and a sphere 1259 1224 1209; 2 x 256^3 334 325 321;
+//   256^3 168 164 162; 512^3 1009 976 965; 224^3 135 132 131; 192^3 94.4 92.6 92.4
+// A small solve alone keeps its memory in L2 and loses (128^3 37.0 and 38.3, 96^3 26.9
+// and 27.4, y and z slabs), so it is for solves of 2^22 cells and more, the x slabs,
+// which are read a phase ahead anyway, for 2^24.  The line looks at one solve, not at
+// the launch: batches of small solves lie on its wrong side (8 x 128^3 195 and 190,
+// 30 x 96^3 398 and 381, 4 x 160^3 194 and 188).  Out of line, as apply_entries is.
 constexpr long long kFetchCells = 1 << 22, kFetchXCells = 1 << 24;
 __device__ __noinline__ void fetch_slabs(const SolveDev& S, const PmlTab& Q, int4 item, int kfirst,
                                          int k) {
@@ -644,8 +644,9 @@ __device__ __forceinline__ void step_item(const SolveDev& S, const PmlTab& Q, in
   // The x-slab memory of a quad is read ahead of its use: the p side's of plane
   // k+1 during the velocity update of plane k, the v side's of plane k during its
   // pressure update.  One warp of every x-end tile would otherwise wait for two
-  // more reads of global memory per plane than the other three (1.39 ms without
-  // this at 8 x 256^3 with CPML and a sphere, 1.31 with it).
+  // more reads of global memory per plane than the other three: without this
+  // 8 x 256^3 with CPML and a sphere takes 1241 us (1209), 8 x 96^3 137 (125),
+  // 192^3 100 (93); 8 x 256^3 without CPML is 2 % faster (735, 748).
   const bool pxm = (q.bits & 0xF000u) && !(q.bits & (1u << 20));
   const bool vxm = (q.bits & 0xF0000u) && !(q.bits & (1u << 20));
   float4 mpx = make_float4(0.f, 0.f, 0.f, 0.f), mvx = mpx;
@@ -903,9 +904,9 @@ __global__ void __launch_bounds__(kStepThreads, kStepCtasPerSm) adf_fdtd_step_ke
 // closed[x tile][y tile][plane] = 1 where a cell of the tile's plane, its halo
 // row and column included, has a closed mask bit (set-up, once per mask): the
 // step kernel reads the mask on those planes of a tile only, so that the rest
-// of the grid has neither the load in the plane's chain nor the selects (512^3
-// with an ellipsoid 1.38 -> 1.20 ms a launch, 8 x 256^3 with a sphere
-// 1.71 -> 1.60).  One warp per (x, y, plane).
+// of the grid has neither the load in the plane's chain nor the selects (read
+// everywhere, 512^3 with an ellipsoid takes 1272 us a launch, 8 x 256^3 with a
+// sphere 1411; so 965 and 1209).  One warp per (x, y, plane).
 __global__ void adf_mask_tiles_kernel(const uint32_t* bits, int nx, int ny, int nz, int mw, int ty,
                                       int nty, int nxt, unsigned char* closed) {
   const long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
@@ -940,7 +941,7 @@ cudaError_t launch_mask_tiles(const SolveDev& d, unsigned char* closed, cudaStre
 // v2vn! :85-90, vn2v! :92-97 into row it+1).  Four lanes per transceiver, one per
 // channel: the kernel does next to nothing and its time is the chain of its reads
 // (a thread per transceiver, through the descriptor in global memory and corner by
-// corner, took 9.9 us cold between a step and the next).  Places are looked up
+// corner, took 9.9 us cold between a step and the next, this 5.4).  Places are looked up
 // before the wait for the step kernel; after it, one round of reads is left.
 constexpr int kEpiThreads = 128;
 __global__ void __launch_bounds__(kEpiThreads) adf_fdtd_epilogue_kernel(const EpiParams p) {

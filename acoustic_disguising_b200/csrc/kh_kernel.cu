@@ -18,7 +18,7 @@
 // Work decomposition (CUDA cores, FP32 FMA bound):
 //   CTA   = 16 targets x one block of 32*T output samples, 16 warps
 //   warp  = KH_RW targets (default 1); lane = T consecutive output samples
-//           of each (T odd: 13 or 17, chosen per call by the padded cost)
+//           of each (T odd: blocks of 17, and a last one of 17, 13 or 7)
 //   loop  = surface points in chunks of SC.  One thread stages chunk c+1's
 //           input windows into shared memory with bulk async copies while
 //           the CTA works on chunk c (double buffer, mbarrier completion);
@@ -518,8 +518,9 @@ __global__ void adf_kh_gather_kernel(const float* q, const float* f, int ntx, in
 // middling one a last wave that is nearly empty; each part repeats a CTA's start
 // (about two surface points' time) and costs one pass over its share of the
 // partial sums.  Estimated in us from the measured time of a surface point.
-// 200 points -> 48 targets x 700 samples: 283 us in one part, 49 in 16 or more;
-// 2048 -> 4096 x 500: 6.95 and 6.16 ms.
+// 200 points -> 48 targets x 700 samples, two launches: 523 us in one part each, 62 in
+// 25 and 24; 2048 -> 4096 x 500: 7.00 and 6.25 ms; 1500 -> 2001 x 1201, velocity: 11.9
+// and 10.5.
 // A part's sums take 8 bytes a target and sample, 256 MB in all at most.
 static int kh_splits(int nsm, long long ctas, int ns, int nr, int samples, double point_us) {
   int best = 1;

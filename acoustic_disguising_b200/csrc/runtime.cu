@@ -419,23 +419,22 @@ void Solve::add_chunk(int solve, int z0, int z1, std::vector<int4>& out) const {
 // waste least and shallow ones spread the work; `resident` CTAs run at once.
 //
 // When every solve fits the resident CTAs at one depth of at most 7, the shallowest
-// such depth is taken: one wave of equal chunks (96^3: 73 us a step at 16 planes, 31 at
-// 4).  The items of several solves alternate, so that each SM gets its share of the
-// chunks inside the z slabs (4 x 64^3: 39 us, 42 one solve after the other).  Above 7
-// planes two and more waves are as fast or faster (2 x 96^3, depth 7: 48.5 and 47.4 us;
-// 8 x 64^3, depth 8: 79 and 65; 128^3, depth 7: 43 and 46).
+// such depth is taken: one wave of equal chunks (96^3 26.8 us a step, cut as below 30.7;
+// 4 x 64^3 28.6 and 32.3; 128^3 37.1 and 38.6).  The items of several solves alternate,
+// so that each SM gets its share of the chunks inside the z slabs.  A wave of deeper
+// items waits for its longest: up to 16 planes, 160^3 takes 86 us (66 as below), though
+// batches of small solves would gain (30 x 40^3 56 and 60, 2 x 96^3 41 and 43).
 //
 // Otherwise the CTAs take items as they finish, and what matters is that they end
 // together: a chunk holds at most the planes that are left per resident CTA, so that the
-// chunks become shallower towards the end, down to 3 planes, and the outer chunks, whose
-// planes lie in the z slabs and take longer (counted as 1.5), come first.  No chunk is
-// more than 0.6 of what a resident CTA gets in all: the first ones would outlast all
-// others (224^3: 166 us without that bound, 142 with it).  Step kernel, against equal
-// chunks of 24, 12 or 8 planes from the bottom up: 256^3 203 -> 177 us, 2 x 256^3
-// 351 -> 328, 8 x 256^3 1263 -> 1231, 512^3 1038 -> 1018, 192^3 120 -> 101, 224^3
-// 159 -> 142, 160^3 92 -> 79, 8 x 96^3 162 -> 145, 30 x 40^3 126 -> 100.  Over 20 batches
-// the time was on average 1.01 times the best of 30 settings of these numbers, 1.16
-// times before.
+// chunks become shallower towards the end, down to 3 planes (or the 2 that halving the
+// last 4 or 5 leaves), and the outer chunks, whose planes lie in the z slabs and take
+// longer (counted as 1.5), come first.  No chunk is more than 0.6 of what a resident CTA
+// gets in all: the first ones could outlast all others (224^3 141 us without that bound,
+// 132 with it; small batches pay for it, 8 x 64^3 47 and 51).  Step kernel in us, equal
+// chunks of 16 planes from the bottom up and this: 256^3 189 and 162, 2 x 256^3 346 and
+// 321, 8 x 256^3 1267 and 1209, 512^3 1002 and 965, 192^3 117 and 93, 224^3 158 and 132,
+// 160^3 85 and 66, 8 x 96^3 148 and 125, 30 x 40^3 77 and 60.
 void cut_items(const std::vector<Solve*>& list, long long resident, std::vector<int4>& out) {
   const int ns = (int)list.size();
   auto cap = [](const Solve* s) { return s->nzc > 0 ? std::min(s->nzc, kMaxZc) : kMaxZc; };

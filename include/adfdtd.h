@@ -99,7 +99,10 @@ int adf_version(void);
 /* Copies the calling thread's last error message (NUL-terminated). */
 int adf_last_error(char* buf, size_t n);
 
-/* Context: one device, one HBM budget (bytes, 0 = 90% of free memory). */
+/* Context: one device, one HBM budget (bytes, 0 = 90% of free memory).
+ * Device memory that a call frees stays with the context for later calls, until
+ * adf_ctx_destroy: all of it after GF solves and KH calls, at most 1 GiB (or
+ * what the context held before) after adf_run_fdtd and adf_gf_postprocess.  */
 int adf_ctx_create(int device, size_t hbm_budget, adf_ctx** out);
 int adf_ctx_destroy(adf_ctx* ctx);
 
